@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <new>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -24,6 +25,7 @@
 #include "gemm_limb.h"
 #include "internal.h"
 #include "prep.h"
+#include "quad_gemm.h"
 #include "results.h"
 #include "threshold.h"
 
@@ -133,6 +135,20 @@ struct irs_sharedb {
   uint16_t* results = nullptr;
   size_t res_offset = 0, res_len = 0;
   uint64_t batch = 0;
+  // rotation-structured GEMM (quad_gemm.cu): the records' derived sums, one
+  // allocation (outer lo, hi [db_cap][K/2], inner lo, hi [db_cap][3K/4]), and
+  // the query forms (lo, hi [9][n_pad/4][K/4]) with the slots' row masks
+  uint8_t* sums = nullptr;
+  uint8_t* forms = nullptr;
+  uint32_t* row_valid = nullptr;
+  uint32_t* quad_flag = nullptr;  // device copy of quad_rows, for captured launches
+  bool flag_set = false;      // what the last upload left in it
+  bool quad_rows = false;     // the uploaded rows are quads of rotations and the forms hold them
+  size_t stale_end = 0;       // records below it have sums that a small gather left behind
+  size_t forms_pad = 0;       // padded rows that the form maps are for (0: none)
+  bool sums_captured = false; // a captured launch reads the sums: they stay until alloc_db or destroy
+  CUtensorMap tm_sum_lo[2]{}, tm_sum_hi[2]{}, tm_form_lo[kQuadWidths]{},
+      tm_form_hi[kQuadWidths]{};
   CUtensorMap tm_db_lo{}, tm_db_hi{}, tm_q_lo{}, tm_q_hi{};
   int block_n = 0;
   cudaEvent_t done = nullptr;  // recorded after the engine's last dot launch
@@ -182,10 +198,71 @@ cudaStream_t party_stream(irs_device_manager* dm, int party, void* s) {
   return s ? static_cast<cudaStream_t>(s) : dm->streams[party];
 }
 
+// Engines that hold derived sums, over all device managers of the process.
+// The sums are an extra layout of records that are resident anyway, so they
+// give way when an allocation of the library fails.  The lock covers every
+// read of an engine's sums up to the launch that uses them.
+struct SumHolders {
+  std::mutex mu;
+  std::vector<irs_sharedb*> engines;
+};
+SumHolders& sum_holders() {
+  static SumHolders h;
+  return h;
+}
+
+// Frees an engine's sums and forms (the holders' lock is held).  cudaFree
+// waits for the launches that read them.
+void drop_sums_locked(irs_sharedb* db) {
+  auto& v = sum_holders().engines;
+  v.erase(std::remove(v.begin(), v.end(), db), v.end());
+  if (db->sums) cudaFree(db->sums);
+  if (db->forms) cudaFree(db->forms);
+  db->sums = db->forms = nullptr;
+  db->row_valid = db->quad_flag = nullptr;
+  db->quad_rows = db->flag_set = false;
+  db->stale_end = 0;
+  db->forms_pad = 0;
+  db->sums_captured = false;
+}
+
+void drop_sums(irs_sharedb* db) {
+  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  drop_sums_locked(db);
+}
+
+// Gives back the sums of every engine on `device` that no captured graph
+// reads; whether there were any.
+bool reclaim_sums(int device) {
+  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  const std::vector<irs_sharedb*> all = sum_holders().engines;
+  bool any = false;
+  for (irs_sharedb* db : all)
+    if (db->dm->device == device && !db->sums_captured && !db->dm->capturing) {
+      drop_sums_locked(db);
+      any = true;
+    }
+  return any;
+}
+
+// cudaMalloc that gives the derived sums back before it fails.
+cudaError_t device_malloc(irs_device_manager* dm, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (!dm->capturing && reclaim_sums(dm->device)) e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 int pool_alloc(irs_device_manager* dm, int party, size_t bytes, void** out) {
   *out = nullptr;
   if (!bytes) return IRS_OK;
   cudaError_t e = cudaMallocFromPoolAsync(out, bytes, dm->pools[party], dm->streams[party]);
+  if (e == cudaErrorMemoryAllocation && !dm->capturing) {
+    cudaGetLastError();
+    if (reclaim_sums(dm->device)) e = cudaMallocFromPoolAsync(out, bytes, dm->pools[party], dm->streams[party]);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(IRS_ERR_NOMEM, "device allocation of %zu bytes for party %d failed: %s", bytes, party,
@@ -237,9 +314,143 @@ static size_t padded_query_rows(size_t rows, size_t n_cap) {
   return wide <= n_cap ? wide : n64;
 }
 
+// ---- rotation-structured GEMM (quad_gemm.cu) ----
+
+// Fewest padded query rows for which the quad GEMM runs: it reads 2.25x the DB
+// bytes of the plain one.  Six engines over 32,768 entries, quad against the
+// better plain GEMM: 256 rows 1.73 / 1.05 ms, 384 1.93 / 1.83, 512 2.02 / 2.04,
+// 640 2.20 / 2.58, 768 2.40 / 2.78, 2048 5.3 / 7.3.
+constexpr size_t kQuadMinRows = 576;
+// Fewest records for which an engine keeps (or a gather brings along) the sums:
+// under that a launch has too few tiles for the nine products to pay (700
+// entries x 2048 rows: 0.19 ms either way; 2,048 entries: 0.35 / 0.52 ms).
+constexpr size_t kQuadMinRecords = 1024;
+
+size_t sums_bytes(size_t cap, size_t K) { return 2 * cap * (K / 2 + 3 * K / 4); }
+size_t forms_bytes(size_t n_cap, size_t K) { return 2 * (kQuadProducts * (n_cap / 4) * (K / 4)); }
+
+// Allocates the derived sums and query forms of an engine whose DB planes have
+// just been allocated (and zeroed, so the sums start at zero too).  Optional:
+// without them the engine runs the plain GEMM.  They are kept out of the way
+// of the program's other allocations: a sixth of the device's memory stays
+// free, and reclaim_sums gives them back when the library needs the room.
+void alloc_sums(irs_sharedb* db) {
+  irs_device_manager* dm = db->dm;
+  const size_t K = db->code_length, cap = db->db_cap;
+  if (K % kRowLen || db->n_cap < kQuadMinRows || cap < kQuadMinRecords || dm->capturing) return;
+  const size_t forms = forms_bytes(db->n_cap, K), masks = db->n_cap / kSlotRows * 4 + 4;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < sums_bytes(cap, K) + forms + total_b / 6) {
+    cudaGetLastError();
+    return;
+  }
+  void *s = nullptr, *f = nullptr;
+  if (cudaMalloc(&s, sums_bytes(cap, K)) != cudaSuccess || cudaMalloc(&f, forms + masks) != cudaSuccess) {
+    cudaGetLastError();
+    if (s) cudaFree(s);
+    return;
+  }
+  db->sums = static_cast<uint8_t*>(s);
+  db->forms = static_cast<uint8_t*>(f);
+  db->row_valid = reinterpret_cast<uint32_t*>(db->forms + forms);
+  db->quad_flag = db->row_valid + db->n_cap / kSlotRows;
+  cudaStream_t st = dm->streams[db->peer];
+  uint8_t* inner = db->sums + 2 * cap * (K / 2);
+  if (make_tmap_plane(&db->tm_sum_lo[0], db->sums, cap, K / 2, 128) ||
+      make_tmap_plane(&db->tm_sum_hi[0], db->sums + cap * (K / 2), cap, K / 2, 128) ||
+      make_tmap_plane(&db->tm_sum_lo[1], inner, cap, 3 * K / 4, 128) ||
+      make_tmap_plane(&db->tm_sum_hi[1], inner + cap * (3 * K / 4), cap, 3 * K / 4, 128) ||
+      cudaMemsetAsync(db->sums, 0, sums_bytes(cap, K), st) != cudaSuccess ||
+      cudaMemsetAsync(db->quad_flag, 0, 4, st) != cudaSuccess) {
+    cudaGetLastError();
+    drop_sums(db);
+    return;
+  }
+  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  sum_holders().engines.push_back(db);
+}
+
+// Whether a gather of n records leaves the sums behind: for a few records the
+// quad GEMM does not run, and the sums would be the larger part of the gather.
+bool gather_skips_sums(const irs_sharedb* db, size_t n) { return n < kQuadMinRecords && !db->sums_captured; }
+
+// Brings the sums of records [first, first + n) in line with the planes, on
+// the stream that wrote them.
+cudaError_t update_sums(irs_sharedb* db, size_t first, size_t n, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  if (!db->sums || !n) return cudaSuccess;
+  const size_t K = db->code_length, cap = db->db_cap, o = K / 2, i = 3 * K / 4;
+  uint8_t* inner = db->sums + 2 * cap * o;
+  return launch_derive_sums(db->db_lo + first * K, db->db_hi + first * K, (uint32_t)K, n, db->sums + first * o,
+                            db->sums + cap * o + first * o, inner + first * i, inner + cap * i + first * i, s);
+}
+
+// Prepares the query forms' tensor maps for the active row count; false where
+// the quad GEMM does not run.
+bool quad_forms_ready(irs_sharedb* db) {
+  if (!db->sums || db->n_pad < kQuadMinRows) return false;
+  if (db->forms_pad == db->n_pad) return true;
+  const size_t K = db->code_length, rows = kQuadProducts * (db->n_pad / 4);
+  db->forms_pad = 0;
+  for (int w = 0; w < kQuadWidths; w++) {
+    const uint32_t box = (uint32_t)quad_tile_n((uint32_t)db->n_pad, w) / 2;
+    if (make_tmap_plane(&db->tm_form_lo[w], db->forms, rows, K / 4, box) ||
+        make_tmap_plane(&db->tm_form_hi[w], db->forms + rows * (K / 4), rows, K / 4, box))
+      return false;
+  }
+  db->forms_pad = db->n_pad;
+  return true;
+}
+
+// Whether the live rows of every quad (rows i, i + 2, i + 4, i + 6 of a slot,
+// i in 0, 1, 8, 9, ...) are rotations of one base that keep their distance:
+// the rows the quad GEMM can run.  Empty rows fit anywhere.
+bool rows_are_quads(const uint32_t* desc, size_t n_rows) {
+  for (size_t b = 0; b < n_rows; b += 8)
+    for (size_t i = b; i < b + 2; i++) {
+      uint32_t want = 0xFFFFFFFFu;  // descriptor of row i, rotation counted back to it (mod 2^32)
+      for (size_t m = 0; m < 4; m++) {
+        const size_t r = i + 2 * m;
+        if (r >= n_rows || desc[r] == 0xFFFFFFFFu) continue;
+        // the rotation field has 7 bits and holds at most 30: + 64 keeps the
+        // subtraction inside it
+        const uint32_t back = desc[r] + 64 - (uint32_t)(2 * m);
+        if (want == 0xFFFFFFFFu) want = back;
+        else if (want != back) return false;
+      }
+    }
+  return true;
+}
+
+uint8_t* forms_hi(irs_sharedb* db) { return db->forms + kQuadProducts * (db->n_pad / 4) * (db->code_length / 4); }
+
+// Notes whether the rows about to be expanded are quads, and where the
+// expansion puts their forms and (if it changes) the device flag.  The holders'
+// lock is held until the expansion is enqueued.
+QuadForms begin_forms(irs_sharedb* db, bool quads) {
+  db->quad_rows = quads;
+  QuadForms f{nullptr, nullptr, nullptr, nullptr};
+  if (quads) f = {db->forms, forms_hi(db), db->row_valid, nullptr};
+  if (db->sums && db->flag_set != quads) {
+    f.flag = db->quad_flag;
+    db->flag_set = quads;
+  }
+  return f;
+}
+
+// Planes and forms of a row table whose bases and table are in the staging.
+int expand_row_table(irs_sharedb* db, const uint32_t* desc, size_t n_rows, const uint32_t* d_desc, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  const QuadForms f = begin_forms(db, quad_forms_ready(db) && rows_are_quads(desc, n_rows));
+  CU(launch_expand_rows(db->q_stage, (uint32_t)db->code_length, d_desc, (uint32_t)n_rows, (uint32_t)db->n_pad, db->q_lo,
+                        db->q_hi, f, s));
+  return IRS_OK;
+}
+
 int set_active_rows(irs_sharedb* db, size_t rows) {
   const size_t n = padded_query_rows(rows, db->n_cap);
   if (n > db->n_cap) return fail(IRS_ERR_INVALID, "%zu rows exceed the query capacity %zu", rows, db->n_cap);
+  if (n != db->n_pad) db->quad_rows = false;  // the forms are for another row count; the upload decides
   int bn = gemm_block_n_for((uint32_t)n);
   if (db->tile_override && n % (size_t)db->tile_override == 0) bn = db->tile_override;
   const bool rebuild = bn != db->block_n;
@@ -480,7 +691,7 @@ int irs_device_manager_sm_count(irs_device_manager* dm, int* n) {
 
 int irs_device_alloc(irs_device_manager* dm, size_t bytes, void** ptr) {
   CHECK(dm && ptr, IRS_ERR_INVALID, "bad arguments");
-  cudaError_t e = cudaMalloc(ptr, bytes ? bytes : 16);
+  cudaError_t e = device_malloc(dm, ptr, bytes ? bytes : 16);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(IRS_ERR_NOMEM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
@@ -580,6 +791,7 @@ int irs_sharedb_destroy(irs_sharedb* db) {
   if (!db) return IRS_OK;
   irs_device_manager* dm = db->dm;
   cudaSetDevice(dm->device);
+  drop_sums(db);
   pool_free(dm, db->peer, db->db_lo);
   pool_free(dm, db->peer, db->db_hi);
   pool_free(dm, db->peer, db->q_lo);
@@ -599,6 +811,7 @@ int irs_sharedb_alloc_db(irs_sharedb* db, size_t max_db_length) {
         max_db_length);
   irs_device_manager* dm = db->dm;
   CU(cudaSetDevice(dm->device));
+  drop_sums(db);
   pool_free(dm, db->peer, db->db_lo);
   pool_free(dm, db->peer, db->db_hi);
   db->db_lo = db->db_hi = nullptr;
@@ -616,6 +829,7 @@ int irs_sharedb_alloc_db(irs_sharedb* db, size_t max_db_length) {
   if (make_tmap_u8(&db->tm_db_lo, db->db_lo, cap, db->code_length, 128) ||
       make_tmap_u8(&db->tm_db_hi, db->db_hi, cap, db->code_length, 128))
     return fail(IRS_ERR_CUDA, "tensor map for the DB planes failed");
+  alloc_sums(db);
   CU(cudaStreamSynchronize(dm->streams[db->peer]));
   return IRS_OK;
 }
@@ -633,7 +847,9 @@ int irs_sharedb_load_records(irs_sharedb* db, size_t first, size_t n, const uint
   for (size_t done = 0; done < n;) {
     const size_t c = std::min(per, n - done);
     CU(cudaMemcpyAsync(db->q_stage, records + done * K, c * K * 2, cudaMemcpyHostToDevice, s));
-    CU(launch_split_limbs(db->q_stage, db->db_lo + (first + done) * K, db->db_hi + (first + done) * K, c * K, s));
+    CU(launch_split_limbs(db->q_stage, (uint32_t)K, db->db_lo + (first + done) * K, db->db_hi + (first + done) * K,
+                          c * K, s));
+    CU(update_sums(db, first + done, c, s));
     CU(cudaStreamSynchronize(s));
     done += c;
   }
@@ -649,11 +865,27 @@ int irs_sharedb_load_records_i8(irs_sharedb* db, size_t first, size_t n, const u
   CU(cudaSetDevice(dm->device));
   cudaStream_t s = dm->streams[db->peer];
   const size_t K = db->code_length;
-  CU(cudaMemcpyAsync(db->db_lo + first * K, limb0, n * K, cudaMemcpyHostToDevice, s));
-  CU(cudaMemcpyAsync(db->db_hi + first * K, limb1, n * K, cudaMemcpyHostToDevice, s));
-  CU(launch_xor80(db->db_lo + first * K, n * K, s));
-  CU(launch_xor80(db->db_hi + first * K, n * K, s));
-  CU(cudaStreamSynchronize(s));
+  // through a bounded staging buffer of its own (the query staging may hold a
+  // server's resident bases)
+  const size_t per = std::min<size_t>(n, std::max<size_t>(1, (64u << 20) / K));
+  void* stage = nullptr;
+  int rc = n ? pool_alloc(dm, db->peer, 2 * per * K, &stage) : IRS_OK;
+  if (rc) return rc;
+  uint8_t* st = static_cast<uint8_t*>(stage);
+  cudaError_t e = cudaSuccess;
+  for (size_t done = 0; done < n && e == cudaSuccess;) {
+    const size_t c = std::min(per, n - done), at = (first + done) * K;
+    e = cudaMemcpyAsync(st, limb0 + done * K, c * K, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(st + per * K, limb1 + done * K, c * K, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = launch_i8_plane(st, (uint32_t)K, db->db_lo + at, c * K, s);
+    if (e == cudaSuccess) e = launch_i8_plane(st + per * K, (uint32_t)K, db->db_hi + at, c * K, s);
+    if (e == cudaSuccess) e = update_sums(db, first + done, c, s);
+    done += c;
+  }
+  if (stage) pool_free(dm, db->peer, stage);
+  const cudaError_t sync = cudaStreamSynchronize(s);
+  CU(e);
+  CU(sync);
   db->db_len = std::max(db->db_len, first + n);
   return IRS_OK;
 }
@@ -670,7 +902,12 @@ int irs_sharedb_fetch_records(irs_sharedb* db, size_t first, size_t n, uint16_t*
   CU(cudaMemcpyAsync(lo.data(), db->db_lo + first * K, n * K, cudaMemcpyDeviceToHost, s));
   CU(cudaMemcpyAsync(hi.data(), db->db_hi + first * K, n * K, cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
-  for (size_t i = 0; i < n * K; i++) records[i] = (uint16_t)(lo[i] | (hi[i] << 8));
+  // planes are in quarter order (prep.cu): octet o of a row sits in quarter o % 4
+  for (size_t r = 0; r < n; r++)
+    for (size_t k = 0; k < K; k++) {
+      const size_t o = k / 8, at = r * K + (o % 4) * (K / 4) + o / 4 * 8 + k % 8;
+      records[r * K + k] = (uint16_t)(lo[at] | (hi[at] << 8));
+    }
   return IRS_OK;
 }
 
@@ -710,6 +947,10 @@ int irs_sharedb_synth_db(irs_sharedb* const code_engines[3], irs_sharedb* const 
     const uint32_t c = (uint32_t)std::min(step, n - done);
     CU(launch_synth_db(seed, (uint32_t)(first + done), c, o, dm->streams[0]));
   }
+  for (int p = 0; p < 3; p++) {
+    CU(update_sums(code_engines[p], first, n, dm->streams[0]));
+    CU(update_sums(mask_engines[p], first, n, dm->streams[0]));
+  }
   CU(cudaStreamSynchronize(dm->streams[0]));
   for (int p = 0; p < 3; p++) {
     code_engines[p]->db_len = std::max(code_engines[p]->db_len, first + n);
@@ -734,8 +975,10 @@ int irs_sharedb_fill_random(irs_sharedb* db, uint64_t seed, size_t n) {
   CU(cudaSetDevice(dm->device));
   cudaStream_t s = dm->streams[db->peer];
   CU(wait_last_dot(db, s));
-  CU(launch_fill_random(db->db_lo, n * db->code_length, seed, s));
-  CU(launch_fill_random(db->db_hi, n * db->code_length, seed ^ 0x5A5A5A5A5A5A5A5Aull, s));
+  const uint32_t K = (uint32_t)db->code_length;
+  CU(launch_fill_random(db->db_lo, n * db->code_length, seed, K, s));
+  CU(launch_fill_random(db->db_hi, n * db->code_length, seed ^ 0x5A5A5A5A5A5A5A5Aull, K, s));
+  CU(update_sums(db, 0, n, s));
   CU(cudaStreamSynchronize(s));
   db->db_len = std::max(db->db_len, n);
   return IRS_OK;
@@ -744,7 +987,7 @@ int irs_sharedb_fill_random(irs_sharedb* db, uint64_t seed, size_t n) {
 int irs_device_fill_random(void* ptr, size_t bytes, uint64_t seed, void* stream) {
   CHECK(ptr && bytes % 8 == 0 && reinterpret_cast<uintptr_t>(ptr) % 8 == 0, IRS_ERR_INVALID,
         "8-byte aligned pointer and a multiple of 8 bytes needed");
-  CU(launch_fill_random(ptr, bytes, seed, static_cast<cudaStream_t>(stream)));
+  CU(launch_fill_random(ptr, bytes, seed, 0, static_cast<cudaStream_t>(stream)));
   return IRS_OK;
 }
 
@@ -759,7 +1002,11 @@ int irs_sharedb_query_upload(irs_sharedb* db, const uint16_t* rows, size_t n_row
   const size_t K = db->code_length;
   CU(cudaMemsetAsync(db->q_stage, 0, db->n_pad * K * 2, s));
   if (n_rows) CU(cudaMemcpyAsync(db->q_stage, rows, n_rows * K * 2, cudaMemcpyHostToDevice, s));
-  CU(launch_split_limbs(db->q_stage, db->q_lo, db->q_hi, db->n_pad * K, s));
+  CU(launch_split_limbs(db->q_stage, (uint32_t)K, db->q_lo, db->q_hi, db->n_pad * K, s));
+  {
+    std::lock_guard<std::mutex> lock(sum_holders().mu);
+    if (begin_forms(db, false).flag) CU(cudaMemsetAsync(db->quad_flag, 0, 4, s));  // rows of no known structure
+  }
   db->have_query = true;
   return IRS_OK;
 }
@@ -786,8 +1033,12 @@ int irs_sharedb_query_upload_slots(irs_sharedb* db, const uint16_t* base, size_t
   CU(cudaMemcpyAsync(db->q_stage, base, n_base * K * 2, cudaMemcpyHostToDevice, s));
   static_assert(sizeof(QuerySlot) == sizeof(irs_query_slot), "slot layout");
   CU(cudaMemcpyAsync(db->d_slots, slots, n_slots * sizeof(QuerySlot), cudaMemcpyHostToDevice, s));
-  CU(launch_expand_slots(db->q_stage, (uint32_t)K, db->d_slots, (uint32_t)n_slots, (uint32_t)db->n_pad, db->q_lo,
-                         db->q_hi, s));
+  {
+    std::lock_guard<std::mutex> lock(sum_holders().mu);
+    const QuadForms f = begin_forms(db, quad_forms_ready(db));  // a slot's rows are consecutive rotations
+    CU(launch_expand_slots(db->q_stage, (uint32_t)K, db->d_slots, (uint32_t)n_slots, (uint32_t)db->n_pad, db->q_lo,
+                           db->q_hi, f, s));
+  }
   CU(cudaStreamSynchronize(s));  // slots / base are caller-owned host memory
   db->have_query = true;
   return IRS_OK;
@@ -814,8 +1065,7 @@ int irs_sharedb_query_upload_rows(irs_sharedb* db, const uint16_t* base, size_t 
   const size_t table_off = (base_bytes + 15) / 16 * 16;
   CU(cudaMemcpyAsync(stage, base, base_bytes, cudaMemcpyHostToDevice, s));
   CU(cudaMemcpyAsync(stage + table_off, row_desc, table_bytes, cudaMemcpyHostToDevice, s));
-  CU(launch_expand_rows(db->q_stage, (uint32_t)K, reinterpret_cast<const uint32_t*>(stage + table_off), (uint32_t)n_rows,
-                        (uint32_t)db->n_pad, db->q_lo, db->q_hi, s));
+  if ((rc = expand_row_table(db, row_desc, n_rows, reinterpret_cast<const uint32_t*>(stage + table_off), s))) return rc;
   if (dm->host_sync) CU(cudaStreamSynchronize(s));  // base / row_desc are caller-owned host memory
   db->have_query = true;
   return IRS_OK;
@@ -854,8 +1104,7 @@ int irs_sharedb_query_expand_rows(irs_sharedb* db, size_t n_base, const uint32_t
   uint8_t* stage = reinterpret_cast<uint8_t*>(db->q_stage);
   const size_t table_off = (base_bytes + 15) / 16 * 16;
   CU(cudaMemcpyAsync(stage + table_off, row_desc, table_bytes, cudaMemcpyHostToDevice, s));
-  CU(launch_expand_rows(db->q_stage, (uint32_t)K, reinterpret_cast<const uint32_t*>(stage + table_off), (uint32_t)n_rows,
-                        (uint32_t)db->n_pad, db->q_lo, db->q_hi, s));
+  if ((rc = expand_row_table(db, row_desc, n_rows, reinterpret_cast<const uint32_t*>(stage + table_off), s))) return rc;
   if (dm->host_sync) CU(cudaStreamSynchronize(s));  // row_desc is caller-owned host memory
   db->have_query = true;
   return IRS_OK;
@@ -879,6 +1128,12 @@ int irs_sharedb_gather_records(irs_sharedb* dst, irs_sharedb* src, const uint32_
   CU(cudaMemcpyAsync(dst->q_stage, ids, n * 4, cudaMemcpyHostToDevice, s));
   CU(launch_gather_rows(src->db_lo, src->db_hi, reinterpret_cast<const uint32_t*>(dst->q_stage), (uint32_t)n,
                         (uint32_t)K, dst->db_lo, dst->db_hi, s));
+  if (dst->sums && gather_skips_sums(dst, n)) {
+    dst->stale_end = std::max(dst->stale_end, n);
+  } else {
+    CU(update_sums(dst, 0, n, s));
+    if (n >= dst->stale_end) dst->stale_end = 0;
+  }
   if (dm->host_sync) CU(cudaStreamSynchronize(s));  // ids is caller-owned host memory
   dst->db_len = n;
   return IRS_OK;
@@ -935,6 +1190,48 @@ static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t le
   return IRS_OK;
 }
 
+// The tile width with which a launch over `len` entries can run as the
+// rotation-structured GEMM, or -1: every engine holds sums and form maps, the
+// caller left the GEMM open (no tile width asked for) or chose the two-SM one,
+// and the quad GEMM is expected to take less.  Whether it does run depends on
+// the uploaded rows.
+static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t len) {
+  uint32_t K[kMaxGemmProblems];
+  for (int i = 0; i < n; i++) {
+    const irs_sharedb* e = engines[i];
+    if (!e->sums || e->n_pad != engines[0]->n_pad || e->forms_pad != e->n_pad || offset < e->stale_end) return -1;
+    if (e->tile_override && !gemm_pair_applies(e->pair, e->block_n)) return -1;
+    K[i] = (uint32_t)e->code_length;
+  }
+  const irs_sharedb* e = engines[0];
+  return quad_width_for(K, n, (uint32_t)len, (uint32_t)e->n_pad, e->block_n, gemm_pair_applies(e->pair, e->block_n),
+                        e->dm->n_sms);
+}
+
+static void fill_quad_problem(const irs_sharedb* db, const GemmProblem& g, int width, QuadProblem& pr) {
+  pr.tm_a_lo[0] = db->tm_db_lo;
+  pr.tm_a_hi[0] = db->tm_db_hi;
+  for (int k = 0; k < 2; k++) {
+    pr.tm_a_lo[1 + k] = db->tm_sum_lo[k];
+    pr.tm_a_hi[1 + k] = db->tm_sum_hi[k];
+  }
+  pr.tm_b_lo = db->tm_form_lo[width];
+  pr.tm_b_hi = db->tm_form_hi[width];
+  pr.out = g.out;
+  pr.row_valid = db->row_valid;
+  pr.m0 = g.m0;
+  pr.m_len = g.m_len;
+  pr.n_pad = g.n_pad;
+  pr.quarter = (uint32_t)(db->code_length / 4);
+  pr.mult = g.mult;
+  pr.mask_on = g.mask_on;
+  pr.key_own = g.key_own;
+  pr.key_prev = g.key_prev;
+  pr.nonce = g.nonce;
+  pr.batch = g.batch;
+  pr.batch_dev = g.batch_dev;
+}
+
 int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multipliers, int n, size_t offset, size_t len,
                          void* stream) {
   CHECK(engines && multipliers && n > 0 && n <= kMaxGemmProblems, IRS_ERR_INVALID, "1..6 engines per launch");
@@ -967,7 +1264,31 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
       dm->stall_limit_ns = 0;
     }
     StageTimer timer(dm, s, "dot");
-    CU(launch_limb_gemm(P, engines[0]->block_n, engines[0]->pair, dm->n_sms, s));
+    std::lock_guard<std::mutex> lock(sum_holders().mu);
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(s, &st));
+    const bool captured = st != cudaStreamCaptureStatusNone;
+    // (the quad kernel has no stall hook)
+    const int width = P.test_stall ? -1 : quad_width(engines, n, offset, len);
+    bool quads = width >= 0;
+    for (int i = 0; i < n && !captured; i++) quads = quads && engines[i]->quad_rows;
+    if (quads) {
+      QuadParams Q;
+      memset(&Q, 0, sizeof Q);
+      Q.n_prob = n;
+      Q.err = dm->d_err;
+      Q.tile_n = quad_tile_n((uint32_t)engines[0]->n_pad, width);
+      for (int i = 0; i < n; i++) {
+        fill_quad_problem(engines[i], P.prob[i], width, Q.prob[i]);
+        if (!captured) continue;
+        engines[i]->sums_captured = true;
+        Q.run.word[i] = engines[i]->quad_flag;
+        Q.run.n = n;
+      }
+      P.skip = Q.run;
+      CU(launch_quad_gemm(Q, dm->n_sms, s));
+    }
+    if (!quads || captured) CU(launch_limb_gemm(P, engines[0]->block_n, engines[0]->pair, dm->n_sms, s));
   }
   for (int i = 0; i < n; i++) {
     engines[i]->res_offset = offset;
@@ -1277,7 +1598,7 @@ int irs_dc_init(irs_device_manager* dm, size_t max_queries, size_t max_db_length
       {(void**)&dc->d_take, max_queries * (2 + kMaxMatchesLen) * 4},
   };
   for (auto& a : allocs) {
-    cudaError_t e = cudaMalloc(a.p, a.bytes);
+    cudaError_t e = device_malloc(dm, a.p, a.bytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
       irs_dc_destroy(dc);
@@ -1513,7 +1834,7 @@ int irs_dc_scan_fused(irs_distance_comparator* dc, irs_circuits* c, irs_sharedb*
     dc->ring = nullptr;
     dc->ring_bytes = 0;
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, need);
+    cudaError_t e = device_malloc(dm, &p, need);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(IRS_ERR_NOMEM, "fused scan ring of %zu bytes: %s", need, cudaGetErrorString(e));
@@ -1648,7 +1969,7 @@ int irs_dc_enable_distance_capture(irs_distance_comparator* dc, size_t cap) {
     dc->d_dist = nullptr;
   }
   void* p = nullptr;
-  if (cudaMalloc(&p, dist_bytes(cap)) != cudaSuccess) {
+  if (device_malloc(dm, &p, dist_bytes(cap)) != cudaSuccess) {
     cudaGetLastError();
     return fail(IRS_ERR_NOMEM, "distance capture allocation of %zu bytes failed", dist_bytes(cap));
   }
@@ -1669,7 +1990,7 @@ int irs_dc_set_forced_distances(irs_distance_comparator* dc, const uint32_t* que
   cudaStream_t s = dm->streams[0];
   if (!dc->d_forced) {
     void* p = nullptr;
-    if (cudaMalloc(&p, 2 * kMaxForced * 4) != cudaSuccess) {
+    if (device_malloc(dm, &p, 2 * kMaxForced * 4) != cudaSuccess) {
       cudaGetLastError();
       return fail(IRS_ERR_NOMEM, "forced-pair table allocation failed");
     }

@@ -29,7 +29,9 @@
 #include <stdlib.h>
 #include "common.cuh"
 #include "gemm_limb.h"
+#include "quad_gemm.h"
 #include "tc_sm100.cuh"
+#include "tc_pair.cuh"
 #include "launch_attr.cuh"
 
 namespace irs {
@@ -68,6 +70,7 @@ __device__ __forceinline__ bool tile_of(const GemmParams& P, int t, Tile& out) {
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1) limb_gemm_kernel(const __grid_constant__ GemmParams P) {
   using C = Cfg<BN>;
+  if (P.skip.n && P.skip.all_set()) return;  // the quad GEMM runs; the same words for every CTA
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* a_lo = smem;
@@ -278,61 +281,6 @@ __global__ void __launch_bounds__(kThreads, 1) limb_gemm_kernel(const __grid_con
 // accumulator barriers are released to both CTAs with multicast commits; the
 // follower's epilogue releases the accumulator on the leader's barrier.
 // ---------------------------------------------------------------------------
-constexpr int kBM2 = 256;
-
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-
-__device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-  return r;
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x,
-                                                 int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-      "[%4];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar_cluster_addr)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_u8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate));
-}
-
-// Arrives on the barrier at the same offset in both CTAs of the pair once the
-// leader's preceding MMAs have completed.
-__device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
-  const uint16_t mask = 0x3;
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "h"(mask)
-      : "memory");
-}
-
-__host__ __device__ constexpr uint32_t idesc_u8_m256(int bn) {
-  return (2u << 4) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kBM2 >> 4) << 24);
-}
-
 struct Cfg2 {
   static constexpr int BN = 256;
   static constexpr int kHalfN = BN / 2;
@@ -361,6 +309,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     limb_gemm_pair_kernel(const __grid_constant__ GemmParams P) {
   using C = Cfg2;
   constexpr int BN = C::BN;
+  if (P.skip.n && P.skip.all_set()) return;  // the quad GEMM runs; the same words for every CTA
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* a_lo = smem;
@@ -573,10 +522,10 @@ EncodeTiledFn encode_fn() {
 
 }  // namespace
 
-int make_tmap_u8(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k, uint32_t box_rows) {
+int make_tmap_plane(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k, uint32_t box_rows) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return -1;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (k % kBK) || box_rows > 256) return -2;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (k % 16) || box_rows > 256) return -2;
   cuuint64_t dims[2] = {k, rows};
   cuuint64_t strides[1] = {k};
   cuuint32_t box[2] = {(cuuint32_t)kBK, box_rows};
@@ -585,6 +534,10 @@ int make_tmap_u8(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k, 
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -3;
+}
+
+int make_tmap_u8(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k, uint32_t box_rows) {
+  return k % kBK ? -2 : make_tmap_plane(map, base, rows, k, box_rows);
 }
 
 template <int BN>

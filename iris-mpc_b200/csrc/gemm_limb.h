@@ -31,10 +31,27 @@ struct alignas(64) GemmProblem {
 };
 
 constexpr int kMaxGemmProblems = 6;
+// Device words that are nonzero while an engine's uploaded rows are quads of
+// rotations.  A captured launch holds both GEMMs, since later uploads decide
+// which one a replay needs: the quad GEMM runs when all words are set, the
+// plain one when not.
+struct QuadFlags {
+  const uint32_t* word[kMaxGemmProblems];
+  int n;  // 0: not captured, no check
+#ifdef __CUDACC__
+  __device__ __forceinline__ bool all_set() const {
+    bool all = true;
+    for (int i = 0; i < n; i++) all = all && *word[i] != 0;
+    return all;
+  }
+#endif
+};
+
 constexpr uint64_t kGemmWaitTimeoutNs = 2000000000ull;  // default limit of a bounded wait: 2 s
 
 struct GemmParams {
   GemmProblem prob[kMaxGemmProblems];
+  QuadFlags skip;  // the launch does nothing when they are all set
   int n_prob;
   int total_tiles;
   int* err;

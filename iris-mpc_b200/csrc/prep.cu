@@ -8,6 +8,12 @@
 // Rotations: row r of a query slot is all_rotations()[r] of the query share,
 // i.e. every 800-coefficient row rotated left by 4*(15 - r) coefficients
 // (iris-mpc-common/src/galois_engine.rs:42-52,197-206).
+//
+// Limb planes, of records and of query rows alike, hold a row's K coefficients
+// as four quarters: each group of 32 consecutive coefficients (8 columns)
+// gives its q-th 8 to quarter q, so quarter 2o + n holds the columns with bit 2
+// (value 4) = o and bit 1 (value 2) = n, which is how the rotation-structured
+// GEMM (quad_gemm.cu) splits them.  A dot product does not depend on the order.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "common.cuh"
@@ -17,92 +23,220 @@ namespace irs {
 
 namespace {
 
-__global__ void split_limbs_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ lo,
-                                   uint8_t* __restrict__ hi, size_t n4) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n4) return;
-  const uint2 v = reinterpret_cast<const uint2*>(in)[i];  // 4 u16
-  const uint32_t l = (v.x & 0xFFu) | ((v.x >> 8) & 0xFF00u) | ((v.y & 0xFFu) << 16) | ((v.y & 0xFF0000u) << 8);
-  const uint32_t h = ((v.x >> 8) & 0xFFu) | ((v.x >> 16) & 0xFF00u) | ((v.y & 0xFF00u) << 8) | (v.y & 0xFF000000u);
-  reinterpret_cast<uint32_t*>(lo)[i] = l;
-  reinterpret_cast<uint32_t*>(hi)[i] = h;
+// Position in a plane row of the octet (8 coefficients) o of the record order.
+__device__ __forceinline__ uint32_t plane_octet(uint32_t o, uint32_t K) { return (o & 3u) * (K / 32) + (o >> 2); }
+
+// The same for a block of 4 coefficients.
+__device__ __forceinline__ uint32_t plane_block(uint32_t b, uint32_t K) {
+  return 2 * plane_octet(b >> 1, K) + (b & 1u);
 }
 
-__global__ void xor80_kernel(uint8_t* __restrict__ p, size_t n16) {
+// The low and the high bytes of four u16.
+__device__ __forceinline__ uint32_t low_bytes(uint2 v) { return __byte_perm(v.x, v.y, 0x6420); }
+__device__ __forceinline__ uint32_t high_bytes(uint2 v) { return __byte_perm(v.x, v.y, 0x7531); }
+
+// One thread per octet of `n8` (rows of K coefficients).
+__global__ void split_limbs_kernel(const uint16_t* __restrict__ in, uint32_t K, uint8_t* __restrict__ lo,
+                                   uint8_t* __restrict__ hi, size_t n8) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n16) return;
-  uint4 v = reinterpret_cast<uint4*>(p)[i];
-  v.x ^= 0x80808080u; v.y ^= 0x80808080u; v.z ^= 0x80808080u; v.w ^= 0x80808080u;
-  reinterpret_cast<uint4*>(p)[i] = v;
+  if (i >= n8) return;
+  const uint4 v = reinterpret_cast<const uint4*>(in)[i];
+  const uint2 a = make_uint2(v.x, v.y), b = make_uint2(v.z, v.w);
+  const uint32_t per = K / 8;
+  const size_t d = i / per * per + plane_octet((uint32_t)(i % per), K);
+  reinterpret_cast<uint2*>(lo)[d] = make_uint2(low_bytes(a), low_bytes(b));
+  reinterpret_cast<uint2*>(hi)[d] = make_uint2(high_bytes(a), high_bytes(b));
 }
 
-// One thread per (slot row, 4-coefficient block).  Slot s row r holds
-// rotation rot_lo[s] + r of query slot_src[s] for r < n_rot[s]; other rows 0.
-// mirror_flags bit s: use the mirrored query (already mirrored on the host).
-__global__ void expand_slots_kernel(const uint16_t* __restrict__ base, uint32_t K, const QuerySlot* __restrict__ slots,
-                                    uint32_t n_slots, uint32_t n_pad, uint8_t* __restrict__ lo,
-                                    uint8_t* __restrict__ hi) {
-  const uint32_t blocks_per_row = K / 4;
+// Stored i8 limbs (byte - 128) in record order to a plane, one thread per octet.
+__global__ void i8_plane_kernel(const uint8_t* __restrict__ in, uint32_t K, uint8_t* __restrict__ out, size_t n8) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t total = (size_t)n_pad * blocks_per_row;
-  if (i >= total) return;
-  const uint32_t row = (uint32_t)(i / blocks_per_row);
-  const uint32_t b = (uint32_t)(i % blocks_per_row);
-  const uint32_t s = row / kSlotRows, r = row % kSlotRows;
-  uint32_t l = 0, h = 0;
-  if (s < n_slots && r < slots[s].n_rot) {
-    const QuerySlot sl = slots[s];
-    const int rot = (int)sl.rot_lo + (int)r;  // index into all_rotations, 15 = centre
-    const int left_blocks = 15 - rot;         // net left rotation in 4-coef blocks
-    const uint32_t row800 = b / 200, col = b % 200;
-    const uint32_t src_col = (uint32_t)(((int)col + left_blocks % 200 + 200) % 200);
-    const uint16_t* src = base + (size_t)sl.src * K + (size_t)row800 * kRowLen + (size_t)src_col * 4;
-    const uint2 v = *reinterpret_cast<const uint2*>(src);
-    l = (v.x & 0xFFu) | ((v.x >> 8) & 0xFF00u) | ((v.y & 0xFFu) << 16) | ((v.y & 0xFF0000u) << 8);
-    h = ((v.x >> 8) & 0xFFu) | ((v.x >> 16) & 0xFF00u) | ((v.y & 0xFF00u) << 8) | (v.y & 0xFF000000u);
+  if (i >= n8) return;
+  const uint2 v = reinterpret_cast<const uint2*>(in)[i];
+  const uint32_t per = K / 8;
+  reinterpret_cast<uint2*>(out)[i / per * per + plane_octet((uint32_t)(i % per), K)] =
+      make_uint2(v.x ^ 0x80808080u, v.y ^ 0x80808080u);
+}
+
+// Bytewise sums of two u16 vectors given as limb words: (al, ah) + (bl, bh).
+__device__ __forceinline__ void add_limbs(uint32_t al, uint32_t ah, uint32_t bl, uint32_t bh, uint32_t& sl,
+                                          uint32_t& sh) {
+  sl = __vadd4(al, bl);
+  const uint32_t carry = __vcmpltu4(sl, al) & 0x01010101u;
+  sh = __vadd4(__vadd4(ah, bh), carry);
+}
+__device__ __forceinline__ void add_limbs(const uint4& al, const uint4& ah, const uint4& bl, const uint4& bh, uint4& sl,
+                                          uint4& sh) {
+  add_limbs(al.x, ah.x, bl.x, bh.x, sl.x, sh.x);
+  add_limbs(al.y, ah.y, bl.y, bh.y, sl.y, sh.y);
+  add_limbs(al.z, ah.z, bl.z, bh.z, sl.z, sh.z);
+  add_limbs(al.w, ah.w, bl.w, bh.w, sl.w, sh.w);
+}
+
+// The sums of a record's quarters that the rotation-structured GEMM reads:
+// outer = (q0 + q2, q1 + q3), inner = (all four, q0 + q1, q2 + q3).  One
+// thread per 16 coefficients of a quarter; bound by HBM (2 bytes read and 2.5
+// written per coefficient).
+__global__ void derive_sums_kernel(const uint8_t* __restrict__ lo, const uint8_t* __restrict__ hi, uint32_t K, size_t n,
+                                   uint8_t* __restrict__ outer_lo, uint8_t* __restrict__ outer_hi,
+                                   uint8_t* __restrict__ inner_lo, uint8_t* __restrict__ inner_hi) {
+  const uint32_t per = K / 64, Q = K / 4;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n * per) return;
+  const size_t row = i / per;
+  const uint32_t x = (uint32_t)(i % per) * 16;
+  uint4 l[4], h[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    l[q] = *reinterpret_cast<const uint4*>(lo + row * K + q * Q + x);
+    h[q] = *reinterpret_cast<const uint4*>(hi + row * K + q * Q + x);
   }
-  reinterpret_cast<uint32_t*>(lo)[i] = l;
-  reinterpret_cast<uint32_t*>(hi)[i] = h;
+  auto put = [&](uint8_t* pl, uint8_t* ph, size_t at, const uint4& sl, const uint4& sh) {
+    *reinterpret_cast<uint4*>(pl + at) = sl;
+    *reinterpret_cast<uint4*>(ph + at) = sh;
+  };
+  uint4 s0l, s0h, s1l, s1h, tl, th;
+  add_limbs(l[0], h[0], l[2], h[2], s0l, s0h);
+  add_limbs(l[1], h[1], l[3], h[3], s1l, s1h);
+  put(outer_lo, outer_hi, row * 2 * Q + x, s0l, s0h);
+  put(outer_lo, outer_hi, row * 2 * Q + Q + x, s1l, s1h);
+  add_limbs(s0l, s0h, s1l, s1h, tl, th);
+  put(inner_lo, inner_hi, row * 3 * Q + x, tl, th);
+  add_limbs(l[0], h[0], l[1], h[1], tl, th);
+  put(inner_lo, inner_hi, row * 3 * Q + Q + x, tl, th);
+  add_limbs(l[2], h[2], l[3], h[3], tl, th);
+  put(inner_lo, inner_hi, row * 3 * Q + 2 * Q + x, tl, th);
 }
 
-// One thread per (row, 4-coefficient block).  row_desc[r] = (src << 8) |
-// mirror << 7 | rot puts rotation `rot` (0..30, 15 = centre) of base query
-// `src` in row r, of its mirrored form when the mirror bit is set;
-// 0xFFFFFFFF leaves the row zero.  Lets a batch pack queries with different
-// rotation counts densely (no 32-row slot per query).
+// The query source of a row: base query, mirror bit, rotation index into
+// all_rotations() (15 = centre).
+struct RowSource {
+  uint32_t src;
+  bool mirror, live;
+  int rot;
+};
+
+// Row sources of a slot list: slot s row r holds rotation rot_lo[s] + r of
+// query src[s] for r < n_rot[s]; other rows are zero.
+struct SlotRows {
+  const QuerySlot* slots;
+  uint32_t n_slots;
+  __device__ RowSource operator()(uint32_t row) const {
+    const uint32_t s = row / kSlotRows, r = row % kSlotRows;
+    if (s >= n_slots || r >= slots[s].n_rot) return {0u, false, false, 0};
+    return {slots[s].src, false, true, (int)(slots[s].rot_lo + r)};
+  }
+};
+
+// Row sources of a row table: desc[r] = (src << 8) | mirror << 7 | rot puts
+// rotation `rot` (0..30) of base query `src` in row r, of its mirrored form
+// when the mirror bit is set; 0xFFFFFFFF leaves the row zero.  Lets a batch
+// pack queries with different rotation counts densely (no 32-row slot per
+// query).
+struct TableRows {
+  const uint32_t* desc;
+  uint32_t n_rows;
+  __device__ RowSource operator()(uint32_t row) const {
+    const uint32_t d = row < n_rows ? desc[row] : 0xFFFFFFFFu;
+    if (d == 0xFFFFFFFFu) return {0u, false, false, 0};
+    return {d >> 8, (d & 0x80u) != 0, true, (int)(d & 0x7Fu)};
+  }
+};
+
+// Column `col` (any integer above -400) of 800-coefficient row `row800` of the
+// row source's query, rotation not applied.
 //
 // Mirror (mirrored_code / mirrored_mask of the query share,
 // iris-mpc-common/src/galois_engine.rs:218-225,520-543): 4-coefficient
 // column c of each 800-coefficient row moves to 99 - c (c < 100) or 299 - c
 // (c >= 100), and a code share's imaginary half (rows 8..15) is negated.
-// The column map is its own inverse, so rotated row column `col` reads base
-// column mirror((col + left) mod 200).
-__global__ void expand_rows_kernel(const uint16_t* __restrict__ base, uint32_t K, const uint32_t* __restrict__ row_desc,
-                                   uint32_t n_rows, uint32_t n_pad, uint8_t* __restrict__ lo, uint8_t* __restrict__ hi) {
-  const uint32_t blocks_per_row = K / 4;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (size_t)n_pad * blocks_per_row) return;
-  const uint32_t row = (uint32_t)(i / blocks_per_row);
-  const uint32_t b = (uint32_t)(i % blocks_per_row);
-  uint32_t l = 0, h = 0;
-  const uint32_t d = row < n_rows ? row_desc[row] : 0xFFFFFFFFu;
-  if (d != 0xFFFFFFFFu) {
-    const uint32_t src = d >> 8, rot = d & 0x7Fu;
-    const bool mirror = (d & 0x80u) != 0;
-    const int left_blocks = 15 - (int)rot;
-    const uint32_t row800 = b / 200, col = b % 200;
-    uint32_t src_col = (uint32_t)(((int)col + left_blocks % 200 + 200) % 200);
-    if (mirror) src_col = src_col < 100 ? 99 - src_col : 299 - src_col;
-    uint2 v = *reinterpret_cast<const uint2*>(base + (size_t)src * K + (size_t)row800 * kRowLen + (size_t)src_col * 4);
-    if (mirror && row800 >= 8) {  // imaginary half: only code shares reach it
-      v.x = sub2(0u, v.x);
-      v.y = sub2(0u, v.y);
+// The column map is its own inverse.
+__device__ __forceinline__ uint2 query_column(const uint16_t* __restrict__ base, uint32_t K, const RowSource& q,
+                                              uint32_t row800, int col) {
+  uint32_t c = (uint32_t)(col + 400) % 200u;
+  if (q.mirror) c = c < 100 ? 99 - c : 299 - c;
+  uint2 v = *reinterpret_cast<const uint2*>(base + (size_t)q.src * K + (size_t)row800 * kRowLen + (size_t)c * 4);
+  if (q.mirror && row800 >= 8) v = make_uint2(sub2(0u, v.x), sub2(0u, v.y));  // only code shares reach it
+  return v;
+}
+
+__device__ __forceinline__ void put_octet(uint8_t* lo, uint8_t* hi, size_t at, uint2 a, uint2 b) {
+  reinterpret_cast<uint2*>(lo)[at] = make_uint2(low_bytes(a), low_bytes(b));
+  reinterpret_cast<uint2*>(hi)[at] = make_uint2(high_bytes(a), high_bytes(b));
+}
+
+// The query planes of n_pad rows and, when `quads.lo` is set, the query forms
+// of the rotation-structured GEMM beside them (blocks from plain_blocks on).
+//
+// Planes: one thread per (row, octet).  A rotated row's column c reads base
+// column c + 15 - rot (mod 200).
+//
+// Forms (quad_gemm.cu): planes [9 products][n_pad / 4 quads][K / 4], one thread
+// per (quad, octet of a quarter).  Quad s of a slot is rows i, i + 2, i + 4,
+// i + 6 with i = 16 s2 + 8 s1 + s0 (the bits of s); its live rows are rotations
+// of one query that keep their distance (the caller checked), so row i stands
+// for rotation `rot` even where it is not live itself.  With f(k) the query at
+// column offset c - rot shifted by 2k columns (column c of quarter 0), the
+// forms are the outer and inner differences x: f(+D) - f, y: f(-D) - f at D = 4
+// and D = 2, "2": f itself.  Quads without a live row are zero.
+template <class Rows>
+__global__ void expand_kernel(const uint16_t* __restrict__ base, uint32_t K, Rows rows, uint32_t n_pad,
+                              uint8_t* __restrict__ lo, uint8_t* __restrict__ hi, uint32_t plain_blocks, QuadForms quads) {
+  if (blockIdx.x < plain_blocks) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t per = K / 8;
+    if (i == 0 && quads.flag) *quads.flag = quads.lo ? 1u : 0u;
+    if (i >= (size_t)n_pad * per) return;
+    const uint32_t row = (uint32_t)(i / per), o = (uint32_t)(i % per);
+    const RowSource q = rows(row);
+    uint2 a = make_uint2(0u, 0u), b = a;
+    if (q.live) {
+      const uint32_t row800 = o / 100;
+      const int col = (int)(o % 100) * 2 + 15 - q.rot;
+      a = query_column(base, K, q, row800, col);
+      b = query_column(base, K, q, row800, col + 1);
     }
-    l = (v.x & 0xFFu) | ((v.x >> 8) & 0xFF00u) | ((v.y & 0xFFu) << 16) | ((v.y & 0xFF0000u) << 8);
-    h = ((v.x >> 8) & 0xFFu) | ((v.x >> 16) & 0xFF00u) | ((v.y & 0xFF00u) << 8) | (v.y & 0xFF000000u);
+    put_octet(lo, hi, (size_t)row * per + plane_octet(o, K), a, b);
+    return;
   }
-  reinterpret_cast<uint32_t*>(lo)[i] = l;
-  reinterpret_cast<uint32_t*>(hi)[i] = h;
+  const size_t i = (size_t)(blockIdx.x - plain_blocks) * blockDim.x + threadIdx.x;
+  const uint32_t per = K / 32, n_quads = n_pad / 4;
+  if (i >= (size_t)n_quads * per) return;
+  const uint32_t p = (uint32_t)(i / per), g = (uint32_t)(i % per);
+  if (g == 0 && (p & 7u) == 0) {  // the rows of this slot that hold a query row
+    uint32_t bits = 0;
+    for (uint32_t r = 0; r < (uint32_t)kSlotRows; r++) bits |= (uint32_t)rows((p >> 3) * kSlotRows + r).live << r;
+    quads.valid[p >> 3] = bits;
+  }
+  const uint32_t row0 = (p >> 3) * kSlotRows + ((p >> 2) & 1u) * 16 + ((p >> 1) & 1u) * 8 + (p & 1u);
+  RowSource q{0u, false, false, 0};
+#pragma unroll
+  for (int m = 3; m >= 0; m--) {
+    const RowSource r = rows(row0 + 2 * m);
+    if (r.live) q = {r.src, r.mirror, true, r.rot - 2 * m};
+  }
+  uint2 f[7][2];  // f(k - 3), the octet's two columns
+#pragma unroll
+  for (int k = 0; k < 7; k++)
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+      f[k][c] = q.live ? query_column(base, K, q, g / 25, (int)(g % 25) * 8 + c + 2 * (k - 3) + 15 - q.rot)
+                       : make_uint2(0u, 0u);
+#pragma unroll
+  for (int j = 0; j < 9; j++) {
+    // terms of product j (outer, inner) = 22 2x 2y x2 xx xy y2 yx yy
+    const int o = j / 3 == 0 ? 0 : (j / 3 == 1 ? 2 : -2), n = j % 3 == 0 ? 0 : (j % 3 == 1 ? 1 : -1);
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      auto at = [&](int k) { return (e & 1) ? f[k + 3][e >> 1].y : f[k + 3][e >> 1].x; };
+      uint32_t v = at(0);
+      if (n) v = sub2(at(n), v);
+      if (o) v = sub2(n ? sub2(at(o + n), at(o)) : at(o), v);
+      w[e] = v;
+    }
+    put_octet(quads.lo, quads.hi, ((size_t)j * n_quads + p) * per + g, make_uint2(w[0], w[1]), make_uint2(w[2], w[3]));
+  }
 }
 
 // Copies DB rows ids[k] of (src_lo, src_hi) into rows k of (dst_lo, dst_hi),
@@ -148,12 +282,14 @@ __device__ __forceinline__ void gr4_mul(const uint32_t a[4], const uint32_t b[4]
 // probability 0.9, share randomness r = rng64(share seed, block)).
 // Seeded uniform bytes (splitmix64 of the 8-byte word index): random shares
 // for benchmark buffers whose values do not matter, only their bit activity.
-__global__ void fill_random_kernel(uint64_t* __restrict__ p, size_t n_words, uint64_t seed) {
+// With K > 0 the words go to a limb plane of rows of K in record order.
+__global__ void fill_random_kernel(uint64_t* __restrict__ p, size_t n_words, uint64_t seed, uint32_t K) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += (size_t)gridDim.x * blockDim.x) {
     uint64_t z = seed + (i + 1) * 0x9E3779B97F4A7C15ull;
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    p[i] = z ^ (z >> 31);
+    const size_t d = K ? i / (K / 8) * (K / 8) + plane_octet((uint32_t)(i % (K / 8)), K) : i;
+    p[d] = z ^ (z >> 31);
   }
 }
 
@@ -207,8 +343,9 @@ __global__ void synth_db_kernel(uint64_t seed, uint32_t first, uint32_t count, S
         const size_t K = which == 0 ? (size_t)kIrisCodeLength : (size_t)kMaskCodeLength;
         uint8_t* plo = which == 0 ? out.code_lo[p] : out.mask_lo[p];
         uint8_t* phi = which == 0 ? out.code_hi[p] : out.mask_hi[p];
-        reinterpret_cast<uint32_t*>(plo + (size_t)e * K)[blk] = lo;
-        reinterpret_cast<uint32_t*>(phi + (size_t)e * K)[blk] = hi;
+        const uint32_t at = plane_block((uint32_t)blk, (uint32_t)K);
+        reinterpret_cast<uint32_t*>(plo + (size_t)e * K)[at] = lo;
+        reinterpret_cast<uint32_t*>(phi + (size_t)e * K)[at] = hi;
       }
     }
   }
@@ -216,36 +353,51 @@ __global__ void synth_db_kernel(uint64_t seed, uint32_t first, uint32_t count, S
 
 }  // namespace
 
-cudaError_t launch_split_limbs(const uint16_t* in, uint8_t* lo, uint8_t* hi, size_t n, cudaStream_t stream) {
-  if (n % 4) return cudaErrorInvalidValue;
-  const size_t n4 = n / 4;
-  if (!n4) return cudaSuccess;
-  split_limbs_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, stream>>>(in, lo, hi, n4);
+cudaError_t launch_split_limbs(const uint16_t* in, uint32_t K, uint8_t* lo, uint8_t* hi, size_t n,
+                               cudaStream_t stream) {
+  if (n % 8) return cudaErrorInvalidValue;
+  const size_t n8 = n / 8;
+  if (!n8) return cudaSuccess;
+  split_limbs_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(in, K, lo, hi, n8);
   return cudaGetLastError();
 }
 
-cudaError_t launch_xor80(uint8_t* p, size_t n, cudaStream_t stream) {
-  if (n % 16) return cudaErrorInvalidValue;
-  const size_t n16 = n / 16;
-  if (!n16) return cudaSuccess;
-  xor80_kernel<<<(unsigned)((n16 + 255) / 256), 256, 0, stream>>>(p, n16);
+cudaError_t launch_i8_plane(const uint8_t* in, uint32_t K, uint8_t* out, size_t n, cudaStream_t stream) {
+  if (n % 8) return cudaErrorInvalidValue;
+  const size_t n8 = n / 8;
+  if (!n8) return cudaSuccess;
+  i8_plane_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(in, K, out, n8);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_derive_sums(const uint8_t* lo, const uint8_t* hi, uint32_t K, size_t n, uint8_t* outer_lo,
+                               uint8_t* outer_hi, uint8_t* inner_lo, uint8_t* inner_hi, cudaStream_t stream) {
+  if (K % 64) return cudaErrorInvalidValue;
+  const size_t total = n * (K / 64);
+  if (!total) return cudaSuccess;
+  derive_sums_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(lo, hi, K, n, outer_lo, outer_hi, inner_lo,
+                                                                          inner_hi);
+  return cudaGetLastError();
+}
+
+template <class Rows>
+static cudaError_t launch_expand(const uint16_t* base, uint32_t K, Rows rows, uint32_t n_pad, uint8_t* lo, uint8_t* hi,
+                                 const QuadForms& quads, cudaStream_t stream) {
+  const size_t plain = ((size_t)n_pad * (K / 8) + 255) / 256;
+  const size_t forms = quads.lo ? ((size_t)(n_pad / 4) * (K / 32) + 255) / 256 : 0;
+  if (!plain) return cudaSuccess;
+  expand_kernel<<<(unsigned)(plain + forms), 256, 0, stream>>>(base, K, rows, n_pad, lo, hi, (uint32_t)plain, quads);
   return cudaGetLastError();
 }
 
 cudaError_t launch_expand_slots(const uint16_t* base, uint32_t K, const QuerySlot* slots, uint32_t n_slots,
-                                uint32_t n_pad, uint8_t* lo, uint8_t* hi, cudaStream_t stream) {
-  const size_t total = (size_t)n_pad * (K / 4);
-  if (!total) return cudaSuccess;
-  expand_slots_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(base, K, slots, n_slots, n_pad, lo, hi);
-  return cudaGetLastError();
+                                uint32_t n_pad, uint8_t* lo, uint8_t* hi, const QuadForms& quads, cudaStream_t stream) {
+  return launch_expand(base, K, SlotRows{slots, n_slots}, n_pad, lo, hi, quads, stream);
 }
 
 cudaError_t launch_expand_rows(const uint16_t* base, uint32_t K, const uint32_t* row_desc, uint32_t n_rows,
-                               uint32_t n_pad, uint8_t* lo, uint8_t* hi, cudaStream_t stream) {
-  const size_t total = (size_t)n_pad * (K / 4);
-  if (!total) return cudaSuccess;
-  expand_rows_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(base, K, row_desc, n_rows, n_pad, lo, hi);
-  return cudaGetLastError();
+                               uint32_t n_pad, uint8_t* lo, uint8_t* hi, const QuadForms& quads, cudaStream_t stream) {
+  return launch_expand(base, K, TableRows{row_desc, n_rows}, n_pad, lo, hi, quads, stream);
 }
 
 cudaError_t launch_gather_rows(const uint8_t* src_lo, const uint8_t* src_hi, const uint32_t* ids, uint32_t n,
@@ -256,11 +408,11 @@ cudaError_t launch_gather_rows(const uint8_t* src_lo, const uint8_t* src_hi, con
   return cudaGetLastError();
 }
 
-cudaError_t launch_fill_random(void* p, size_t bytes, uint64_t seed, cudaStream_t stream) {
+cudaError_t launch_fill_random(void* p, size_t bytes, uint64_t seed, uint32_t K, cudaStream_t stream) {
   const size_t n = bytes / 8;
   if (n) {
     const size_t blocks = (n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16;
-    fill_random_kernel<<<(unsigned)blocks, 256, 0, stream>>>(static_cast<uint64_t*>(p), n, seed);
+    fill_random_kernel<<<(unsigned)blocks, 256, 0, stream>>>(static_cast<uint64_t*>(p), n, seed, K);
   }
   return cudaGetLastError();
 }
