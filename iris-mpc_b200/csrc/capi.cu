@@ -150,6 +150,7 @@ struct irs_sharedb {
   CUtensorMap tm_sum_lo[2]{}, tm_sum_hi[2]{}, tm_form_lo[kQuadWidths]{},
       tm_form_hi[kQuadWidths]{};
   CUtensorMap tm_db_lo{}, tm_db_hi{}, tm_q_lo{}, tm_q_hi{};
+  CUtensorMap tm_qh_lo{}, tm_qh_hi{};  // half a 256-row tile, for the two-SM GEMM
   int block_n = 0;
   cudaEvent_t done = nullptr;  // recorded after the engine's last dot launch
 };
@@ -294,9 +295,11 @@ ChaChaKey key_of(const uint32_t k[8]) {
 // a query tile per CTA).
 int rebuild_query_maps(irs_sharedb* db) {
   if (db->block_n <= 0) return IRS_OK;  // no valid tile width: dot reports it
-  const uint32_t q_box = (uint32_t)(gemm_pair_applies(db->pair, db->block_n) ? db->block_n / 2 : db->block_n);
-  if (make_tmap_u8(&db->tm_q_lo, db->q_lo, db->n_cap, db->code_length, q_box) ||
-      make_tmap_u8(&db->tm_q_hi, db->q_hi, db->n_cap, db->code_length, q_box))
+  const uint32_t box = (uint32_t)db->block_n;
+  if (make_tmap_u8(&db->tm_q_lo, db->q_lo, db->n_cap, db->code_length, box) ||
+      make_tmap_u8(&db->tm_q_hi, db->q_hi, db->n_cap, db->code_length, box) ||
+      make_tmap_u8(&db->tm_qh_lo, db->q_lo, db->n_cap, db->code_length, box / 2) ||
+      make_tmap_u8(&db->tm_qh_hi, db->q_hi, db->n_cap, db->code_length, box / 2))
     return fail(IRS_ERR_CUDA, "tensor map for the query planes failed");
   return IRS_OK;
 }
@@ -1150,9 +1153,8 @@ int irs_sharedb_set_tile(irs_sharedb* db, int block_n) {
 
 int irs_sharedb_set_pair(irs_sharedb* db, int on) {
   CHECK(db, IRS_ERR_INVALID, "db is NULL");
-  const bool rebuild = db->pair != (on != 0) && db->block_n == 256;
   db->pair = on != 0;
-  return rebuild ? rebuild_query_maps(db) : IRS_OK;
+  return IRS_OK;
 }
 
 int irs_sharedb_set_batch(irs_sharedb* db, uint64_t batch_id) {
@@ -1162,7 +1164,7 @@ int irs_sharedb_set_batch(irs_sharedb* db, uint64_t batch_id) {
   return IRS_OK;
 }
 
-static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t len, GemmProblem& pr) {
+static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t len, bool pair, GemmProblem& pr) {
   CHECK(db->db_lo, IRS_ERR_STATE, "alloc_db not called");
   CHECK(db->have_query, IRS_ERR_STATE, "no query uploaded");
   CHECK(offset % 32 == 0, IRS_ERR_INVALID, "offset %zu must be a multiple of 32", offset);
@@ -1172,8 +1174,8 @@ static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t le
   memset(&pr, 0, sizeof pr);
   pr.tm_a_lo = db->tm_db_lo;
   pr.tm_a_hi = db->tm_db_hi;
-  pr.tm_b_lo = db->tm_q_lo;
-  pr.tm_b_hi = db->tm_q_hi;
+  pr.tm_b_lo = pair ? db->tm_qh_lo : db->tm_q_lo;
+  pr.tm_b_hi = pair ? db->tm_qh_hi : db->tm_q_hi;
   pr.out = db->results;
   pr.m0 = (uint32_t)offset;
   pr.m_len = (uint32_t)len;
@@ -1195,7 +1197,7 @@ static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t le
 // caller left the GEMM open (no tile width asked for) or chose the two-SM one,
 // and the quad GEMM is expected to take less.  Whether it does run depends on
 // the uploaded rows.
-static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t len) {
+static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t len, bool pair) {
   uint32_t K[kMaxGemmProblems];
   for (int i = 0; i < n; i++) {
     const irs_sharedb* e = engines[i];
@@ -1204,8 +1206,20 @@ static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t 
     K[i] = (uint32_t)e->code_length;
   }
   const irs_sharedb* e = engines[0];
-  return quad_width_for(K, n, (uint32_t)len, (uint32_t)e->n_pad, e->block_n, gemm_pair_applies(e->pair, e->block_n),
-                        e->dm->n_sms);
+  return quad_width_for(K, n, (uint32_t)len, (uint32_t)e->n_pad, e->block_n, pair, e->dm->n_sms);
+}
+
+// Whether the plain GEMM of a launch runs on SM pairs: where the caller chose
+// it, and, where the caller left the GEMM open, for launches short enough that
+// the clock has not dropped to the power limit.  One engine x 960 rows x 32,768
+// entries: 0.73 ms, one-SM 0.81; 1984 rows 1.51 / 1.60; 832 rows 0.70 / 0.78.
+// Six engines x 1024 rows x 32,768 entries: 3.79 / 3.69.
+static bool plain_pair(irs_sharedb* const* engines, int n, size_t len) {
+  const irs_sharedb* e = engines[0];
+  if (e->pair || e->tile_override || e->block_n != 256) return gemm_pair_applies(e->pair, e->block_n);
+  double macs = 0;
+  for (int i = 0; i < n; i++) macs += 3.0 * (double)engines[i]->code_length * (double)e->n_pad * (double)len;
+  return macs < 3e12;  // about 2 ms
 }
 
 static void fill_quad_problem(const irs_sharedb* db, const GemmProblem& g, int width, QuadProblem& pr) {
@@ -1245,7 +1259,12 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
     CHECK(engines[i] && engines[i]->dm == dm, IRS_ERR_INVALID, "engine %d missing or on another device", i);
     CHECK(engines[i]->block_n == engines[0]->block_n, IRS_ERR_INVALID, "engines need the same padded query length");
     CHECK(engines[i]->pair == engines[0]->pair, IRS_ERR_INVALID, "engines need the same GEMM variant (set_pair)");
-    int rc = fill_problem(engines[i], multipliers[i], offset, len, P.prob[i]);
+  }
+  // the stall hook is the one-SM kernel's
+  const bool stall = len && dm->stall_limit_ns && !dm->capturing;
+  const bool pair = !stall && plain_pair(engines, n, len);
+  for (int i = 0; i < n; i++) {
+    int rc = fill_problem(engines[i], multipliers[i], offset, len, pair, P.prob[i]);
     if (rc) return rc;
   }
   cudaStream_t s = party_stream(dm, engines[0]->peer, stream);
@@ -1258,7 +1277,7 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
       CU(cudaStreamWaitEvent(s, engines[i]->done, 0));
     }
   if (len) {
-    if (dm->stall_limit_ns && !dm->capturing) {  // one-shot test hook
+    if (stall) {  // one-shot test hook
       P.test_stall = 1;
       P.wait_timeout_ns = dm->stall_limit_ns;
       dm->stall_limit_ns = 0;
@@ -1268,8 +1287,7 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     CU(cudaStreamIsCapturing(s, &st));
     const bool captured = st != cudaStreamCaptureStatusNone;
-    // (the quad kernel has no stall hook)
-    const int width = P.test_stall ? -1 : quad_width(engines, n, offset, len);
+    const int width = stall ? -1 : quad_width(engines, n, offset, len, pair);
     bool quads = width >= 0;
     for (int i = 0; i < n && !captured; i++) quads = quads && engines[i]->quad_rows;
     if (quads) {
@@ -1288,7 +1306,7 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
       P.skip = Q.run;
       CU(launch_quad_gemm(Q, dm->n_sms, s));
     }
-    if (!quads || captured) CU(launch_limb_gemm(P, engines[0]->block_n, engines[0]->pair, dm->n_sms, s));
+    if (!quads || captured) CU(launch_limb_gemm(P, engines[0]->block_n, pair, dm->n_sms, s));
   }
   for (int i = 0; i < n; i++) {
     engines[i]->res_offset = offset;
@@ -1813,7 +1831,7 @@ int irs_dc_scan_fused(irs_distance_comparator* dc, irs_circuits* c, irs_sharedb*
   memset(&F, 0, sizeof F);
   const uint16_t mults[kFusedEngines] = {1, 1, 1, 2, 2, 2};
   for (int e = 0; e < kFusedEngines; e++) {
-    int rc = fill_problem(eng[e], mults[e], offset, len, F.prob[e]);
+    int rc = fill_problem(eng[e], mults[e], offset, len, false, F.prob[e]);
     if (rc) return rc;
     // the fused kernel's query tile is 128 rows whatever the engine's own tile width
     if (make_tmap_u8(&F.prob[e].tm_b_lo, eng[e]->q_lo, eng[e]->n_cap, eng[e]->code_length, kFusedBlockN) ||

@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(kThreads, 1) limb_gemm_kernel(const __grid_con
 #pragma unroll
         for (int c = 0; c < kCols / 32; c++) {
           const uint32_t n = (uint32_t)(tl.n_tile * BN + half * kCols + c * 32);
+          if (n >= pr.n_pad) break;  // part-filled last tile
           uint32_t v[16];
 #pragma unroll
           for (int j = 0; j < 16; j++) {
@@ -472,6 +473,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int c = 0; c < kCols / 32; c++) {
           const uint32_t n = (uint32_t)(tl.n_tile * BN + half * kCols + c * 32);
+          if (n >= pr.n_pad) break;  // part-filled last tile
           uint32_t v[16];
 #pragma unroll
           for (int j = 0; j < 16; j++) {
@@ -563,22 +565,21 @@ static cudaError_t launch_pair(const GemmParams& P, int n_sms, cudaStream_t stre
 }
 
 // The pair kernel reaches a higher MAC rate per clock but, at the B200's
-// 1000 W limit, pulls the SM clock down about as far as it gains, so the
-// one-SM kernel is the default and the batch autotuner decides per batch
-// shape (irs_sharedb_set_pair).
+// 1000 W limit, pulls the SM clock down about as far as it gains, so for long
+// launches the one-SM kernel is the default and the batch autotuner decides per
+// batch shape (irs_sharedb_set_pair).
 bool gemm_pair_applies(bool pair, int block_n) { return pair && block_n == 256; }
 
 // Measured on 65,536-entry chunks of the six engines: up to 768 query rows
 // the 128-row tile (3 pipeline stages) beats the 256-row tile (2 stages) by
 // 5-20%, since the pass is still close to streaming the DB; from 1024 rows,
 // and on whole-DB passes, the 256-row tile wins (1024 rows: 66.8 against
-// 76.9 ms on 524,288 entries).
+// 76.9 ms on 524,288 entries).  Row counts that are no multiple of the tile
+// part-fill the last one: the 64-row tile that would divide them runs at half
+// the rate (960 rows x 32,768 entries, one engine: 1.51 ms, against 0.81).
 int gemm_block_n_for(uint32_t n_pad) {
-  if (n_pad <= 768 && n_pad % 128 == 0) return 128;
-  if (n_pad % 256 == 0) return 256;
-  if (n_pad % 128 == 0) return 128;
-  if (n_pad % 64 == 0) return 64;
-  return 0;
+  if (n_pad == 0 || n_pad % 64) return 0;
+  return n_pad <= 64 ? 64 : n_pad <= 768 ? 128 : 256;
 }
 
 // L2 policy of the one-SM kernel's loads (GemmParams::l2_hint), opt-in through
@@ -602,8 +603,7 @@ static uint32_t gemm_l2_hint() {
 }
 
 cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair_wanted, int n_sms, cudaStream_t stream) {
-  // the stall hook is the one-SM kernel's
-  const bool pair = gemm_pair_applies(pair_wanted, block_n) && !P.test_stall;
+  const bool pair = gemm_pair_applies(pair_wanted, block_n);
   if (P.wait_timeout_ns == 0) P.wait_timeout_ns = kGemmWaitTimeoutNs;
   P.l2_hint = gemm_l2_hint();
   // Serpentine K order (GemmParams::serpentine), on unless IRS_GEMM_SERPENTINE=0.
@@ -621,7 +621,7 @@ cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair_wanted, int n
   for (int i = 0; i < P.n_prob; i++) {
     GemmProblem& pr = P.prob[i];
     pr.tiles_m = (pr.m_len + bm - 1) / bm;
-    pr.tiles_n = pr.n_pad / (uint32_t)block_n;
+    pr.tiles_n = (pr.n_pad + (uint32_t)block_n - 1) / (uint32_t)block_n;
     P.total_tiles += (int)(pr.tiles_m * pr.tiles_n);
   }
   if (pair) return launch_pair(P, n_sms, stream);

@@ -447,7 +447,7 @@ int quad_width_for(const uint32_t* K, int n_prob, uint32_t m_len, uint32_t n_pad
   for (int i = 0; i < n_prob; i++) bytes += 2.0 * K[i] * m_len;
   const uint32_t bm = pair ? (uint32_t)kBM2 : (uint32_t)kBM;
   for (int i = 0; i < n_prob; i++) {
-    tiles[i] = (m_len + bm - 1) / bm * (n_pad / (uint32_t)block_n);
+    tiles[i] = (m_len + bm - 1) / bm * ((n_pad + (uint32_t)block_n - 1) / (uint32_t)block_n);
     cost[i] = K[i] / 128 * (pair ? 1536 : block_n == 256 ? 1920 : kRoundTrip) + kDrain;
   }
   const double plain = std::max(last_done(tiles, cost, n_prob, pair ? n_sms / 2 : n_sms), bytes / kHbmBytesPerCycle);

@@ -146,3 +146,25 @@ def test_check_shared_matmul_and_distances(dm, oracle):
             assert int(mask_dot[qi, j]) == mc
             dist = 0.5 - (int(code_dot[qi, j]) - 65536 * (int(code_dot[qi, j]) >= 32768)) / (2.0 * mc)
             assert abs(dist - hd / mc) <= 1e-6
+
+
+# padded rows that no tile divides: one part-filled 128-row tile, 256-row tiles
+# with 64, 128 and 192 columns in the last, on one SM and on SM pairs
+@pytest.mark.parametrize("q_len", [192, 320, 832, 896, 930])
+def test_part_filled_query_tiles(dm, oracle, q_len):
+    rng = np.random.default_rng(q_len)
+    n, width = 700, 6400
+    db = rng.integers(0, 65535, (n, width)).astype(np.uint16)
+    q = rng.integers(0, 65535, (q_len, width)).astype(np.uint16)
+    e = _engine(dm, 0, n, q_len, width, remote=False)
+    try:
+        e.load_records(0, db)
+        e.query_upload(q)
+        exp = oracle.dot_u16(q, db)
+        for pair, tile in ((False, 0), (True, 0), (False, 64)):
+            e.set_pair(pair)
+            e.set_tile(tile)
+            e.dot(0, n, 1)
+            assert np.array_equal(e.fetch_results(n), exp)
+    finally:
+        e.close()
