@@ -278,11 +278,31 @@ void pool_free(irs_device_manager* dm, int party, void* p) {
   if (p) cudaFreeAsync(p, dm->streams[party]);
 }
 
+// Scratch of one call, ordered on the call's own stream (freed there with
+// cudaFreeAsync): unlike pool_alloc it does not wait for the stream.
+int scratch_alloc(irs_device_manager* dm, cudaStream_t s, size_t bytes, void** out) {
+  *out = nullptr;
+  cudaError_t e = cudaMallocFromPoolAsync(out, bytes, dm->pools[0], s);
+  if (e == cudaErrorMemoryAllocation && !dm->capturing) {
+    cudaGetLastError();
+    if (reclaim_sums(dm->device)) e = cudaMallocFromPoolAsync(out, bytes, dm->pools[0], s);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(IRS_ERR_NOMEM, "device scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
+  }
+  return IRS_OK;
+}
+
+int device_error(int code) {
+  if (code) return fail(IRS_ERR_DEVICE, "kernel reported error code %d (bounded wait expired)", code);
+  return IRS_OK;
+}
+
 int check_device_error(irs_device_manager* dm) {
   int code = 0;
   CU(cudaMemcpy(&code, dm->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (code) return fail(IRS_ERR_DEVICE, "kernel reported error code %d (bounded wait expired)", code);
-  return IRS_OK;
+  return device_error(code);
 }
 
 ChaChaKey key_of(const uint32_t k[8]) {
@@ -1403,6 +1423,23 @@ __global__ void scatter_views_kernel(const uint32_t* comp, size_t n_words32, uin
   if (opened) opened[i] = c0 ^ c1 ^ c2;
 }
 
+// Whether a result array of a flat call shares memory with an input: the kernel
+// then may not write results while other words' shares are still to be read.
+static bool results_overlap_shares(const ThresholdParams& P, int stage, uint64_t* const res_a[3],
+                                   uint64_t* const res_b[3], const uint64_t* opened) {
+  const uintptr_t in = P.n_words * 64, out = P.n_words * 4;
+  for (int k = 0; k < 7; k++) {
+    const void* r = k == 6 ? opened : k < 3 ? (res_a ? res_a[k] : nullptr) : (res_b ? res_b[k - 3] : nullptr);
+    if (!r) continue;
+    const uintptr_t a = reinterpret_cast<uintptr_t>(r);
+    for (int p = 0; p < 3; p++) {
+      const uintptr_t c = reinterpret_cast<uintptr_t>(P.code[p]), m = reinterpret_cast<uintptr_t>(P.mask[p]);
+      if ((a < c + in && c < a + out) || (stage == kStageFull && a < m + in && m < a + out)) return true;
+    }
+  }
+  return false;
+}
+
 static int run_flat(irs_circuits* c, const uint16_t* const code_a[3], const uint16_t* const mask_a[3], size_t n,
                     uint32_t threshold_a, uint64_t* const res_a[3], uint64_t* const res_b[3], uint64_t* opened,
                     int stage, void* stream) {
@@ -1425,9 +1462,19 @@ static int run_flat(irs_circuits* c, const uint16_t* const code_a[3], const uint
   P.threshold_a = threshold_a;
   P.n_words = n / 32;
   P.word_base = 0;
+  if (threshold_writes_shares(P.n_words) && !results_overlap_shares(P, stage, res_a, res_b, opened)) {
+    for (int p = 0; p < 3; p++) {
+      P.res_a[p] = res_a ? reinterpret_cast<uint32_t*>(res_a[p]) : nullptr;
+      P.res_b[p] = res_b ? reinterpret_cast<uint32_t*>(res_b[p]) : nullptr;
+    }
+    P.revealed = reinterpret_cast<uint32_t*>(opened);
+    CU(launch_threshold_flat(P, stage, s));
+    return IRS_OK;
+  }
+  // (or results over the shares: every share is read before the first is written)
   uint32_t* comp = nullptr;
   void* p;
-  int rc = pool_alloc(dm, 0, 3 * P.n_words * 4, &p);
+  int rc = scratch_alloc(dm, s, 3 * P.n_words * 4, &p);
   if (rc) return rc;
   comp = (uint32_t*)p;
   P.res_comp = comp;
@@ -1462,17 +1509,20 @@ static int run_or_tree(irs_circuits* c, const uint32_t* comp, size_t n_words, ui
   P.nonce = nonce_of(kDomOrTree, (uint32_t)dm->device);
   P.batch = c->batch;
   P.batch_dev = c->batch_from_device ? dm->d_batch : nullptr;
+  P.err = dm->d_err;
   void* p;
-  int rc = pool_alloc(dm, 0, (6 * n_words + 4) * 4, &p);
+  int rc = scratch_alloc(dm, s, (6 * n_words + 5) * 4, &p);
   if (rc) return rc;
   uint32_t* scratch = static_cast<uint32_t*>(p);
-  uint32_t* out4 = scratch + 6 * n_words;
-  cudaError_t e = launch_or_tree(P, comp, n_words, scratch, out4, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(out, out4, 16, cudaMemcpyDeviceToHost, s);
+  uint32_t* out5 = scratch + 6 * n_words;
+  uint32_t got[5] = {};
+  cudaError_t e = launch_or_tree(P, comp, n_words, scratch, out5, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(got, out5, sizeof got, cudaMemcpyDeviceToHost, s);
   cudaFreeAsync(scratch, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(IRS_ERR_CUDA, "or tree: %s", cudaGetErrorString(e));
-  return check_device_error(dm);
+  memcpy(out, got, 16);
+  return device_error((int)got[4]);
 }
 
 int irs_circuits_or_reduce(irs_circuits* c, const uint64_t* const res_a[3], size_t n, uint32_t out[4], void* stream) {
@@ -1485,7 +1535,7 @@ int irs_circuits_or_reduce(irs_circuits* c, const uint64_t* const res_a[3], size
   const size_t n_words = n / 32;
   // gather the three a-shares (u64 words = pairs of u32 words) into one [3][n_words] vector
   void* p;
-  int rc = pool_alloc(dm, 0, 3 * n_words * 4, &p);
+  int rc = scratch_alloc(dm, s, 3 * n_words * 4, &p);
   if (rc) return rc;
   uint32_t* comp = static_cast<uint32_t*>(p);
   cudaError_t e = cudaSuccess;
@@ -1518,7 +1568,7 @@ int irs_circuits_compare_threshold_masked_many_with_or_tree(irs_circuits* c, con
   P.threshold_a = threshold_a;
   P.n_words = n / 32;
   void* p;
-  int rc = pool_alloc(dm, 0, 3 * P.n_words * 4, &p);
+  int rc = scratch_alloc(dm, s, 3 * P.n_words * 4, &p);
   if (rc) return rc;
   P.res_comp = static_cast<uint32_t*>(p);
   cudaError_t e = launch_threshold_flat(P, kStageFull, s);
@@ -1550,7 +1600,7 @@ int irs_circuits_lift_mpc(irs_circuits* c, const uint16_t* const mask_a[3], size
   }
   P.n_words = n / 32;
   void* p;
-  int rc = pool_alloc(dm, 0, 6 * n * 2, &p);
+  int rc = scratch_alloc(dm, s, 6 * n * 2, &p);
   if (rc) return rc;
   uint16_t* tmp = (uint16_t*)p;
   cudaError_t e = launch_lift_flat(P, tmp, s);

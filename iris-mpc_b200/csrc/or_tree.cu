@@ -6,30 +6,36 @@
 // Tree shape (the reference's): at each level the first half of the words is
 // combined with the second half, word i with word i + num, and an odd last
 // word moves down; after the word tree, the 32 bits of the last word are
-// collapsed with shifted copies of itself (16, 8, 4, 2, 1).  One launch per
-// level, ping-ponging between two scratch vectors.
+// collapsed with shifted copies of itself (16, 8, 4, 2, 1).
 //
 // Randomness of the AND gate of level L, index i: word 0 of the ChaCha12 block
 // at counter (batch << 40) | (L << 34) | i of each party's stream, nonce
 // domain 4; party p's mask is k_p ^ k_{p-1} (zero-sharing).  Word levels are
 // 1.., the collapse steps 40..44.
+//
+// What bounds it: latency.  A gate is three ChaCha blocks and a few logic
+// operations, and a launch per level spends its 5 us on the launch and on the
+// three blocks one after another.  So a block here takes the whole subtree of
+// one word several levels down: its threads draw the keystream of all the
+// subtree's gates at once, one block each, and the levels themselves are then
+// a few loads apart in shared memory.  32,770 words (2^20 elements): 2 launches
+// instead of 17, and 93 us for
+// the whole call with the comparison, against 177.
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <algorithm>
 #include "or_tree.h"
 
 namespace irs {
 
 namespace {
 
-__device__ __forceinline__ void or_gate(uint32_t x[3], const uint32_t y[3], const OrTreeParams& P, uint64_t gate) {
-  const uint64_t batch = P.batch_dev ? *P.batch_dev : P.batch;
-  uint32_t k[3];
-#pragma unroll 1
-  for (int s = 0; s < 3; s++) {
-    uint32_t blk[16];
-    chacha_block<12>(P.key[s], counter_of(batch, gate), P.nonce, blk);
-    k[s] = blk[0];
-  }
+constexpr int kMostLevels = 9;               // of one launch: 512 leaves
+constexpr int kStageLevels = 7;              // of a launch that is not the last
+constexpr int kMostLeaves = 1 << kMostLevels;
+constexpr uint64_t kCollapseLevel = 40;
+
+__device__ __forceinline__ void or_gate(uint32_t x[3], const uint32_t y[3], const uint32_t k[3]) {
   uint32_t z[3];
 #pragma unroll
   for (int p = 0; p < 3; p++) {
@@ -40,67 +46,140 @@ __device__ __forceinline__ void or_gate(uint32_t x[3], const uint32_t y[3], cons
   for (int p = 0; p < 3; p++) x[p] = x[p] ^ y[p] ^ z[p];
 }
 
-__global__ void or_level_kernel(const uint32_t* __restrict__ in, uint64_t in_stride, uint32_t* __restrict__ out,
-                                uint64_t out_stride, uint64_t num, int odd, uint32_t level, const OrTreeParams P) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < num) {
-    uint32_t x[3], y[3];
+// Words of a level below a level of n words.
+__device__ __forceinline__ uint64_t halved(uint64_t n) { return (n >> 1) + (n & 1); }
+
+// The word at position `pos` of level `level` (0 = this launch's input, n
+// words) in the subtree of word `root` at level `levels`: the position's bits,
+// highest first, choose between the two words i and i + num that make a word i.
+// An odd level's last word has one source.  False where there is no such word.
+__device__ __forceinline__ bool word_at(uint64_t n, int levels, int level, uint32_t pos, uint64_t root, uint64_t& idx) {
+  uint64_t size[kMostLevels + 1];
+  size[0] = n;
 #pragma unroll
-    for (int p = 0; p < 3; p++) {
-      x[p] = in[p * in_stride + i];
-      y[p] = in[p * in_stride + i + num];
-    }
-    or_gate(x, y, P, ((uint64_t)level << 34) | i);
+  for (int l = 0; l < kMostLevels; l++) size[l + 1] = halved(size[l]);
+  idx = root;
+  bool there = true;
 #pragma unroll
-    for (int p = 0; p < 3; p++) out[p * out_stride + i] = x[p];
-  } else if (odd && i == num) {
-#pragma unroll
-    for (int p = 0; p < 3; p++) out[p * out_stride + num] = in[p * in_stride + 2 * num];
+  for (int l = kMostLevels - 1; l >= 0; l--) {
+    if (l >= levels || l < level) continue;
+    const uint64_t num = size[l] >> 1;
+    const bool second = (pos >> (l - level)) & 1u;
+    if (idx < num) idx += second ? num : 0;
+    else { there = there && !second; idx = 2 * num; }
   }
+  return there;
 }
 
-__global__ void or_collapse_kernel(const uint32_t* __restrict__ in, uint64_t stride, uint32_t* __restrict__ out4,
-                                   const OrTreeParams P) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
-  uint32_t x[3] = {in[0], in[stride], in[2 * stride]};
-  int j = 0;
-  for (int s = 16; s >= 1; s >>= 1, j++) {
-    const uint32_t y[3] = {x[0] >> s, x[1] >> s, x[2] >> s};
-    or_gate(x, y, P, (uint64_t)(40 + j) << 34);
+// Each block reduces the subtree of output word blockIdx.x over `levels`
+// levels; with `last`, that is the whole tree, and the word collapses to one bit.
+__global__ void or_subtree_kernel(const uint32_t* __restrict__ in, uint64_t in_stride, uint64_t n, int levels,
+                                  uint32_t first_level, uint32_t* __restrict__ out, uint64_t out_stride, int last,
+                                  const OrTreeParams P) {
+  __shared__ uint32_t word[2][3][kMostLeaves];
+  __shared__ uint32_t key[3][kMostLeaves + 8];
+  const int leaves = 1 << levels;
+  const uint64_t batch = P.batch_dev ? *P.batch_dev : P.batch;
+  for (int t = threadIdx.x; t < leaves; t += blockDim.x) {
+    uint64_t i;
+    const bool there = word_at(n, levels, 0, (uint32_t)t, blockIdx.x, i);
+#pragma unroll
+    for (int p = 0; p < 3; p++) word[0][p][t] = there ? in[p * in_stride + i] : 0u;
   }
-  out4[0] = x[0] & 1u;
-  out4[1] = x[1] & 1u;
-  out4[2] = x[2] & 1u;
-  out4[3] = (x[0] ^ x[1] ^ x[2]) & 1u;
+  // Gates: those of the first level (leaves / 2 of them), of the second, ...,
+  // then the collapse steps; gate g's keystream word of stream s at key[s][g].
+  const int gates = leaves - 1, all = gates + (last ? 5 : 0);
+  for (int c = threadIdx.x; c < 3 * all; c += blockDim.x) {
+    const int g = c / 3, s = c % 3;
+    uint64_t gate = (kCollapseLevel + (uint64_t)(g - gates)) << 34;
+    bool there = true;
+    if (g < gates) {
+      int l = 0, pos = g;
+      for (; pos >= (leaves >> (l + 1)); l++) pos -= leaves >> (l + 1);
+      uint64_t i;
+      there = word_at(n, levels, l + 1, (uint32_t)pos, blockIdx.x, i);
+      gate = ((uint64_t)(first_level + (uint32_t)l) << 34) | i;
+    }
+    if (there) {
+      uint32_t blk[16];
+      chacha_block<12>(P.key[s], counter_of(batch, gate), P.nonce, blk);
+      key[s][g] = blk[0];
+    }
+  }
+  __syncthreads();
+  int cur = 0, first_gate = 0;
+  for (int l = 0; l < levels; l++) {
+    const int nodes = leaves >> (l + 1);
+    for (int t = threadIdx.x; t < nodes; t += blockDim.x) {
+      uint64_t i, num = n;
+      for (int q = 0; q < l; q++) num = halved(num);
+      num >>= 1;
+      const bool there = word_at(n, levels, l + 1, (uint32_t)t, blockIdx.x, i);
+      uint32_t x[3], y[3], k[3];
+#pragma unroll
+      for (int p = 0; p < 3; p++) {
+        x[p] = word[cur][p][2 * t];
+        y[p] = word[cur][p][2 * t + 1];
+        k[p] = key[p][first_gate + t];
+      }
+      if (there && i < num) or_gate(x, y, k);
+#pragma unroll
+      for (int p = 0; p < 3; p++) word[cur ^ 1][p][t] = x[p];
+    }
+    __syncthreads();
+    cur ^= 1;
+    first_gate += nodes;
+  }
+  if (threadIdx.x) return;
+  uint32_t x[3] = {word[cur][0][0], word[cur][1][0], word[cur][2][0]};
+  if (!last) {
+#pragma unroll
+    for (int p = 0; p < 3; p++) out[p * out_stride + blockIdx.x] = x[p];
+    return;
+  }
+  for (int j = 0; j < 5; j++) {
+    const int s = 16 >> j;
+    const uint32_t y[3] = {x[0] >> s, x[1] >> s, x[2] >> s};
+    const uint32_t k[3] = {key[0][gates + j], key[1][gates + j], key[2][gates + j]};
+    or_gate(x, y, k);
+  }
+  out[0] = x[0] & 1u;
+  out[1] = x[1] & 1u;
+  out[2] = x[2] & 1u;
+  out[3] = (x[0] ^ x[1] ^ x[2]) & 1u;
+  out[4] = (uint32_t)*P.err;
 }
 
 }  // namespace
 
 cudaError_t launch_or_tree(const OrTreeParams& P, const uint32_t* comp, size_t n_words, uint32_t* scratch,
-                           uint32_t* out4, cudaStream_t stream) {
+                           uint32_t* out5, cudaStream_t stream) {
   if (n_words == 0) return cudaErrorInvalidValue;
   const uint32_t* cur = comp;
-  uint64_t cur_stride = n_words;
+  uint64_t cur_stride = n_words, num = n_words;
   uint32_t* bufs[2] = {scratch, scratch + 3 * n_words};
   int which = 0;
-  uint64_t num = n_words;
   uint32_t level = 1;
-  while (num > 1) {
-    const int odd = (int)(num & 1);
-    num >>= 1;
-    const uint64_t threads = num + (uint64_t)odd;
-    const unsigned grid = (unsigned)((threads + 255) / 256);
-    or_level_kernel<<<grid, 256, 0, stream>>>(cur, cur_stride, bufs[which], n_words, num, odd, level, P);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+  while (true) {
+    int levels = 0;
+    uint64_t left = num;
+    for (; left > 1 && levels < kMostLevels; levels++) left = (left >> 1) + (left & 1);
+    const bool last = left == 1;
+    if (!last) {
+      left = num;
+      for (levels = 0; levels < kStageLevels; levels++) left = (left >> 1) + (left & 1);
+    }
+    const unsigned threads = (unsigned)std::min(1024, std::max(32, 3 << levels));
+    or_subtree_kernel<<<(unsigned)left, threads, 0, stream>>>(cur, cur_stride, num, levels, level,
+                                                              last ? out5 : bufs[which], n_words, last, P);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || last) return e;
     cur = bufs[which];
     cur_stride = n_words;
     which ^= 1;
-    num += (uint64_t)odd;
-    level++;
+    num = left;
+    level += (uint32_t)levels;
   }
-  or_collapse_kernel<<<1, 32, 0, stream>>>(cur, cur_stride, out4, P);
-  return cudaGetLastError();
 }
 
 }  // namespace irs

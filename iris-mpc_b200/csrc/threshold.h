@@ -19,6 +19,10 @@ struct ThresholdParams {
   uint64_t word_base;
   uint32_t* revealed;   // [n_words], optional
   uint32_t* res_comp;   // [3][n_words], optional: component p of the result
+  // [n_words], optional, where threshold_writes_shares: party p's shares (a, b)
+  // of the result
+  uint32_t* res_a[3];
+  uint32_t* res_b[3];
   // bitmap mode
   uint32_t n_entries;   // entries in this call
   uint32_t m0;          // global index of the first entry (multiple of 32)
@@ -52,6 +56,11 @@ struct ThresholdParams {
   const uint32_t* forced_entry;
   uint32_t n_forced;
 };
+
+// Whether a flat launch over n_words writes res_a and res_b itself (the
+// few-words kernel; in the other one the seven stores per word cost more than
+// the launch that splits the components: 397 us against 393 at 2^24 elements).
+bool threshold_writes_shares(uint64_t n_words);
 
 cudaError_t launch_threshold_flat(const ThresholdParams& P, int stage, cudaStream_t stream);
 cudaError_t launch_threshold_bitmap(const ThresholdParams& P, cudaStream_t stream);

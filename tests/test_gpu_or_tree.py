@@ -55,3 +55,24 @@ def test_or_tree_matches_plaintext_and_oracle(dm, oracle, n, planted):
         c.close()
         for b in dcode + dmask:
             b.free()
+
+
+# word counts around one launch's 512 leaves and two launches' 512 x 128, odd
+# levels among them, every party's share of the opened bit against the oracle
+@pytest.mark.parametrize("words", [2, 6, 510, 512, 514, 1022, 65534, 65536, 65538, 70002])
+def test_or_reduce_sizes(dm, oracle, words):
+    rng = np.random.default_rng(words)
+    ra = [rng.integers(0, 1 << 63, words // 2, dtype=np.uint64) for _ in range(3)]
+    if words % 4:  # a vector of zeros, but for one bit in every other case
+        ra[2] = ra[0] ^ ra[1]
+        ra[2][words // 4] ^= np.uint64(1 << 40) * np.uint64(words % 8 == 6)
+    bufs = [irisb200.DeviceBuffer.from_array(dm, a) for a in ra]
+    c = irisb200.Circuits(dm, W.SEEDS)
+    try:
+        comps, opened = c.or_reduce(bufs, words * 32)
+        ocomps, oopened = oracle.or_tree([a.view(np.uint32) for a in ra], KEYS)
+        assert opened == oopened and np.array_equal(comps, ocomps)
+    finally:
+        c.close()
+        for b in bufs:
+            b.free()

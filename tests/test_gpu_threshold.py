@@ -121,3 +121,38 @@ def test_rejects_bad_shapes(dm):
     with pytest.raises(irisb200.IrisError):
         irisb200.Circuits(dm, bad)
     c.close()
+
+
+# the few-words kernel at one word, part and whole warps of words, and its last
+# and first sizes, against the prefix of a call that runs one thread per word
+# (a word's keystream depends on its index alone)
+def test_few_words_equal_the_prefix_of_many(dm):
+    import irisb200
+    big = 889 * 32 * 32 + 64
+    rng = np.random.default_rng(12)
+    shares = [rng.integers(0, 1 << 16, big, dtype=np.uint16) for _ in range(6)]
+    bufs = [irisb200.DeviceBuffer.from_array(dm, s) for s in shares]
+    c = irisb200.Circuits(dm, SEEDS)
+    c.set_batch(3)
+
+    def run(n, msb_only):
+        res = [irisb200.DeviceBuffer(dm, n // 8) for _ in range(7)]
+        if msb_only:
+            c.extract_msb_of_code(bufs[:3], n, res_a=res[:3], res_b=res[3:6], opened=res[6])
+        else:
+            c.compare_threshold_masked_many(bufs[:3], bufs[3:], n, 16384, res_a=res[:3], res_b=res[3:6], opened=res[6])
+        dm.synchronize()
+        return [r.download(np.uint32, n // 32) for r in res]
+    for msb_only in (False, True):
+        want = run(big, msb_only)
+        for words in (2, 30, 32, 34, 4000, 888 * 32):
+            for got, w in zip(run(words * 32, msb_only), want):
+                assert np.array_equal(got, w[:words])
+    # results over the shares: every share is read before it is overwritten
+    want = run(4096, False)
+    into = bufs[0].ptr
+    c.compare_threshold_masked_many(bufs[:3], bufs[3:], 4096, 16384, res_a=[into, into + 4096, into + 8192])
+    dm.synchronize()
+    got = bufs[0].download(np.uint32, 3 * 1024)
+    assert np.array_equal(got[:128], want[0])
+    c.close()
