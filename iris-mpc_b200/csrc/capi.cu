@@ -1184,7 +1184,8 @@ int irs_sharedb_set_batch(irs_sharedb* db, uint64_t batch_id) {
   return IRS_OK;
 }
 
-static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t len, bool pair, GemmProblem& pr) {
+// half_tile: the query maps load 128 of a 256-row tile's rows.
+static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t len, bool half_tile, GemmProblem& pr) {
   CHECK(db->db_lo, IRS_ERR_STATE, "alloc_db not called");
   CHECK(db->have_query, IRS_ERR_STATE, "no query uploaded");
   CHECK(offset % 32 == 0, IRS_ERR_INVALID, "offset %zu must be a multiple of 32", offset);
@@ -1194,8 +1195,8 @@ static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t le
   memset(&pr, 0, sizeof pr);
   pr.tm_a_lo = db->tm_db_lo;
   pr.tm_a_hi = db->tm_db_hi;
-  pr.tm_b_lo = pair ? db->tm_qh_lo : db->tm_q_lo;
-  pr.tm_b_hi = pair ? db->tm_qh_hi : db->tm_q_hi;
+  pr.tm_b_lo = half_tile ? db->tm_qh_lo : db->tm_q_lo;
+  pr.tm_b_hi = half_tile ? db->tm_qh_hi : db->tm_q_hi;
   pr.out = db->results;
   pr.m0 = (uint32_t)offset;
   pr.m_len = (uint32_t)len;
@@ -1242,6 +1243,17 @@ static bool plain_pair(irs_sharedb* const* engines, int n, size_t len) {
   return macs < 3e12;  // about 2 ms
 }
 
+// Whether a launch of 256-row tiles with the GEMM left open has so few tiles
+// that it runs 128-row ones with their K loop shared (gemm_k_split): 64 entries
+// x 2048 rows, six engines, 81 us against 112.
+static bool few_tiles(irs_sharedb* const* engines, int n, size_t len) {
+  const irs_sharedb* e = engines[0];
+  if (e->pair || e->tile_override || e->block_n != 256) return false;
+  for (int i = 0; i < n; i++)
+    if (engines[i]->n_pad != e->n_pad || engines[i]->code_length < 8 * 128) return false;
+  return 3 * (size_t)n * ((len + 127) / 128) * ((e->n_pad + 127) / 128) <= 2 * (size_t)e->dm->n_sms;
+}
+
 static void fill_quad_problem(const irs_sharedb* db, const GemmProblem& g, int width, QuadProblem& pr) {
   pr.tm_a_lo[0] = db->tm_db_lo;
   pr.tm_a_hi[0] = db->tm_db_hi;
@@ -1282,9 +1294,10 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
   }
   // the stall hook is the one-SM kernel's
   const bool stall = len && dm->stall_limit_ns && !dm->capturing;
-  const bool pair = !stall && plain_pair(engines, n, len);
+  const bool few = !stall && few_tiles(engines, n, len);
+  const bool pair = !stall && !few && plain_pair(engines, n, len);
   for (int i = 0; i < n; i++) {
-    int rc = fill_problem(engines[i], multipliers[i], offset, len, pair, P.prob[i]);
+    int rc = fill_problem(engines[i], multipliers[i], offset, len, pair || few, P.prob[i]);
     if (rc) return rc;
   }
   cudaStream_t s = party_stream(dm, engines[0]->peer, stream);
@@ -1326,7 +1339,7 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
       P.skip = Q.run;
       CU(launch_quad_gemm(Q, dm->n_sms, s));
     }
-    if (!quads || captured) CU(launch_limb_gemm(P, engines[0]->block_n, pair, dm->n_sms, s));
+    if (!quads || captured) CU(launch_limb_gemm(P, few ? 128 : engines[0]->block_n, pair, dm->n_sms, s));
   }
   for (int i = 0; i < n; i++) {
     engines[i]->res_offset = offset;

@@ -27,6 +27,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <stdlib.h>
+#include <algorithm>
 #include "common.cuh"
 #include "gemm_limb.h"
 #include "quad_gemm.h"
@@ -505,6 +506,194 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   }
 }
 
+// ---------------------------------------------------------------------------
+// Few tiles: a tile's K loop is a chain of pipeline round trips (about 0.6 us
+// per 128-byte block), and with fewer tiles than SMs most of the GPU has none.
+// Here a cluster of S CTAs (4 or 8) shares a tile, each taking its part of the K
+// blocks, and the partial sums meet over distributed shared memory: CTA r of
+// the cluster adds up columns [32 r, 32 r + 32) of the tile (mod 2^16), adds
+// the mask and stores them (CTAs past BN / 32 only send).  One tile per
+// cluster, not persistent.
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ void st_cluster(uint32_t cluster_addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+}
+
+template <int BN, int S>
+__global__ void __cluster_dims__(S, 1, 1) __launch_bounds__(kThreads, 1)
+    limb_gemm_split_kernel(const __grid_constant__ GemmParams P) {
+  using C = Cfg<BN>;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* a_lo = smem;
+  uint8_t* a_hi = a_lo + C::kStages * kBM * kBK;
+  uint8_t* b_lo = a_hi + C::kStages * kBM * kBK;
+  uint8_t* b_hi = b_lo + C::kStages * BN * kBK;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(b_hi + C::kStages * BN * kBK);
+  uint64_t* full_bar = bars;
+  uint64_t* empty_bar = bars + C::kStages;
+  uint64_t* acc_full = bars + 2 * C::kStages;
+  uint64_t* done_bar = acc_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 2);
+  uint32_t* recv = reinterpret_cast<uint32_t*>(smem);  // [sender][word of 2 columns][row], over the stages
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();
+  int* err = P.err;
+  const uint64_t lim = P.wait_timeout_ns, lim2 = 2 * P.wait_timeout_ns;
+  Tile tl;
+  tile_of(P, blockIdx.x / S, tl);  // one cluster per tile
+  const GemmProblem& pr = P.prob[tl.prob];
+  const uint32_t k_begin = pr.k_iters * (uint32_t)rank / S, k_end = pr.k_iters * (uint32_t)(rank + 1) / S;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::kStages; s++) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    mbar_init(done_bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"((uint32_t)C::kTmemCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  constexpr int kCols = C::kColsPerThread;  // of one epilogue thread
+  const int quad = warp & 3;
+  const int half = (warp - 2) >> 2;
+  const int row = quad * 32 + lane;
+  uint32_t packed[kCols / 2];
+  bool ok = true;
+  if (warp == 0) {
+    if (lane == 0) {
+      int issued_phase[C::kStages];
+      bool issued[C::kStages];
+      for (int s = 0; s < C::kStages; s++) issued[s] = false;
+      int stage = 0;
+      uint32_t phase = 0;
+      const int ya = (int)pr.m0 + tl.m_tile * kBM, yb = tl.n_tile * BN;
+      for (uint32_t ki = k_begin; ki < k_end; ki++) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, err, kErrTimeoutEmpty, lim2)) break;
+        mbar_expect_tx(&full_bar[stage], (uint32_t)C::kStageBytes);
+        const int x = (int)ki * kBK;
+        tma_load_2d(a_lo + stage * kBM * kBK, &pr.tm_a_lo, &full_bar[stage], x, ya);
+        tma_load_2d(a_hi + stage * kBM * kBK, &pr.tm_a_hi, &full_bar[stage], x, ya);
+        tma_load_2d(b_lo + stage * BN * kBK, &pr.tm_b_lo, &full_bar[stage], x, yb);
+        tma_load_2d(b_hi + stage * BN * kBK, &pr.tm_b_hi, &full_bar[stage], x, yb);
+        issued[stage] = true;
+        issued_phase[stage] = (int)phase;
+        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
+      }
+      // no copy into the stages may be in flight when they become the receive buffer
+      for (int s = 0; s < C::kStages; s++)
+        if (issued[s]) mbar_wait_drain(&full_bar[s], (uint32_t)issued_phase[s], err, lim2);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      constexpr uint32_t idesc = idesc_u8(BN);
+      for (uint32_t ki = k_begin; ki < k_end; ki++) {
+        if (!mbar_wait(&full_bar[stage], phase, err, kErrTimeoutFull, lim)) { ok = false; break; }
+        tc_fence_after();
+        const uint64_t dal = smem_desc(a_lo + stage * kBM * kBK);
+        const uint64_t dah = smem_desc(a_hi + stage * kBM * kBK);
+        const uint64_t dbl = smem_desc(b_lo + stage * BN * kBK);
+        const uint64_t dbh = smem_desc(b_hi + stage * BN * kBK);
+#pragma unroll
+        for (int kk = 0; kk < kBK / 32; kk++) {
+          const uint32_t acc = (ki > k_begin || kk > 0) ? 1u : 0u;
+          const uint64_t o = (uint64_t)(2 * kk);
+          mma_u8(tmem, dal + o, dbl + o, idesc, acc);
+          mma_u8(tmem + BN, dal + o, dbh + o, idesc, acc);
+          mma_u8(tmem + BN, dah + o, dbl + o, idesc, 1u);
+        }
+        mma_commit(&empty_bar[stage]);
+        if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
+      }
+      if (ok) mma_commit(acc_full);
+      mma_commit(done_bar);
+      mbar_wait_drain(done_bar, 0, err, lim2);
+    }
+  } else {
+    ok = mbar_wait(acc_full, 0, err, kErrTimeoutAccFull, lim2);
+    if (ok) {
+      tc_fence_after();
+      const uint32_t tbase = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * kCols);
+#pragma unroll
+      for (int c = 0; c < kCols / 32; c++) {
+        uint32_t r0[32], r1[32];
+        tmem_ld32(tbase + (uint32_t)(c * 32), r0);
+        tmem_ld32(tbase + (uint32_t)(BN + c * 32), r1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+          const uint32_t lo = (r0[2 * j] + (r1[2 * j] << 8)) & 0xFFFFu;
+          const uint32_t hi = (r0[2 * j + 1] + (r1[2 * j + 1] << 8)) << 16;
+          packed[c * 16 + j] = lo | hi;
+        }
+      }
+      tc_fence_before();
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();  // every CTA's stages are free
+  if (warp >= 2 && ok) {
+#pragma unroll
+    for (int c = 0; c < kCols / 32; c++) {
+      const int to = half * (kCols / 32) + c;
+      if (to == rank) continue;
+      const uint32_t dst = map_to_rank(recv + (rank * 16) * kBM + row, (uint32_t)to);
+#pragma unroll
+      for (int j = 0; j < 16; j++) st_cluster(dst + (uint32_t)(j * kBM * 4), packed[c * 16 + j]);
+    }
+  }
+  cluster_sync_all();  // the partial sums have arrived
+  const uint32_t m_local = (uint32_t)(tl.m_tile * kBM + row);
+  const uint32_t n = (uint32_t)(tl.n_tile * BN + rank * 32);
+  if (warp >= 2 && half == rank / (kCols / 32) && m_local < pr.m_len && n < pr.n_pad && !has_error(err)) {
+    uint32_t v[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      uint32_t x = packed[j];
+#pragma unroll
+      for (int c = 1; c < kCols / 32; c++)
+        if (rank % (kCols / 32) == c) x = packed[c * 16 + j];
+#pragma unroll
+      for (int s = 0; s < S; s++)
+        if (s != rank) x = add2(x, recv[(s * 16 + j) * kBM + row]);
+      v[j] = (pr.mult == 1) ? x : (((x & 0xFFFFu) * pr.mult) & 0xFFFFu) | (((x >> 16) * pr.mult) << 16);
+    }
+    if (pr.mask_on) {
+      const uint64_t blk = (((uint64_t)pr.m0 + m_local) * pr.n_pad + n) >> 5;
+      const uint64_t batch = pr.batch_dev ? *pr.batch_dev : pr.batch;
+      uint32_t ks[32];
+      chacha12_pair(&pr.key_own, &pr.key_prev, counter_of(batch, blk), pr.nonce, ks);
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] = sub2(add2(v[j], ks[j]), ks[16 + j]);
+    }
+    uint4* dst = reinterpret_cast<uint4*>(pr.out + (size_t)m_local * pr.n_pad + n);
+#pragma unroll
+    for (int q = 0; q < 4; q++) dst[q] = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)C::kTmemCols));
+  }
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -551,6 +740,16 @@ static cudaError_t launch_bn(const GemmParams& P, int n_sms, cudaStream_t stream
   const int grid = P.total_tiles < n_sms ? P.total_tiles : n_sms;
   if (grid <= 0) return cudaSuccess;
   limb_gemm_kernel<BN><<<grid, kThreads, C::kSmemBytes, stream>>>(P);
+  return cudaGetLastError();
+}
+
+template <int BN, int S>
+static cudaError_t launch_split(const GemmParams& P, cudaStream_t stream) {
+  using C = Cfg<BN>;
+  static std::atomic<uint64_t> attr_done{0};
+  cudaError_t e = smem_limit_once(limb_gemm_split_kernel<BN, S>, C::kSmemBytes, attr_done);
+  if (e != cudaSuccess) return e;
+  limb_gemm_split_kernel<BN, S><<<S * P.total_tiles, kThreads, C::kSmemBytes, stream>>>(P);
   return cudaGetLastError();
 }
 
@@ -602,6 +801,19 @@ static uint32_t gemm_l2_hint() {
   return hint;
 }
 
+// CTAs that share a tile's K loop (1: the persistent kernel).  Six engines, cold
+// caches, persistent / four / eight: 64 entries x 64 rows (6 tiles) 62 / 25.6 /
+// 21.5 us; 64 x 256 (12) 71 / 29.8 / 25.6; 500 x 32 (24) 64 / 29.7 / 33.8; 1000 x
+// 32 (48) 66 / 46; 2000 x 32 and 1000 x 256 (96) 75 / 73 and 79 / 73; 300 x 768
+// (108) 79 / 83.  Clusters of eight pay while all of them run at once, of four
+// up to two thirds of the SMs' count in tiles.
+static int gemm_k_split(const GemmParams& P, int block_n, int n_sms) {
+  uint32_t k = ~0u;
+  for (int i = 0; i < P.n_prob; i++) k = std::min(k, P.prob[i].k_iters);
+  if (block_n > 128 || 3 * P.total_tiles > 2 * n_sms || k < 8) return 1;
+  return 8 * P.total_tiles <= n_sms && k >= 16 ? 8 : 4;
+}
+
 cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair_wanted, int n_sms, cudaStream_t stream) {
   const bool pair = gemm_pair_applies(pair_wanted, block_n);
   if (P.wait_timeout_ns == 0) P.wait_timeout_ns = kGemmWaitTimeoutNs;
@@ -625,6 +837,10 @@ cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair_wanted, int n
     P.total_tiles += (int)(pr.tiles_m * pr.tiles_n);
   }
   if (pair) return launch_pair(P, n_sms, stream);
+  switch (P.test_stall ? 1 : gemm_k_split(P, block_n, n_sms)) {
+    case 4: return block_n == 64 ? launch_split<64, 4>(P, stream) : launch_split<128, 4>(P, stream);
+    case 8: return block_n == 64 ? launch_split<64, 8>(P, stream) : launch_split<128, 8>(P, stream);
+  }
   switch (block_n) {
     case 256: return launch_bn<256>(P, n_sms, stream);
     case 128: return launch_bn<128>(P, n_sms, stream);

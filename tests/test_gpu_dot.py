@@ -168,3 +168,36 @@ def test_part_filled_query_tiles(dm, oracle, q_len):
             assert np.array_equal(e.fetch_results(n), exp)
     finally:
         e.close()
+
+
+# launches of few tiles (the K loop shared by a cluster): eight and four CTAs a
+# tile, K too short to share, 64- and 128-row tiles, 256-row ones taken as 128,
+# part-filled tiles both ways, the last count that shares and the first that
+# does not (98 and 99 tiles on 148 SMs)
+@pytest.mark.parametrize("n,q_len,width", [(1, 1, 12800), (130, 64, 6400), (700, 130, 6400), (64, 2048, 2048),
+                                           (300, 96, 768), (300, 96, 1024), (300, 96, 2048), (257, 896, 1152),
+                                           (98 * 128, 64, 1280), (98 * 128 + 1, 64, 1280)])
+def test_few_tiles(dm, oracle, n, q_len, width):
+    rng = np.random.default_rng(n + q_len)
+    db = rng.integers(0, 65535, (n, width)).astype(np.uint16)
+    q = rng.integers(0, 65535, (q_len, width)).astype(np.uint16)
+    masked = _engine(dm, 1, n, q_len, width, remote=True)
+    plain = _engine(dm, 1, n, q_len, width, remote=False)
+    try:
+        exp = oracle.dot_u16(q, db)
+        for e in (plain, masked):
+            e.load_records(0, db)
+            e.query_upload(q)
+            e.dot(0, n, 1)
+        assert np.array_equal(plain.fetch_results(n), exp)
+        got = masked.fetch_results(n)
+        masked.set_tile(64)  # the same masked shares from another tile width, and from an offset
+        masked.dot(0, n, 1)
+        assert np.array_equal(masked.fetch_results(n), got)
+        if n > 64:
+            masked.set_tile(0)
+            masked.dot(64, n - 64, 1)
+            assert np.array_equal(masked.fetch_results(n - 64), got[:, 64:])
+    finally:
+        plain.close()
+        masked.close()
