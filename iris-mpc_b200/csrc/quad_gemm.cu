@@ -56,13 +56,23 @@ namespace irs {
 namespace {
 
 constexpr int kThreads = 576;               // TMA, MMA and 16 epilogue warps
-constexpr int kStages = 3;
+constexpr int kMaxStages = 5;
 constexpr int kMaxN = 256;
 constexpr int kSkew = 2;                     // blocks that go to acc0 ahead of acc1 (see the MMA issuer)
 constexpr int kABytes = 128 * kBK;           // one limb of a CTA's 128 entries
-constexpr int kBBytes = (kMaxN / 2) * kBK;   // one limb of a CTA's half of the quads
-constexpr int kSmemBytes = kStages * 2 * (kABytes + kBBytes) + 1024 + 256;
+constexpr int kStageRoom = 225 * 1024;        // shared memory for the stages
+constexpr int kSmemBytes = kStageRoom + 1024 /*align*/ + 256 /*barriers*/;
 constexpr int kTmemCols = 512;               // acc0 at 0, acc1 at 256
+
+// Stages of 128 K bytes that fit: three for 256 quads, four up to 192, five up
+// to 96 (192 quads on four stages: 2.08 to 2.18 ms per 32,768 entries against
+// 2.27 to 2.30 on three).  Prefetching the DB rows of a later block into L2
+// made every size slower, by 1 to 9%: the kernel is bound by what the SMs draw
+// from L2, not by the latency behind it.
+constexpr int stage_count(int tile_n) {
+  const int s = kStageRoom / (2 * (kABytes + tile_n / 2 * kBK));
+  return s < kMaxStages ? s : kMaxStages;
+}
 
 // Products in order (outer, inner) = 22 2x 2y x2 xx xy y2 yx yy: the DB plane
 // and the quarter of it that each reads.
@@ -144,14 +154,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   if (P.run.n && !P.run.all_set()) return;  // the same words for every CTA
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int bn = P.tile_n, half_n = bn / 2;
+  const int n_stages = P.stages;
+  const int b_bytes = half_n * kBK;  // one limb of a CTA's half of the quads
   uint8_t* a_lo = smem;
-  uint8_t* a_hi = a_lo + kStages * kABytes;
-  uint8_t* b_lo = a_hi + kStages * kABytes;
-  uint8_t* b_hi = b_lo + kStages * kBBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(b_hi + kStages * kBBytes);
+  uint8_t* a_hi = a_lo + n_stages * kABytes;
+  uint8_t* b_lo = a_hi + n_stages * kABytes;
+  uint8_t* b_hi = b_lo + n_stages * b_bytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStageRoom);
   uint64_t* full_bar = bars;
-  uint64_t* empty_bar = bars + kStages;
-  uint64_t* acc_full = bars + 2 * kStages;  // [2]: acc0, acc1
+  uint64_t* empty_bar = bars + kMaxStages;
+  uint64_t* acc_full = bars + 2 * kMaxStages;  // [2]: acc0, acc1
   uint64_t* acc_empty = acc_full + 2;       // [2]
   uint64_t* done_bar = acc_full + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 5);
@@ -162,12 +175,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const bool leader = rank == 0;
   const int cluster = blockIdx.x >> 1;
   const int n_clusters = gridDim.x >> 1;
-  const int bn = P.tile_n, half_n = bn / 2;
   int* err = P.err;
   const uint64_t lim = P.wait_timeout_ns, lim2 = 2 * P.wait_timeout_ns;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; s++) {
+    for (int s = 0; s < n_stages; s++) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -194,9 +206,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      int issued_phase[kStages];
-      bool issued[kStages];
-      for (int s = 0; s < kStages; s++) issued[s] = false;
+      uint32_t issued_phase = 0, issued = 0;  // bit s: stage s
       bool ok = true;
       const uint32_t tx = (uint32_t)(2 * 2 * (kABytes + half_n * kBK));  // both CTAs, both limbs
       for (int k = 0; ok; k++) {
@@ -218,19 +228,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const uint32_t fb = map_to_rank(&full_bar[stage], 0);
             tma_load_2d_pair(a_lo + stage * kABytes, &pr.tm_a_lo[plane], fb, x0 + ki * kBK, ya);
             tma_load_2d_pair(a_hi + stage * kABytes, &pr.tm_a_hi[plane], fb, x0 + ki * kBK, ya);
-            tma_load_2d_pair(b_lo + stage * kBBytes, &pr.tm_b_lo, fb, ki * kBK, yb);
-            tma_load_2d_pair(b_hi + stage * kBBytes, &pr.tm_b_hi, fb, ki * kBK, yb);
-            issued[stage] = true;
-            issued_phase[stage] = (int)phase;
-            if (++stage == kStages) { stage = 0; phase ^= 1u; }
+            tma_load_2d_pair(b_lo + stage * b_bytes, &pr.tm_b_lo, fb, ki * kBK, yb);
+            tma_load_2d_pair(b_hi + stage * b_bytes, &pr.tm_b_hi, fb, ki * kBK, yb);
+            issued |= 1u << stage;
+            issued_phase = (issued_phase & ~(1u << stage)) | phase << stage;
+            if (++stage == n_stages) { stage = 0; phase ^= 1u; }
           }
         }
       }
       // Exit: the leader's stage barriers complete only when both CTAs' copies
       // of that stage have landed.
       if (leader)
-        for (int s = 0; s < kStages; s++)
-          if (issued[s]) mbar_wait_drain(&full_bar[s], (uint32_t)issued_phase[s], err, lim2);
+        for (int s = 0; s < n_stages; s++)
+          if ((issued >> s) & 1u) mbar_wait_drain(&full_bar[s], (issued_phase >> s) & 1u, err, lim2);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
@@ -250,13 +260,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         // 32-byte steps of the last block (the bytes past the quarter belong
         // to the next one)
         const int last_steps = ((int)pr.quarter - (k_iters - 1) * kBK) / 32;
-        // The products of one 128-byte block into acc0 (which = 0) or acc1.
-        auto issue = [&](int ki, int which) {
-          const int st = (stage + ki) % kStages;
+        // The products of block ki, in stage st, into acc0 (which = 0) or acc1.
+        auto issue = [&](int ki, int st, int which) {
           const uint64_t dal = smem_desc(a_lo + st * kABytes);
           const uint64_t dah = smem_desc(a_hi + st * kABytes);
-          const uint64_t dbl = smem_desc(b_lo + st * kBBytes);
-          const uint64_t dbh = smem_desc(b_hi + st * kBBytes);
+          const uint64_t dbl = smem_desc(b_lo + st * b_bytes);
+          const uint64_t dbh = smem_desc(b_hi + st * b_bytes);
           const int steps = ki == k_iters - 1 ? last_steps : kBK / 32;
 #pragma unroll
           for (int kk = 0; kk < kBK / 32; kk++) {
@@ -273,47 +282,53 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           }
           if (which) mma_commit_pair(&empty_bar[st]);
         };
-        auto stage_full = [&](int ki) {
-          const int at = stage + ki;
-          if (!mbar_wait(&full_bar[at % kStages], phase ^ (uint32_t)((at / kStages) & 1), err, kErrTimeoutFull, lim))
-            return false;
+        // Waits for the next stage and moves on; the stage, or -1.
+        auto next_stage = [&] {
+          const int st = stage;
+          if (!mbar_wait(&full_bar[st], phase, err, kErrTimeoutFull, lim)) return -1;
+          if (++stage == n_stages) { stage = 0; phase ^= 1u; }
           tc_fence_after();
-          return true;
+          return st;
         };
         for (int j = 0; ok && j < kQuadProducts; j++) {
           // The first and the last kSkew blocks go into acc0 before any of them
           // goes into acc1, so the epilogue drains acc0 of this product during
           // the last acc1 blocks, and acc1 during the next product's first acc0
           // blocks: neither side waits for a whole drain.
-          int ki = 0;
-          for (; ok && ki < kSkew; ki++) {
-            ok = stage_full(ki);
-            if (ok && ki == 0) ok = mbar_wait(&acc_empty[0], acc_phase ^ 1u, err, kErrTimeoutAccEmpty, lim2);
-            if (!ok) break;
+          int ki = 0, st[kSkew];
+#pragma unroll
+          for (int i = 0; i < kSkew; i++, ki++) {
+            st[i] = ok ? next_stage() : -1;
+            ok = st[i] >= 0;
+            if (ok && i == 0) ok = mbar_wait(&acc_empty[0], acc_phase ^ 1u, err, kErrTimeoutAccEmpty, lim2);
+            if (!ok) continue;
             tc_fence_after();
-            issue(ki, 0);
+            issue(ki, st[i], 0);
           }
           ok = ok && mbar_wait(&acc_empty[1], acc_phase ^ 1u, err, kErrTimeoutAccEmpty, lim2);
           if (!ok) break;
           acc_phase ^= 1u;
           tc_fence_after();
-          for (int i = 0; i < kSkew; i++) issue(i, 1);
-          for (; ok && ki < k_iters - kSkew; ki++) {
-            ok = stage_full(ki);
+#pragma unroll
+          for (int i = 0; i < kSkew; i++) issue(i, st[i], 1);
+          for (; ki < k_iters - kSkew; ki++) {
+            const int s = next_stage();
+            ok = s >= 0;
             if (!ok) break;
-            issue(ki, 0);
-            issue(ki, 1);
+            issue(ki, s, 0);
+            issue(ki, s, 1);
           }
-          for (; ok && ki < k_iters; ki++) {
-            ok = stage_full(ki);
-            if (ok) issue(ki, 0);
+#pragma unroll
+          for (int i = 0; i < kSkew; i++) {
+            st[i] = ok ? next_stage() : -1;
+            ok = st[i] >= 0;
+            if (ok) issue(ki + i, st[i], 0);
           }
           if (!ok) break;
           mma_commit_pair(&acc_full[0]);
-          for (int i = k_iters - kSkew; i < k_iters; i++) issue(i, 1);
+#pragma unroll
+          for (int i = 0; i < kSkew; i++) issue(ki + i, st[i], 1);
           mma_commit_pair(&acc_full[1]);
-          phase ^= (uint32_t)(((stage + k_iters) / kStages) & 1);
-          stage = (stage + k_iters) % kStages;
         }
       }
       asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -473,6 +488,7 @@ cudaError_t launch_quad_gemm(QuadParams& P, int n_sms, cudaStream_t stream) {
   cudaError_t e = smem_limit_once(quad_gemm_kernel, kSmemBytes, attr_done);
   if (e != cudaSuccess) return e;
   if (P.wait_timeout_ns == 0) P.wait_timeout_ns = kGemmWaitTimeoutNs;
+  P.stages = stage_count(P.tile_n);
   P.total_tiles = 0;
   for (int i = 0; i < P.n_prob; i++) {
     QuadProblem& pr = P.prob[i];

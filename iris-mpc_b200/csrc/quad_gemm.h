@@ -43,6 +43,7 @@ struct QuadParams {
   int n_prob;
   int total_tiles;
   int tile_n;  // quads per tile: a multiple of 32, at most 256
+  int stages;  // filled by launch_quad_gemm
   int* err;
   uint64_t wait_timeout_ns;  // 0 = kGemmWaitTimeoutNs
 };

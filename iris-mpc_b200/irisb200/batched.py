@@ -119,6 +119,11 @@ def pack(variant_rows: list) -> Layout:
         else:
             slots.append([(v, 0, n)])
             fill.append(n)
+    return _layout_of(slots, variant_rows)
+
+
+def _layout_of(slots, variant_rows) -> Layout:
+    """The tables of a placement: slots[s] = [(variant, first row, rows)]."""
     n_slots = len(slots)
     row_desc = np.full(n_slots * 32, 0xFFFFFFFF, np.uint32)
     seg_start = [0]
@@ -132,6 +137,59 @@ def pack(variant_rows: list) -> Layout:
         seg_start.append(len(seg_query))
     return Layout(row_desc, np.array(seg_start, np.uint32), np.array(seg_query, np.uint32),
                   np.array(seg_mask, np.uint32), n_slots * 32, n_slots)
+
+
+QUAD_MIN_ROWS = 576  # padded query rows from which the library's quad GEMM runs
+
+
+def first_quads(occupied: int, n: int) -> int:
+    """Lowest quad of a word (8 of them: rows i, i + 2, i + 4, i + 6 of each
+    octet of rows) where a run of n rows has its quads to itself, or -1.  A run
+    starts at an octet (an even quad), a single row takes any one quad."""
+    need = (1 << (n // 8 * 2 + min(n % 8, 2))) - 1
+    for q in range(0, 8, 1 if n == 1 else 2):
+        if need << q < 1 << 8 and not occupied & need << q:
+            return q
+    return -1
+
+
+def pack_quads(variant_rows: list) -> Layout:
+    """First-fit decreasing packing in which no quad of rows holds rows of two
+    variants, so that the rows qualify for the library's quad GEMM: a few more
+    words than pack(), nine sixteenths of the products."""
+    order = sorted(range(len(variant_rows)), key=lambda v: -len(variant_rows[v]))
+    slots, fill = [], []
+    start = last = 0  # words before `start` have no room for a run as long as the last
+    for v in order:
+        n = len(variant_rows[v])
+        if n != last:
+            start, last = 0, n
+        for s in range(start, len(fill)):
+            q = first_quads(fill[s], n)
+            if q >= 0:
+                break
+        else:
+            s, q = len(fill), 0
+            slots.append([])
+            fill.append(0)
+        start = s
+        slots[s].append((v, q // 2 * 8 + q % 2, n))
+        fill[s] |= (1 << (n // 8 * 2 + min(n % 8, 2))) - 1 << q
+    return _layout_of(slots, variant_rows)
+
+
+def pack_for(variant_rows: list, cap: int) -> Layout:
+    """pack_quads where its rows fit the capacity and the quad GEMM then takes
+    less than the plain one over pack()'s rows (0.75 of the time per padded row:
+    six engines x 32,768 entries, 1024 rows 2.8 against 3.7 ms, 640 rows 2.2
+    against 2.6), else pack."""
+    quads = sum(len(r) // 8 * 2 + min(len(r) % 8, 2) for r in variant_rows)
+    rows, before = padded_rows(-(-quads // 8) * 32, cap), padded_rows(sum(len(r) for r in variant_rows), cap)
+    if QUAD_MIN_ROWS <= rows <= cap and rows * 0.75 < before:
+        layout = pack_quads(variant_rows)
+        if layout.n_rows <= cap:
+            return layout
+    return pack(variant_rows)
 
 
 def attach_bases(layout: Layout, base_of, mirrored) -> Layout:
@@ -348,8 +406,8 @@ class BatchedEngine:
         """Bases, row table and segment table of one pass in the page-locked
         buffers; returns (layout, bases, rows used, segments used)."""
         nb, base_of, mirrored = self._fill_bases(requests, variants, code, mask)
-        layout = attach_bases(pack([list(centred_rotations(requests[i].n_rot)) for i, _ in variants]),
-                              base_of, mirrored)
+        rows_of = [list(centred_rotations(requests[i].n_rot)) for i, _ in variants]
+        layout = attach_bases(pack_for(rows_of, cap) if pad else pack(rows_of), base_of, mirrored)
         if pad:
             layout = pad_rows(layout, cap)
         if layout.n_rows > rows.size:

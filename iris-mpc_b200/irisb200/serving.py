@@ -37,7 +37,8 @@ import numpy as np
 
 from . import (IRIS_CODE_LENGTH, MASK_CODE_LENGTH, MAX_MATCHES_LEN, DistanceComparator, Event, IrisError,
                PinnedArray, ShareDB, dot_many, mirror_query_share)
-from .batched import MULTS, Request, Result, attach_bases, centred_rotations, pack, padded_rows
+from .batched import (MULTS, QUAD_MIN_ROWS, Request, Result, attach_bases, centred_rotations, first_quads, pack,
+                      padded_rows)
 
 RESULT_BYTES_PER_ROW_ENTRY = 2 * 6  # u16 dot share per (row, entry) for 6 engines
 
@@ -70,6 +71,14 @@ def _first_run(occupied: int, n: int) -> int:
     if not x:
         return -1
     return (x & -x).bit_length() - 1
+
+
+def _quads_of(occupied: int) -> int:
+    """The quads (rows i, i + 2, i + 4, i + 6 of an octet) of a word that hold
+    an occupied row: bit 2o + b for octet o's even (b = 0) or odd rows."""
+    x = occupied | occupied >> 2
+    x = (x | x >> 4) & 0x03030303
+    return x & 3 | x >> 6 & 12 | x >> 12 & 48 | x >> 18 & 192
 
 
 @dataclass
@@ -195,6 +204,14 @@ class ContinuousServer:
         return max(1, math.ceil(n / self.chunk))
 
     def _place(self, n: int):
+        """First free run of n rows: once as many words are in use as the
+        library's quad GEMM takes (words fill from the front), with its quads
+        of rows to itself where there is such a run; else any."""
+        if self.row_capacity >= QUAD_MIN_ROWS and self.slot_occ[QUAD_MIN_ROWS // 32 - 3]:
+            for s in range(self.n_slot_cap):
+                q = first_quads(_quads_of(self.slot_occ[s]), n)
+                if q >= 0:
+                    return s, q // 2 * 8 + q % 2
         for s in range(self.n_slot_cap):
             f = _first_run(self.slot_occ[s], n)
             if f >= 0:

@@ -211,3 +211,41 @@ def test_autotuner_candidates():
     assert not any(p == "pair" for p, _, _ in c) and any(p == "fused" for p, _, _ in c)
     c = BatchedEngine._candidates(64, 1000)
     assert c == [("split", 64, 1024)]
+
+
+def _quad_pure(row_desc) -> bool:
+    """No quad (rows i, i + 2, i + 4, i + 6 of an octet) holds rows of two
+    variants, and a quad's rows keep their rotation distance."""
+    for b in range(0, row_desc.size, 8):
+        for i in (b, b + 1):
+            live = [(int(d) >> 7, (int(d) & 0x7F) - 2 * m) for m, d in enumerate(row_desc[i:i + 8:2])
+                    if d != 0xFFFFFFFF]
+            if len(set(live)) > 1:
+                return False
+    return True
+
+
+def test_pack_quads_keeps_quads_apart_and_every_row():
+    from irisb200.batched import QUAD_MIN_ROWS, pack_for, pack_quads
+    rng = np.random.default_rng(2)
+    for _ in range(60):
+        k = int(rng.integers(1, 80))
+        rows = [list(centred_rotations(int(n))) for n in rng.choice([1, 2, 7, 8, 9, 16, 25, 31], k)]
+        lay = pack_quads(rows)
+        assert _quad_pure(lay.row_desc)
+        seen = {v: [] for v in range(k)}
+        for r, d in enumerate(lay.row_desc):
+            if d != 0xFFFFFFFF:
+                seen[int(d) >> 8].append((r, int(d) & 0x7F))
+        for v, want in enumerate(rows):
+            at = [r for r, _ in seen[v]]
+            assert [rot for _, rot in seen[v]] == want and at == list(range(at[0], at[0] + len(want)))
+            j = int(np.nonzero(lay.seg_query == v)[0][0])
+            s = int(np.searchsorted(lay.seg_start, j, side="right")) - 1
+            assert s == at[0] // 32 and int(lay.seg_mask[j]) == ((1 << len(want)) - 1) << (at[0] % 32)
+        # no room for it, or too few rows to pay: the dense packing
+        cap = -(-pack(rows).n_rows // 64) * 64
+        small = pack_for(rows, cap)
+        assert small.n_rows <= cap
+        if lay.n_rows < QUAD_MIN_ROWS - 64:
+            assert np.array_equal(pack_for(rows, 1 << 16).row_desc, pack(rows).row_desc)

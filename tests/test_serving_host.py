@@ -210,3 +210,28 @@ def test_async_host_mode_refuses_temporaries():
     for bad in ([1, 2, 3], a.astype(np.int64), a[::2]):
         with pytest.raises(ValueError):
             _host_arg(dm, bad, np.uint32)
+
+
+def test_placement_in_a_large_server_keeps_quads_apart():
+    from irisb200.serving import _quads_of
+    s = _placer(40)
+    rng = np.random.default_rng(6)
+    vs = []
+    for vid in range(16):  # full words: enough in flight for the quad GEMM
+        s._occupy(_Variant(-1, False, list(range(31))), vid, 0)
+    for vid in range(400):
+        n = int(rng.choice([1, 16, 31, 5]))
+        where = s._place(n)
+        if where is None:
+            break
+        v = _Variant(vid, False, list(range(n)))
+        pure = not _quads_of(s.slot_occ[where[0]]) & _quads_of(((1 << n) - 1) << where[1])
+        s._occupy(v, *where)
+        vs.append((v, pure))
+        if len(vs) > 20 and rng.random() < 0.5:
+            s._release(vs.pop(int(rng.integers(len(vs))))[0])
+    first_mixed = next((i for i, (_, pure) in enumerate(vs) if not pure), len(vs))
+    assert first_mixed > 20  # quads are shared only once the server is nearly full
+    for q in range(8):  # the quads of a word, row by row
+        for r in range(32):
+            assert bool(_quads_of(1 << r) >> (r // 8 * 2 + r % 2) & 1)
