@@ -68,6 +68,7 @@ struct irs_device_manager {
   uint64_t* d_batch = nullptr;  // device batch counter (irs_device_manager_set_batch_counter)
   bool capturing = false;  // a graph capture on streams[0] is open
   cudaEvent_t graph_done = nullptr;  // recorded after each graph launch
+  cudaEvent_t uploads[3] = {nullptr, nullptr, nullptr};  // recorded on the parties' streams before one
   bool host_sync = true;  // false: host-buffer calls return once enqueued (irs_device_manager_set_host_sync)
   // stage timers (irs_device_manager_set_timing): event pairs per label, resolved on read
   bool timing = false;
@@ -153,6 +154,7 @@ struct irs_sharedb {
   CUtensorMap tm_qh_lo{}, tm_qh_hi{};  // half a 256-row tile, for the two-SM GEMM
   int block_n = 0;
   cudaEvent_t done = nullptr;  // recorded after the engine's last dot launch
+  cudaEvent_t copied = nullptr;  // recorded after an upload's last read of host memory
 };
 
 struct irs_circuits {
@@ -360,7 +362,7 @@ size_t forms_bytes(size_t n_cap, size_t K) { return 2 * (kQuadProducts * (n_cap 
 void alloc_sums(irs_sharedb* db) {
   irs_device_manager* dm = db->dm;
   const size_t K = db->code_length, cap = db->db_cap;
-  if (K % kRowLen || db->n_cap < kQuadMinRows || cap < kQuadMinRecords || dm->capturing) return;
+  if (K % kRowLen || !forms_fit(K) || db->n_cap < kQuadMinRows || cap < kQuadMinRecords || dm->capturing) return;
   const size_t forms = forms_bytes(db->n_cap, K), masks = db->n_cap / kSlotRows * 4 + 4;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < sums_bytes(cap, K) + forms + total_b / 6) {
@@ -524,6 +526,7 @@ int irs_device_manager_init(int device, irs_device_manager** out) {
   CU(cudaMalloc(&dm->d_batch, sizeof(uint64_t)));
   CU(cudaMemset(dm->d_batch, 0, sizeof(uint64_t)));
   CU(cudaEventCreateWithFlags(&dm->graph_done, cudaEventDisableTiming));
+  for (cudaEvent_t& e : dm->uploads) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   *out = dm;
   return IRS_OK;
 }
@@ -535,6 +538,8 @@ int irs_device_manager_destroy(irs_device_manager* dm) {
   cudaFree(dm->d_err);
   cudaFree(dm->d_batch);
   if (dm->graph_done) cudaEventDestroy(dm->graph_done);
+  for (cudaEvent_t e : dm->uploads)
+    if (e) cudaEventDestroy(e);
   for (auto& t : dm->timers) {
     cudaEventDestroy(t.start);
     cudaEventDestroy(t.stop);
@@ -786,7 +791,9 @@ int irs_sharedb_init(irs_device_manager* dm, int peer_id, size_t max_db_length, 
   db->n_cap = round_up(query_length, 64);
   db->n_pad = db->n_cap;
   db->block_n = gemm_block_n_for((uint32_t)db->n_pad);
-  if (cudaEventCreateWithFlags(&db->done, cudaEventDisableTiming) != cudaSuccess) {
+  if (cudaEventCreateWithFlags(&db->done, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&db->copied, cudaEventDisableTiming) != cudaSuccess) {
+    if (db->done) cudaEventDestroy(db->done);
     delete db;
     return fail(IRS_ERR_CUDA, "event creation failed");
   }
@@ -824,6 +831,7 @@ int irs_sharedb_destroy(irs_sharedb* db) {
   pool_free(dm, db->peer, db->results);
   cudaStreamSynchronize(dm->streams[db->peer]);
   if (db->done) cudaEventDestroy(db->done);
+  if (db->copied) cudaEventDestroy(db->copied);
   delete db;
   return IRS_OK;
 }
@@ -1056,13 +1064,14 @@ int irs_sharedb_query_upload_slots(irs_sharedb* db, const uint16_t* base, size_t
   CU(cudaMemcpyAsync(db->q_stage, base, n_base * K * 2, cudaMemcpyHostToDevice, s));
   static_assert(sizeof(QuerySlot) == sizeof(irs_query_slot), "slot layout");
   CU(cudaMemcpyAsync(db->d_slots, slots, n_slots * sizeof(QuerySlot), cudaMemcpyHostToDevice, s));
+  CU(cudaEventRecord(db->copied, s));
   {
     std::lock_guard<std::mutex> lock(sum_holders().mu);
     const QuadForms f = begin_forms(db, quad_forms_ready(db));  // a slot's rows are consecutive rotations
     CU(launch_expand_slots(db->q_stage, (uint32_t)K, db->d_slots, (uint32_t)n_slots, (uint32_t)db->n_pad, db->q_lo,
                            db->q_hi, f, s));
   }
-  CU(cudaStreamSynchronize(s));  // slots / base are caller-owned host memory
+  CU(cudaEventSynchronize(db->copied));  // slots / base are caller-owned host memory
   db->have_query = true;
   return IRS_OK;
 }
@@ -1088,8 +1097,9 @@ int irs_sharedb_query_upload_rows(irs_sharedb* db, const uint16_t* base, size_t 
   const size_t table_off = (base_bytes + 15) / 16 * 16;
   CU(cudaMemcpyAsync(stage, base, base_bytes, cudaMemcpyHostToDevice, s));
   CU(cudaMemcpyAsync(stage + table_off, row_desc, table_bytes, cudaMemcpyHostToDevice, s));
+  if (dm->host_sync) CU(cudaEventRecord(db->copied, s));
   if ((rc = expand_row_table(db, row_desc, n_rows, reinterpret_cast<const uint32_t*>(stage + table_off), s))) return rc;
-  if (dm->host_sync) CU(cudaStreamSynchronize(s));  // base / row_desc are caller-owned host memory
+  if (dm->host_sync) CU(cudaEventSynchronize(db->copied));  // base / row_desc are caller-owned host memory
   db->have_query = true;
   return IRS_OK;
 }
@@ -1127,8 +1137,9 @@ int irs_sharedb_query_expand_rows(irs_sharedb* db, size_t n_base, const uint32_t
   uint8_t* stage = reinterpret_cast<uint8_t*>(db->q_stage);
   const size_t table_off = (base_bytes + 15) / 16 * 16;
   CU(cudaMemcpyAsync(stage + table_off, row_desc, table_bytes, cudaMemcpyHostToDevice, s));
+  if (dm->host_sync) CU(cudaEventRecord(db->copied, s));
   if ((rc = expand_row_table(db, row_desc, n_rows, reinterpret_cast<const uint32_t*>(stage + table_off), s))) return rc;
-  if (dm->host_sync) CU(cudaStreamSynchronize(s));  // row_desc is caller-owned host memory
+  if (dm->host_sync) CU(cudaEventSynchronize(db->copied));  // row_desc is caller-owned host memory
   db->have_query = true;
   return IRS_OK;
 }
@@ -1149,6 +1160,7 @@ int irs_sharedb_gather_records(irs_sharedb* dst, irs_sharedb* src, const uint32_
   CHECK(n * 4 <= dst->n_cap * K * 2, IRS_ERR_INVALID, "too many records for one gather");
   // Staging reuse: the gather runs before the next query upload of `dst`.
   CU(cudaMemcpyAsync(dst->q_stage, ids, n * 4, cudaMemcpyHostToDevice, s));
+  if (dm->host_sync) CU(cudaEventRecord(dst->copied, s));
   CU(launch_gather_rows(src->db_lo, src->db_hi, reinterpret_cast<const uint32_t*>(dst->q_stage), (uint32_t)n,
                         (uint32_t)K, dst->db_lo, dst->db_hi, s));
   if (dst->sums && gather_skips_sums(dst, n)) {
@@ -1157,7 +1169,7 @@ int irs_sharedb_gather_records(irs_sharedb* dst, irs_sharedb* src, const uint32_
     CU(update_sums(dst, 0, n, s));
     if (n >= dst->stale_end) dst->stale_end = 0;
   }
-  if (dm->host_sync) CU(cudaStreamSynchronize(s));  // ids is caller-owned host memory
+  if (dm->host_sync) CU(cudaEventSynchronize(dst->copied));  // ids is caller-owned host memory
   dst->db_len = n;
   return IRS_OK;
 }
@@ -2000,6 +2012,12 @@ int irs_graph_end_capture(irs_device_manager* dm, irs_graph** out) {
 
 int irs_graph_launch(irs_graph* g, void* stream) {
   CHECK(g && g->exec, IRS_ERR_INVALID, "graph is NULL");
+  // the graph's GEMMs read what the parties' streams have uploaded
+  for (int p = 0; p < 3; p++)
+    if (g->dm->streams[p] != static_cast<cudaStream_t>(stream)) {
+      CU(cudaEventRecord(g->dm->uploads[p], g->dm->streams[p]));
+      CU(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), g->dm->uploads[p], 0));
+    }
   CU(cudaGraphLaunch(g->exec, static_cast<cudaStream_t>(stream)));
   // later query uploads on other party streams wait for the graph's GEMMs
   CU(cudaEventRecord(g->dm->graph_done, static_cast<cudaStream_t>(stream)));

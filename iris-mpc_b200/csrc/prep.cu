@@ -166,76 +166,89 @@ __device__ __forceinline__ void put_octet(uint8_t* lo, uint8_t* hi, size_t at, u
 }
 
 // The query planes of n_pad rows and, when `quads.lo` is set, the query forms
-// of the rotation-structured GEMM beside them (blocks from plain_blocks on).
+// of the rotation-structured GEMM beside them: one block per row (the first
+// n_pad) or quad.
 //
-// Planes: one thread per (row, octet).  A rotated row's column c reads base
-// column c + 15 - rot (mod 200).
+// Planes: a rotated row's column c reads base column c + 15 - rot (mod 200).
 //
-// Forms (quad_gemm.cu): planes [9 products][n_pad / 4 quads][K / 4], one thread
-// per (quad, octet of a quarter).  Quad s of a slot is rows i, i + 2, i + 4,
-// i + 6 with i = 16 s2 + 8 s1 + s0 (the bits of s); its live rows are rotations
-// of one query that keep their distance (the caller checked), so row i stands
-// for rotation `rot` even where it is not live itself.  With f(k) the query at
-// column offset c - rot shifted by 2k columns (column c of quarter 0), the
-// forms are the outer and inner differences x: f(+D) - f, y: f(-D) - f at D = 4
-// and D = 2, "2": f itself.  Quads without a live row are zero.
+// Forms (quad_gemm.cu): planes [9 products][n_pad / 4 quads][K / 4].  Quad s of
+// a slot is rows i, i + 2, i + 4, i + 6 with i = 16 s2 + 8 s1 + s0 (the bits of
+// s); its live rows are rotations of one query that keep their distance (the
+// caller checked), so row i stands for rotation `rot` even where it is not live
+// itself.  With f(k) the query at column offset c - rot shifted by 2k columns
+// (column c of quarter 0), the forms are the outer and inner differences x:
+// f(+D) - f, y: f(-D) - f at D = 4 and D = 2, "2": f itself.  Quads without a
+// live row are zero.
+//
+// Bound by the strided half of the transfer: planes read the query in order and
+// write 64-byte runs of each quarter (reading with a stride to write in order
+// was a third slower), forms read it from shared memory.  64 queries of a code,
+// planes and forms (82 MB written, cold): 32 us, against 46 us with a thread per
+// octet of the whole grid and every division it takes.
 template <class Rows>
 __global__ void expand_kernel(const uint16_t* __restrict__ base, uint32_t K, Rows rows, uint32_t n_pad,
-                              uint8_t* __restrict__ lo, uint8_t* __restrict__ hi, uint32_t plain_blocks, QuadForms quads) {
-  if (blockIdx.x < plain_blocks) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t per = K / 8;
-    if (i == 0 && quads.flag) *quads.flag = quads.lo ? 1u : 0u;
-    if (i >= (size_t)n_pad * per) return;
-    const uint32_t row = (uint32_t)(i / per), o = (uint32_t)(i % per);
-    const RowSource q = rows(row);
-    uint2 a = make_uint2(0u, 0u), b = a;
-    if (q.live) {
-      const uint32_t row800 = o / 100;
-      const int col = (int)(o % 100) * 2 + 15 - q.rot;
-      a = query_column(base, K, q, row800, col);
-      b = query_column(base, K, q, row800, col + 1);
+                              uint8_t* __restrict__ lo, uint8_t* __restrict__ hi, QuadForms quads) {
+  const uint32_t per_quarter = K / 32;
+  if (blockIdx.x < n_pad) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && quads.flag) *quads.flag = quads.lo ? 1u : 0u;
+    const uint32_t row = blockIdx.x;
+    const RowSource src = rows(row);
+    for (uint32_t o = threadIdx.x; o < 4 * per_quarter; o += blockDim.x) {
+      uint2 a = make_uint2(0u, 0u), b = a;
+      if (src.live) {
+        const int col = (int)(o % 100) * 2 + 15 - src.rot;
+        a = query_column(base, K, src, o / 100, col);
+        b = query_column(base, K, src, o / 100, col + 1);
+      }
+      put_octet(lo, hi, (size_t)row * 4 * per_quarter + plane_octet(o, K), a, b);
     }
-    put_octet(lo, hi, (size_t)row * per + plane_octet(o, K), a, b);
     return;
   }
-  const size_t i = (size_t)(blockIdx.x - plain_blocks) * blockDim.x + threadIdx.x;
-  const uint32_t per = K / 32, n_quads = n_pad / 4;
-  if (i >= (size_t)n_quads * per) return;
-  const uint32_t p = (uint32_t)(i / per), g = (uint32_t)(i % per);
-  if (g == 0 && (p & 7u) == 0) {  // the rows of this slot that hold a query row
-    uint32_t bits = 0;
-    for (uint32_t r = 0; r < (uint32_t)kSlotRows; r++) bits |= (uint32_t)rows((p >> 3) * kSlotRows + r).live << r;
-    quads.valid[p >> 3] = bits;
+  const uint32_t n_quads = n_pad / 4, p = blockIdx.x - n_pad;
+  if (threadIdx.x < 32 && (p & 7u) == 0) {  // the rows of this slot that hold a query row
+    const uint32_t bits = __ballot_sync(0xFFFFFFFFu, rows((p >> 3) * kSlotRows + threadIdx.x).live);
+    if (threadIdx.x == 0) quads.valid[p >> 3] = bits;
   }
   const uint32_t row0 = (p >> 3) * kSlotRows + ((p >> 2) & 1u) * 16 + ((p >> 1) & 1u) * 8 + (p & 1u);
-  RowSource q{0u, false, false, 0};
+  RowSource src{0u, false, false, 0};
 #pragma unroll
   for (int m = 3; m >= 0; m--) {
     const RowSource r = rows(row0 + 2 * m);
-    if (r.live) q = {r.src, r.mirror, true, r.rot - 2 * m};
+    if (r.live) src = {r.src, r.mirror, true, r.rot - 2 * m};
   }
-  uint2 f[7][2];  // f(k - 3), the octet's two columns
+  // The query, rotated by `rot` columns, in shared memory: column c of a row at
+  // c + c / 8, so that threads eight columns apart read different banks.
+  extern __shared__ uint2 query[];
+  for (uint32_t i = threadIdx.x; src.live && i < K / 4; i += blockDim.x) {
+    const uint32_t row800 = i / 200, c = i % 200;
+    query[row800 * 225 + c + c / 8] = query_column(base, K, src, row800, (int)c + 15 - src.rot);
+  }
+  __syncthreads();
+  for (uint32_t g = threadIdx.x; g < per_quarter; g += blockDim.x) {
+    uint2 f[7][2];  // f(k - 3), the octet's two columns
 #pragma unroll
-  for (int k = 0; k < 7; k++)
+    for (int k = 0; k < 7; k++)
 #pragma unroll
-    for (int c = 0; c < 2; c++)
-      f[k][c] = q.live ? query_column(base, K, q, g / 25, (int)(g % 25) * 8 + c + 2 * (k - 3) + 15 - q.rot)
-                       : make_uint2(0u, 0u);
+      for (int c = 0; c < 2; c++) {
+        const uint32_t col = ((g % 25) * 8 + (uint32_t)(c + 2 * (k - 3) + 200)) % 200;
+        f[k][c] = src.live ? query[g / 25 * 225 + col + col / 8] : make_uint2(0u, 0u);
+      }
 #pragma unroll
-  for (int j = 0; j < 9; j++) {
-    // terms of product j (outer, inner) = 22 2x 2y x2 xx xy y2 yx yy
-    const int o = j / 3 == 0 ? 0 : (j / 3 == 1 ? 2 : -2), n = j % 3 == 0 ? 0 : (j % 3 == 1 ? 1 : -1);
-    uint32_t w[4];
+    for (int j = 0; j < 9; j++) {
+      // terms of product j (outer, inner) = 22 2x 2y x2 xx xy y2 yx yy
+      const int o = j / 3 == 0 ? 0 : (j / 3 == 1 ? 2 : -2), n = j % 3 == 0 ? 0 : (j % 3 == 1 ? 1 : -1);
+      auto form = [&](auto at) {  // at(k) = f(k)
+        uint32_t v = at(0);
+        if (n) v = sub2(at(n), v);
+        if (o) v = sub2(n ? sub2(at(o + n), at(o)) : at(o), v);
+        return v;
+      };
+      uint2 w[2];
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      auto at = [&](int k) { return (e & 1) ? f[k + 3][e >> 1].y : f[k + 3][e >> 1].x; };
-      uint32_t v = at(0);
-      if (n) v = sub2(at(n), v);
-      if (o) v = sub2(n ? sub2(at(o + n), at(o)) : at(o), v);
-      w[e] = v;
+      for (int c = 0; c < 2; c++)
+        w[c] = make_uint2(form([&](int k) { return f[k + 3][c].x; }), form([&](int k) { return f[k + 3][c].y; }));
+      put_octet(quads.lo, quads.hi, ((size_t)j * n_quads + p) * per_quarter + g, w[0], w[1]);
     }
-    put_octet(quads.lo, quads.hi, ((size_t)j * n_quads + p) * per + g, make_uint2(w[0], w[1]), make_uint2(w[2], w[3]));
   }
 }
 
@@ -380,13 +393,15 @@ cudaError_t launch_derive_sums(const uint8_t* lo, const uint8_t* hi, uint32_t K,
   return cudaGetLastError();
 }
 
+bool forms_fit(size_t K) { return K / kRowLen * 225 * sizeof(uint2) <= 48 * 1024; }
+
 template <class Rows>
 static cudaError_t launch_expand(const uint16_t* base, uint32_t K, Rows rows, uint32_t n_pad, uint8_t* lo, uint8_t* hi,
                                  const QuadForms& quads, cudaStream_t stream) {
-  const size_t plain = ((size_t)n_pad * (K / 8) + 255) / 256;
-  const size_t forms = quads.lo ? ((size_t)(n_pad / 4) * (K / 32) + 255) / 256 : 0;
-  if (!plain) return cudaSuccess;
-  expand_kernel<<<(unsigned)(plain + forms), 256, 0, stream>>>(base, K, rows, n_pad, lo, hi, (uint32_t)plain, quads);
+  if (!n_pad) return cudaSuccess;
+  const size_t smem = quads.lo ? (size_t)K / kRowLen * 225 * sizeof(uint2) : 0;  // 28,800 bytes for a code
+  if (quads.lo && !forms_fit(K)) return cudaErrorInvalidValue;
+  expand_kernel<<<n_pad + (quads.lo ? n_pad / 4 : 0), 256, smem, stream>>>(base, K, rows, n_pad, lo, hi, quads);
   return cudaGetLastError();
 }
 

@@ -35,6 +35,8 @@ cudaError_t launch_split_limbs(const uint16_t* in, uint32_t K, uint8_t* lo, uint
 cudaError_t launch_i8_plane(const uint8_t* in, uint32_t K, uint8_t* out, size_t n, cudaStream_t stream);
 cudaError_t launch_derive_sums(const uint8_t* lo, const uint8_t* hi, uint32_t K, size_t n, uint8_t* outer_lo,
                                uint8_t* outer_hi, uint8_t* inner_lo, uint8_t* inner_hi, cudaStream_t stream);
+// Whether the forms of queries of K coefficients can be expanded (K up to 21,600).
+bool forms_fit(size_t K);
 // Query planes of n_pad rows, and the query forms where quads.lo is set.
 cudaError_t launch_expand_slots(const uint16_t* base, uint32_t K, const QuerySlot* slots, uint32_t n_slots,
                                 uint32_t n_pad, uint8_t* lo, uint8_t* hi, const QuadForms& quads, cudaStream_t stream);
