@@ -260,12 +260,17 @@ int irs_mirror_query_share(uint16_t* coefs, size_t n, int flip_imaginary);
  * reference, where cuBLAS picks its own tiles).  The padded row count of a
  * batch is its uploaded rows rounded up to 64, and further to 128 (up to 768
  * rows) or 256 (above) when the query capacity allows; the extra rows are zero.
- * Default: the 128-row tile up to 768 padded rows, else the 256-row tile. */
+ * Default: the 64-row tile for 64 padded rows, up to 768 the two-SM GEMM (or
+ * 128-row tiles in launches of few tiles), above that the 256-row tile, and the
+ * rotation-structured GEMM where the uploaded rows and the launch suit it; a
+ * width given here runs the one-SM GEMM.  The dot shares do not depend on it. */
 int irs_sharedb_set_tile(irs_sharedb* db, int block_n);
-/* on != 0: the 256-row tile runs as the two-SM GEMM (a cluster of two CTAs
- * with tcgen05.mma.cta_group::2 on a 256-entry x 256-row tile; same results).
- * Off by default: under the B200's power cap it trades clock for MAC rate, so
- * the batch autotuner decides (no counterpart in the reference). */
+/* on != 0: the GEMM runs on SM pairs wherever it can (a cluster of two CTAs with
+ * tcgen05.mma.cta_group::2 on a tile of 256 entries and up to 256 rows; same
+ * results), the rotation-structured GEMM included.  Off by default, which leaves
+ * the choice to the library: under the B200's power cap long launches of many
+ * rows trade clock for MAC rate, so the batch autotuner decides there (no
+ * counterpart in the reference). */
 int irs_sharedb_set_pair(irs_sharedb* db, int on);
 int irs_sharedb_use_batch_counter(irs_sharedb* db, int on);
 /* Starts a new batch: the zero-share mask and circuit keystreams are drawn at

@@ -9,6 +9,7 @@
 #include <stdarg.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <stdlib.h>
 #include <string.h>
 
 #include <algorithm>
@@ -151,7 +152,8 @@ struct irs_sharedb {
   CUtensorMap tm_sum_lo[2]{}, tm_sum_hi[2]{}, tm_form_lo[kQuadWidths]{},
       tm_form_hi[kQuadWidths]{};
   CUtensorMap tm_db_lo{}, tm_db_hi{}, tm_q_lo{}, tm_q_hi{};
-  CUtensorMap tm_qh_lo{}, tm_qh_hi{};  // half a 256-row tile, for the two-SM GEMM
+  CUtensorMap tm_qp_lo{}, tm_qp_hi{};    // half a tile of the two-SM GEMM
+  CUtensorMap tm_q128_lo{}, tm_q128_hi{};  // 128 rows, for launches of few tiles
   int block_n = 0;
   cudaEvent_t done = nullptr;  // recorded after the engine's last dot launch
   cudaEvent_t copied = nullptr;  // recorded after an upload's last read of host memory
@@ -318,10 +320,13 @@ ChaChaKey key_of(const uint32_t k[8]) {
 int rebuild_query_maps(irs_sharedb* db) {
   if (db->block_n <= 0) return IRS_OK;  // no valid tile width: dot reports it
   const uint32_t box = (uint32_t)db->block_n;
+  const uint32_t half = (uint32_t)gemm_pair_n((uint32_t)db->n_pad) / 2;
   if (make_tmap_u8(&db->tm_q_lo, db->q_lo, db->n_cap, db->code_length, box) ||
       make_tmap_u8(&db->tm_q_hi, db->q_hi, db->n_cap, db->code_length, box) ||
-      make_tmap_u8(&db->tm_qh_lo, db->q_lo, db->n_cap, db->code_length, box / 2) ||
-      make_tmap_u8(&db->tm_qh_hi, db->q_hi, db->n_cap, db->code_length, box / 2))
+      make_tmap_u8(&db->tm_qp_lo, db->q_lo, db->n_cap, db->code_length, half) ||
+      make_tmap_u8(&db->tm_qp_hi, db->q_hi, db->n_cap, db->code_length, half) ||
+      make_tmap_u8(&db->tm_q128_lo, db->q_lo, db->n_cap, db->code_length, 128) ||
+      make_tmap_u8(&db->tm_q128_hi, db->q_hi, db->n_cap, db->code_length, 128))
     return fail(IRS_ERR_CUDA, "tensor map for the query planes failed");
   return IRS_OK;
 }
@@ -478,7 +483,7 @@ int set_active_rows(irs_sharedb* db, size_t rows) {
   if (n != db->n_pad) db->quad_rows = false;  // the forms are for another row count; the upload decides
   int bn = gemm_block_n_for((uint32_t)n);
   if (db->tile_override && n % (size_t)db->tile_override == 0) bn = db->tile_override;
-  const bool rebuild = bn != db->block_n;
+  const bool rebuild = bn != db->block_n || n != db->n_pad;
   db->n_pad = n;
   db->block_n = bn;
   db->rows_uploaded = rows;
@@ -1196,8 +1201,10 @@ int irs_sharedb_set_batch(irs_sharedb* db, uint64_t batch_id) {
   return IRS_OK;
 }
 
-// half_tile: the query maps load 128 of a 256-row tile's rows.
-static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t len, bool half_tile, GemmProblem& pr) {
+// The GEMM that a launch's query maps are for.
+enum class Gemm { kOneSm, kPair, kFewTiles };
+
+static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t len, Gemm gemm, GemmProblem& pr) {
   CHECK(db->db_lo, IRS_ERR_STATE, "alloc_db not called");
   CHECK(db->have_query, IRS_ERR_STATE, "no query uploaded");
   CHECK(offset % 32 == 0, IRS_ERR_INVALID, "offset %zu must be a multiple of 32", offset);
@@ -1207,8 +1214,8 @@ static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t le
   memset(&pr, 0, sizeof pr);
   pr.tm_a_lo = db->tm_db_lo;
   pr.tm_a_hi = db->tm_db_hi;
-  pr.tm_b_lo = half_tile ? db->tm_qh_lo : db->tm_q_lo;
-  pr.tm_b_hi = half_tile ? db->tm_qh_hi : db->tm_q_hi;
+  pr.tm_b_lo = gemm == Gemm::kPair ? db->tm_qp_lo : gemm == Gemm::kFewTiles ? db->tm_q128_lo : db->tm_q_lo;
+  pr.tm_b_hi = gemm == Gemm::kPair ? db->tm_qp_hi : gemm == Gemm::kFewTiles ? db->tm_q128_hi : db->tm_q_hi;
   pr.out = db->results;
   pr.m0 = (uint32_t)offset;
   pr.m_len = (uint32_t)len;
@@ -1235,21 +1242,35 @@ static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t 
   for (int i = 0; i < n; i++) {
     const irs_sharedb* e = engines[i];
     if (!e->sums || e->n_pad != engines[0]->n_pad || e->forms_pad != e->n_pad || offset < e->stale_end) return -1;
-    if (e->tile_override && !gemm_pair_applies(e->pair, e->block_n)) return -1;
+    if (e->tile_override && !gemm_pair_applies(e->pair, (uint32_t)e->n_pad)) return -1;
     K[i] = (uint32_t)e->code_length;
   }
   const irs_sharedb* e = engines[0];
   return quad_width_for(K, n, (uint32_t)len, (uint32_t)e->n_pad, e->block_n, pair, e->dm->n_sms);
 }
 
-// Whether the plain GEMM of a launch runs on SM pairs: where the caller chose
-// it, and, where the caller left the GEMM open, for launches short enough that
-// the clock has not dropped to the power limit.  One engine x 960 rows x 32,768
-// entries: 0.73 ms, one-SM 0.81; 1984 rows 1.51 / 1.60; 832 rows 0.70 / 0.78.
-// Six engines x 1024 rows x 32,768 entries: 3.79 / 3.69.
+// Tiles of 128 entries x 128 query rows of a launch.
+static size_t tiles_128(irs_sharedb* const* engines, int n, size_t len) {
+  return (size_t)n * ((len + 127) / 128) * ((engines[0]->n_pad + 127) / 128);
+}
+
+// Whether the plain GEMM of a launch runs on SM pairs.  Six engines x 32,768
+// entries, one-SM against pair: 128 rows 0.86 / 0.87 ms, 192 1.32 / 1.01, 256
+// 1.37 / 1.18, 384 1.93 / 1.74, 512 2.46 / 2.10, 768 3.58 / 3.03, 960 4.18 /
+// 4.25, 1024 4.24 / 3.94; at 65,536 entries the last two are 8.6 / 9.0 and 8.4 /
+// 8.0.  So from 192 to 768 rows it is the default, as far as there are more
+// 128-row tiles than SMs (4,000 entries x 512 rows of one engine: 0.072 / 0.110
+// ms); above, where the caller chose it or the launch is short enough that the
+// clock has not dropped to the power limit (one engine x 32,768 entries, 960
+// rows 0.94 / 0.89, 1984 rows 1.60 / 1.51).
 static bool plain_pair(irs_sharedb* const* engines, int n, size_t len) {
   const irs_sharedb* e = engines[0];
-  if (e->pair || e->tile_override || e->block_n != 256) return gemm_pair_applies(e->pair, e->block_n);
+  if (!gemm_pair_applies(true, (uint32_t)e->n_pad) || (e->tile_override && !e->pair)) return false;
+  for (int i = 1; i < n; i++)
+    if (engines[i]->n_pad != e->n_pad) return false;  // one tile width for the launch
+  if (e->n_pad <= 768)
+    return tiles_128(engines, n, len) > (size_t)e->dm->n_sms && (e->pair || e->n_pad >= 192);
+  if (e->pair) return true;
   double macs = 0;
   for (int i = 0; i < n; i++) macs += 3.0 * (double)engines[i]->code_length * (double)e->n_pad * (double)len;
   return macs < 3e12;  // about 2 ms
@@ -1263,7 +1284,7 @@ static bool few_tiles(irs_sharedb* const* engines, int n, size_t len) {
   if (e->pair || e->tile_override || e->block_n != 256) return false;
   for (int i = 0; i < n; i++)
     if (engines[i]->n_pad != e->n_pad || engines[i]->code_length < 8 * 128) return false;
-  return 3 * (size_t)n * ((len + 127) / 128) * ((e->n_pad + 127) / 128) <= 2 * (size_t)e->dm->n_sms;
+  return 3 * tiles_128(engines, n, len) <= 2 * (size_t)e->dm->n_sms;
 }
 
 static void fill_quad_problem(const irs_sharedb* db, const GemmProblem& g, int width, QuadProblem& pr) {
@@ -1309,7 +1330,8 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
   const bool few = !stall && few_tiles(engines, n, len);
   const bool pair = !stall && !few && plain_pair(engines, n, len);
   for (int i = 0; i < n; i++) {
-    int rc = fill_problem(engines[i], multipliers[i], offset, len, pair || few, P.prob[i]);
+    int rc = fill_problem(engines[i], multipliers[i], offset, len,
+                          pair ? Gemm::kPair : few ? Gemm::kFewTiles : Gemm::kOneSm, P.prob[i]);
     if (rc) return rc;
   }
   cudaStream_t s = party_stream(dm, engines[0]->peer, stream);
@@ -1906,7 +1928,7 @@ int irs_dc_scan_fused(irs_distance_comparator* dc, irs_circuits* c, irs_sharedb*
   memset(&F, 0, sizeof F);
   const uint16_t mults[kFusedEngines] = {1, 1, 1, 2, 2, 2};
   for (int e = 0; e < kFusedEngines; e++) {
-    int rc = fill_problem(eng[e], mults[e], offset, len, false, F.prob[e]);
+    int rc = fill_problem(eng[e], mults[e], offset, len, Gemm::kOneSm, F.prob[e]);
     if (rc) return rc;
     // the fused kernel's query tile is 128 rows whatever the engine's own tile width
     if (make_tmap_u8(&F.prob[e].tm_b_lo, eng[e]->q_lo, eng[e]->n_cap, eng[e]->code_length, kFusedBlockN) ||

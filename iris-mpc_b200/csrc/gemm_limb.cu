@@ -129,14 +129,13 @@ __global__ void __launch_bounds__(kThreads, 1) limb_gemm_kernel(const __grid_con
       // Test hook (GemmParams::test_stall): CTA 0 issues no loads at all, so
       // its MMA's first stage wait runs out.  Nothing is in flight to drain.
       if (P.test_stall && blockIdx.x == 0) ok = false;
-      int it = 0;
-      for (int t = blockIdx.x; ok && t < P.total_tiles; t += gridDim.x, it++) {
+      for (int k = 0; ok && k * (int)gridDim.x < P.total_tiles; k++) {
         Tile tl;
-        if (!tile_of(P, t, tl)) break;
+        if (!tile_of(P, tile_index(k, blockIdx.x, gridDim.x), tl)) continue;
         const GemmProblem& pr = P.prob[tl.prob];
         const int ya = (int)pr.m0 + tl.m_tile * kBM;
         const int yb = tl.n_tile * BN;
-        const bool rev = P.serpentine && (it & 1);
+        const bool rev = P.serpentine && (k & 1);
         for (uint32_t ki = 0; ki < pr.k_iters; ki++) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, err, kErrTimeoutEmpty, lim2)) { ok = false; break; }
           mbar_expect_tx(&full_bar[stage], (uint32_t)C::kStageBytes);
@@ -169,9 +168,9 @@ __global__ void __launch_bounds__(kThreads, 1) limb_gemm_kernel(const __grid_con
       uint32_t acc_phase = 0;
       bool ok = true;
       constexpr uint32_t idesc = idesc_u8(BN);
-      for (int t = blockIdx.x; ok && t < P.total_tiles; t += gridDim.x) {
+      for (int k = 0; ok && k * (int)gridDim.x < P.total_tiles; k++) {
         Tile tl;
-        if (!tile_of(P, t, tl)) break;
+        if (!tile_of(P, tile_index(k, blockIdx.x, gridDim.x), tl)) continue;
         const GemmProblem& pr = P.prob[tl.prob];
         if (!mbar_wait(acc_empty, acc_phase ^ 1u, err, kErrTimeoutAccEmpty, lim2)) { ok = false; break; }
         acc_phase ^= 1u;
@@ -207,9 +206,9 @@ __global__ void __launch_bounds__(kThreads, 1) limb_gemm_kernel(const __grid_con
     const int row = quad * 32 + lane;          // entry within the tile
     constexpr int kCols = C::kColsPerThread;
     uint32_t acc_phase = 0;
-    for (int t = blockIdx.x; t < P.total_tiles; t += gridDim.x) {
+    for (int k = 0; k * (int)gridDim.x < P.total_tiles; k++) {
       Tile tl;
-      if (!tile_of(P, t, tl)) break;
+      if (!tile_of(P, tile_index(k, blockIdx.x, gridDim.x), tl)) continue;
       const GemmProblem& pr = P.prob[tl.prob];
       if (!mbar_wait(acc_full, acc_phase, err, kErrTimeoutAccFull, lim2)) break;
       acc_phase ^= 1u;
@@ -283,45 +282,29 @@ __global__ void __launch_bounds__(kThreads, 1) limb_gemm_kernel(const __grid_con
 // accumulator barriers are released to both CTAs with multicast commits; the
 // follower's epilogue releases the accumulator on the leader's barrier.
 // ---------------------------------------------------------------------------
-struct Cfg2 {
-  static constexpr int BN = 256;
-  static constexpr int kHalfN = BN / 2;
-  static constexpr int kStageBytes = 2 * 128 * kBK + 2 * kHalfN * kBK;  // per CTA
-  static constexpr int kStages = 3;
-  static constexpr int kTmemCols = 2 * BN;
-  static constexpr int kColsPerThread = BN / 2;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
-};
-
-__device__ __forceinline__ bool tile_of2(const GemmParams& P, int t, Tile& out) {
-  for (int i = 0; i < P.n_prob; i++) {
-    const int nt = (int)(P.prob[i].tiles_m * P.prob[i].tiles_n);
-    if (t < nt) {
-      out.prob = i;
-      out.m_tile = t / (int)P.prob[i].tiles_n;
-      out.n_tile = t % (int)P.prob[i].tiles_n;
-      return true;
-    }
-    t -= nt;
-  }
-  return false;
-}
+// Tiles are 64 to 256 rows wide, in multiples of 64 (an epilogue half then holds
+// whole keystream blocks), a problem's as equal as that allows.
+constexpr int kPairRoom = 225 * 1024;  // shared memory for the stages
+constexpr int kPairMaxStages = 5;
+constexpr int kPairMaxN = 256;
+constexpr int kPairSmem = kPairRoom + 1024 /*align*/ + 256 /*barriers*/;
+constexpr int pair_stage_bytes(int bn) { return 2 * 128 * kBK + 2 * (bn / 2) * kBK; }  // per CTA
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     limb_gemm_pair_kernel(const __grid_constant__ GemmParams P) {
-  using C = Cfg2;
-  constexpr int BN = C::BN;
   if (P.skip.n && P.skip.all_set()) return;  // the quad GEMM runs; the same words for every CTA
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int n_stages = P.pair_stages;
+  const int b_bytes = P.pair_n / 2 * kBK;  // one limb of a CTA's half of the query rows
   uint8_t* a_lo = smem;
-  uint8_t* a_hi = a_lo + C::kStages * 128 * kBK;
-  uint8_t* b_lo = a_hi + C::kStages * 128 * kBK;
-  uint8_t* b_hi = b_lo + C::kStages * C::kHalfN * kBK;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(b_hi + C::kStages * C::kHalfN * kBK);
+  uint8_t* a_hi = a_lo + n_stages * 128 * kBK;
+  uint8_t* b_lo = a_hi + n_stages * 128 * kBK;
+  uint8_t* b_hi = b_lo + n_stages * b_bytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kPairRoom);
   uint64_t* full_bar = bars;
-  uint64_t* empty_bar = bars + C::kStages;
-  uint64_t* acc_full = bars + 2 * C::kStages;
+  uint64_t* empty_bar = bars + kPairMaxStages;
+  uint64_t* acc_full = bars + 2 * kPairMaxStages;
   uint64_t* acc_empty = acc_full + 1;
   uint64_t* done_bar = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 3);
@@ -332,11 +315,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   const bool leader = rank == 0;
   const int cluster = blockIdx.x >> 1;
   const int n_clusters = gridDim.x >> 1;
+  // A problem's rows, in units of 64, dealt out over its tiles: the first
+  // `wider` are pair_n rows, the others 64 fewer.
+  auto tile_width = [&](const Tile& tl) { return P.pair_n - (tl.n_tile < P.pair_wider ? 0 : 64); };
+  auto tile_row = [&](const Tile& tl) {
+    return tl.n_tile * P.pair_n - (tl.n_tile > P.pair_wider ? 64 * (tl.n_tile - P.pair_wider) : 0);
+  };
   int* err = P.err;
   const uint64_t lim = P.wait_timeout_ns, lim2 = 2 * P.wait_timeout_ns;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < C::kStages; s++) {
+    for (int s = 0; s < n_stages; s++) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
@@ -347,7 +336,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"((uint32_t)C::kTmemCols));
+                 "r"(512u));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
   }
   tc_fence_before();
@@ -361,37 +350,34 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      int issued_phase[C::kStages];
-      bool issued[C::kStages];
-      for (int s = 0; s < C::kStages; s++) issued[s] = false;
+      uint32_t issued_phase = 0, issued = 0;  // bit s: stage s
       bool ok = true;
-      int it = 0;  // both CTAs of a pair walk the same tiles, so they agree on the order
-      for (int t = cluster; ok && t < P.total_tiles; t += n_clusters, it++) {
+      for (int k = 0; ok && k * n_clusters < P.total_tiles; k++) {
         Tile tl;
-        if (!tile_of2(P, t, tl)) break;
+        if (!tile_of(P, tile_index(k, cluster, n_clusters), tl)) continue;
         const GemmProblem& pr = P.prob[tl.prob];
         const int ya = (int)pr.m0 + tl.m_tile * kBM2 + (int)rank * 128;
-        const int yb = tl.n_tile * BN + (int)rank * C::kHalfN;
-        const bool rev = P.serpentine && (it & 1);
+        const int yb = tile_row(tl) + (int)rank * (tile_width(tl) / 2);
+        const bool rev = P.serpentine && (k & 1);
         for (uint32_t ki = 0; ki < pr.k_iters; ki++) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1u, err, kErrTimeoutEmpty, lim2)) { ok = false; break; }
-          if (leader) mbar_expect_tx(&full_bar[stage], (uint32_t)(2 * C::kStageBytes));
+          if (leader) mbar_expect_tx(&full_bar[stage], (uint32_t)(2 * pair_stage_bytes(P.pair_n)));
           const uint32_t fb = map_to_rank(&full_bar[stage], 0);
           const int x = (int)(rev ? pr.k_iters - 1 - ki : ki) * kBK;
           tma_load_2d_pair(a_lo + stage * 128 * kBK, &pr.tm_a_lo, fb, x, ya);
           tma_load_2d_pair(a_hi + stage * 128 * kBK, &pr.tm_a_hi, fb, x, ya);
-          tma_load_2d_pair(b_lo + stage * C::kHalfN * kBK, &pr.tm_b_lo, fb, x, yb);
-          tma_load_2d_pair(b_hi + stage * C::kHalfN * kBK, &pr.tm_b_hi, fb, x, yb);
-          issued[stage] = true;
-          issued_phase[stage] = (int)phase;
-          if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
+          tma_load_2d_pair(b_lo + stage * b_bytes, &pr.tm_b_lo, fb, x, yb);
+          tma_load_2d_pair(b_hi + stage * b_bytes, &pr.tm_b_hi, fb, x, yb);
+          issued |= 1u << stage;
+          issued_phase = (issued_phase & ~(1u << stage)) | phase << stage;
+          if (++stage == n_stages) { stage = 0; phase ^= 1u; }
         }
       }
       // Exit: the leader's stage barriers complete only when both CTAs' copies
       // of that stage have landed.
       if (leader)
-        for (int s = 0; s < C::kStages; s++)
-          if (issued[s]) mbar_wait_drain(&full_bar[s], (uint32_t)issued_phase[s], err, lim2);
+        for (int s = 0; s < n_stages; s++)
+          if ((issued >> s) & 1u) mbar_wait_drain(&full_bar[s], (issued_phase >> s) & 1u, err, lim2);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
@@ -400,11 +386,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
       uint32_t phase = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      constexpr uint32_t idesc = idesc_u8_m256(BN);
-      for (int t = cluster; ok && t < P.total_tiles; t += n_clusters) {
+      for (int k = 0; ok && k * n_clusters < P.total_tiles; k++) {
         Tile tl;
-        if (!tile_of2(P, t, tl)) break;
+        if (!tile_of(P, tile_index(k, cluster, n_clusters), tl)) continue;
         const GemmProblem& pr = P.prob[tl.prob];
+        const uint32_t idesc = idesc_u8_m256(tile_width(tl));
         if (!mbar_wait(acc_empty, acc_phase ^ 1u, err, kErrTimeoutAccEmpty, lim2)) { ok = false; break; }
         acc_phase ^= 1u;
         tc_fence_after();
@@ -413,18 +399,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
           tc_fence_after();
           const uint64_t dal = smem_desc(a_lo + stage * 128 * kBK);
           const uint64_t dah = smem_desc(a_hi + stage * 128 * kBK);
-          const uint64_t dbl = smem_desc(b_lo + stage * C::kHalfN * kBK);
-          const uint64_t dbh = smem_desc(b_hi + stage * C::kHalfN * kBK);
+          const uint64_t dbl = smem_desc(b_lo + stage * b_bytes);
+          const uint64_t dbh = smem_desc(b_hi + stage * b_bytes);
 #pragma unroll
           for (int kk = 0; kk < kBK / 32; kk++) {
             const uint32_t acc = (ki > 0 || kk > 0) ? 1u : 0u;
             const uint64_t o = (uint64_t)(2 * kk);
             mma_u8_pair(tmem, dal + o, dbl + o, idesc, acc);
-            mma_u8_pair(tmem + BN, dal + o, dbh + o, idesc, acc);
-            mma_u8_pair(tmem + BN, dah + o, dbl + o, idesc, 1u);
+            mma_u8_pair(tmem + kPairMaxN, dal + o, dbh + o, idesc, acc);
+            mma_u8_pair(tmem + kPairMaxN, dah + o, dbl + o, idesc, 1u);
           }
           mma_commit_pair(&empty_bar[stage]);
-          if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
+          if (++stage == n_stages) { stage = 0; phase ^= 1u; }
         }
         if (ok) mma_commit_pair(acc_full);
       }
@@ -438,23 +424,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
     const int row = quad * 32 + lane;
-    constexpr int kCols = C::kColsPerThread;
+    constexpr int kCols = kPairMaxN / 2;  // at most
     const uint32_t acc_empty_leader = map_to_rank(acc_empty, 0);
     uint32_t acc_phase = 0;
-    for (int t = cluster; t < P.total_tiles; t += n_clusters) {
+    for (int k = 0; k * n_clusters < P.total_tiles; k++) {
       Tile tl;
-      if (!tile_of2(P, t, tl)) break;
+      if (!tile_of(P, tile_index(k, cluster, n_clusters), tl)) continue;
       const GemmProblem& pr = P.prob[tl.prob];
+      const int cols = tile_width(tl) / 2;  // this half's query rows, a multiple of 32
       if (!mbar_wait(acc_full, acc_phase, err, kErrTimeoutAccFull, lim2)) break;
       acc_phase ^= 1u;
       tc_fence_after();
       uint32_t packed[kCols / 2];
-      const uint32_t tbase = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * kCols);
+      const uint32_t tbase = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * cols);
 #pragma unroll
       for (int c = 0; c < kCols / 32; c++) {
+        if (c * 32 >= cols) break;
         uint32_t r0[32], r1[32];
         tmem_ld32(tbase + (uint32_t)(c * 32), r0);
-        tmem_ld32(tbase + (uint32_t)(BN + c * 32), r1);
+        tmem_ld32(tbase + (uint32_t)(kPairMaxN + c * 32), r1);
         tmem_wait_ld();
 #pragma unroll
         for (int j = 0; j < 16; j++) {
@@ -473,8 +461,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         uint16_t* out_row = pr.out + (size_t)m_local * pr.n_pad;
 #pragma unroll
         for (int c = 0; c < kCols / 32; c++) {
-          const uint32_t n = (uint32_t)(tl.n_tile * BN + half * kCols + c * 32);
-          if (n >= pr.n_pad) break;  // part-filled last tile
+          const uint32_t n = (uint32_t)(tile_row(tl) + half * cols + c * 32);
+          if (c * 32 >= cols || n >= pr.n_pad) break;
           uint32_t v[16];
 #pragma unroll
           for (int j = 0; j < 16; j++) {
@@ -502,7 +490,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   cluster_sync_all();  // no CTA leaves while its peer may still touch its memory
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)C::kTmemCols));
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
   }
 }
 
@@ -755,19 +743,24 @@ static cudaError_t launch_split(const GemmParams& P, cudaStream_t stream) {
 
 static cudaError_t launch_pair(const GemmParams& P, int n_sms, cudaStream_t stream) {
   static std::atomic<uint64_t> attr_done{0};
-  cudaError_t e = smem_limit_once(limb_gemm_pair_kernel, Cfg2::kSmemBytes, attr_done);
+  cudaError_t e = smem_limit_once(limb_gemm_pair_kernel, kPairSmem, attr_done);
   if (e != cudaSuccess) return e;
   const int clusters = P.total_tiles < n_sms / 2 ? P.total_tiles : n_sms / 2;
   if (clusters <= 0) return cudaSuccess;
-  limb_gemm_pair_kernel<<<2 * clusters, kThreads, Cfg2::kSmemBytes, stream>>>(P);
+  limb_gemm_pair_kernel<<<2 * clusters, kThreads, kPairSmem, stream>>>(P);
   return cudaGetLastError();
 }
 
 // The pair kernel reaches a higher MAC rate per clock but, at the B200's
-// 1000 W limit, pulls the SM clock down about as far as it gains, so for long
-// launches the one-SM kernel is the default and the batch autotuner decides per
-// batch shape (irs_sharedb_set_pair).
-bool gemm_pair_applies(bool pair, int block_n) { return pair && block_n == 256; }
+// 1000 W limit, pulls the SM clock down with it: up to 768 query rows it gains
+// all the same, above that the one-SM kernel is the default for long launches
+// and the batch autotuner decides per batch shape (irs_sharedb_set_pair).
+bool gemm_pair_applies(bool pair, uint32_t n_pad) { return pair && n_pad >= 128; }
+
+int gemm_pair_n(uint32_t n_pad) {
+  const uint32_t tiles = (n_pad + kPairMaxN - 1) / kPairMaxN;
+  return (int)(((n_pad + tiles - 1) / tiles + 63) / 64 * 64);
+}
 
 // Measured on 65,536-entry chunks of the six engines: up to 768 query rows
 // the 128-row tile (3 pipeline stages) beats the 256-row tile (2 stages) by
@@ -804,18 +797,29 @@ static uint32_t gemm_l2_hint() {
 // CTAs that share a tile's K loop (1: the persistent kernel).  Six engines, cold
 // caches, persistent / four / eight: 64 entries x 64 rows (6 tiles) 62 / 25.6 /
 // 21.5 us; 64 x 256 (12) 71 / 29.8 / 25.6; 500 x 32 (24) 64 / 29.7 / 33.8; 1000 x
-// 32 (48) 66 / 46; 2000 x 32 and 1000 x 256 (96) 75 / 73 and 79 / 73; 300 x 768
-// (108) 79 / 83.  Clusters of eight pay while all of them run at once, of four
-// up to two thirds of the SMs' count in tiles.
+// 32 (48) 66 / 46; 700 x 256 (72) 77 / 67; 2000 x 32 (96) 75 / 73.  One engine
+// (tiles of one length, so the persistent kernel has no short ones to wait
+// with): 39 tiles 13.2 / 14.3, 68 tiles 40 / 50.  Eight pay while all tiles run
+// at once; four while the longest do, and the shorter ones add at most half as
+// much again.
 static int gemm_k_split(const GemmParams& P, int block_n, int n_sms) {
-  uint32_t k = ~0u;
-  for (int i = 0; i < P.n_prob; i++) k = std::min(k, P.prob[i].k_iters);
-  if (block_n > 128 || 3 * P.total_tiles > 2 * n_sms || k < 8) return 1;
-  return 8 * P.total_tiles <= n_sms && k >= 16 ? 8 : 4;
+  uint32_t least = ~0u, most = 0;
+  for (int i = 0; i < P.n_prob; i++) {
+    least = std::min(least, P.prob[i].k_iters);
+    most = std::max(most, P.prob[i].k_iters);
+  }
+  if (block_n > 128 || least < 8) return 1;
+  if (8 * P.total_tiles <= n_sms && least >= 16) return 8;
+  uint64_t longest = 0, blocks = 0;
+  for (int i = 0; i < P.n_prob; i++) {
+    const uint64_t tiles = (uint64_t)P.prob[i].tiles_m * P.prob[i].tiles_n;
+    if (P.prob[i].k_iters == most) longest += tiles;
+    blocks += tiles * P.prob[i].k_iters;
+  }
+  return 4 * longest <= (uint64_t)n_sms && 8 * blocks <= 3ull * (uint64_t)n_sms * most ? 4 : 1;
 }
 
-cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair_wanted, int n_sms, cudaStream_t stream) {
-  const bool pair = gemm_pair_applies(pair_wanted, block_n);
+cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair, int n_sms, cudaStream_t stream) {
   if (P.wait_timeout_ns == 0) P.wait_timeout_ns = kGemmWaitTimeoutNs;
   P.l2_hint = gemm_l2_hint();
   // Serpentine K order (GemmParams::serpentine), on unless IRS_GEMM_SERPENTINE=0.
@@ -829,6 +833,16 @@ cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair_wanted, int n
   }();
   P.serpentine = serp;
   const uint32_t bm = pair ? (uint32_t)kBM2 : (uint32_t)kBM;
+  if (pair) {
+    P.pair_n = gemm_pair_n(P.prob[0].n_pad);
+    const int units = (int)P.prob[0].n_pad / 64, tiles = (int)(P.prob[0].n_pad + kPairMaxN - 1) / kPairMaxN;
+    // 960 rows as 4 x 256: 0.73 ms (one engine x 32,768 entries), as 256 x 3 +
+    // 192 0.77: tiles of unequal length drift apart and share less of L2
+    const int spare = P.pair_n / 64 * tiles - units;  // units of padding if all tiles were as wide
+    P.pair_wider = 15 * spare <= units ? tiles : units % tiles;
+    block_n = kPairMaxN;  // the tiles of a problem: as many as 256-row ones
+    P.pair_stages = std::min(kPairMaxStages, kPairRoom / pair_stage_bytes(P.pair_n));
+  }
   P.total_tiles = 0;
   for (int i = 0; i < P.n_prob; i++) {
     GemmProblem& pr = P.prob[i];

@@ -68,19 +68,26 @@ struct GemmParams {
   // so the query K blocks the previous wave of CTAs loaded last are the first
   // this wave needs.  Integer accumulation: the result does not depend on it.
   uint32_t serpentine;
+  // two-SM kernel (filled by launch_limb_gemm): the widest tile's query rows,
+  // how many tiles of a problem have them, pipeline stages
+  int pair_n;
+  int pair_wider;
+  int pair_stages;
 };
 
 // Builds a 2-D u8 tensor map (inner dim K, outer dim rows) with 128x`box_rows`
 // boxes and 128-byte swizzle.  Returns 0 on success.
 int make_tmap_u8(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k, uint32_t box_rows);
 
-// Tile width along the query rows that divides n_pad (256, 128 or 64; 0 if none).
+// Tile width along the query rows for n_pad of them (256, 128 or 64; 0 if n_pad
+// is no multiple of 64).
 int gemm_block_n_for(uint32_t n_pad);
 
-// True when launch_limb_gemm runs the two-SM (cta_group::2) kernel: asked for
-// (`pair`) and the 256-row tile; its query tensor maps must then use boxes of
-// block_n / 2 rows.
-bool gemm_pair_applies(bool pair, int block_n);
+// Whether the two-SM (cta_group::2) kernel can run n_pad query rows where it is
+// asked for; its query tensor maps then use boxes of gemm_pair_n / 2 rows.
+bool gemm_pair_applies(bool pair, uint32_t n_pad);
+// Its widest tile for n_pad query rows (a multiple of 64, at most 256).
+int gemm_pair_n(uint32_t n_pad);
 
 cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair, int n_sms, cudaStream_t stream);
 

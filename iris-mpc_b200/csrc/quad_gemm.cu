@@ -101,13 +101,6 @@ __device__ __forceinline__ bool tile_of(const QuadParams& P, int t, Tile& out) {
   return false;
 }
 
-// Round k of cluster c: rounds alternate direction, so the clusters that get
-// a part-filled round of the long (code) tiles are not also those that get
-// the part-filled last round.
-__device__ __forceinline__ int tile_index(int k, int cluster, int n_clusters) {
-  return k * n_clusters + ((k & 1) ? n_clusters - 1 - cluster : cluster);
-}
-
 // The 32 rows of one slot for one entry, from the s-th slot of a thread's pair
 // sums f.  Out of line: one copy of its ChaCha code, with the keystream added
 // from registers.
@@ -462,8 +455,9 @@ int quad_width_for(const uint32_t* K, int n_prob, uint32_t m_len, uint32_t n_pad
   for (int i = 0; i < n_prob; i++) bytes += 2.0 * K[i] * m_len;
   const uint32_t bm = pair ? (uint32_t)kBM2 : (uint32_t)kBM;
   for (int i = 0; i < n_prob; i++) {
-    tiles[i] = (m_len + bm - 1) / bm * ((n_pad + (uint32_t)block_n - 1) / (uint32_t)block_n);
-    cost[i] = K[i] / 128 * (pair ? 1536 : block_n == 256 ? 1920 : kRoundTrip) + kDrain;
+    const uint32_t bn = pair ? 256u : (uint32_t)block_n;
+    tiles[i] = (m_len + bm - 1) / bm * ((n_pad + bn - 1) / bn);
+    cost[i] = K[i] / 128 * (pair ? std::max(6.0 * gemm_pair_n(n_pad), kRoundTrip) : block_n == 256 ? 1920 : kRoundTrip) + kDrain;
   }
   const double plain = std::max(last_done(tiles, cost, n_prob, pair ? n_sms / 2 : n_sms), bytes / kHbmBytesPerCycle);
   int best = -1;

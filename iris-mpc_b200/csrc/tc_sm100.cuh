@@ -174,6 +174,13 @@ __device__ __forceinline__ void tmem_wait_ld16(uint32_t (&r)[16]) {
                : "memory");
 }
 
+// The tile of worker (CTA or cluster) w in round k of a persistent GEMM: rounds
+// alternate direction, so the workers that get a part-filled round of the long
+// (code) tiles are not also those that get the part-filled last round.
+__device__ __forceinline__ int tile_index(int k, int w, int n_workers) {
+  return k * n_workers + ((k & 1) ? n_workers - 1 - w : w);
+}
+
 // Keystream blocks of the party's own and previous seed at one counter; out of
 // line so the epilogue carries a single copy of the ChaCha code.
 __device__ __noinline__ void chacha12_pair(const ChaChaKey* own, const ChaChaKey* prev, uint64_t counter,

@@ -534,7 +534,7 @@ class ShareDB:
         _check(lib().irs_sharedb_set_batch(self.h, batch_id))
 
     def set_pair(self, on: bool) -> None:
-        """Two-SM GEMM for the 256-row tile (irs_sharedb_set_pair)."""
+        """The GEMM on SM pairs wherever it can run so (irs_sharedb_set_pair)."""
         _check(lib().irs_sharedb_set_pair(self.h, int(on)))
 
     def set_tile(self, block_n: int) -> None:
