@@ -174,12 +174,15 @@ struct irs_distance_comparator {
   uint32_t* match_list = nullptr;   // pairs
   uint32_t* counters = nullptr;     // [0] match count, [1] partial count
   uint32_t* partial = nullptr;      // [max_db] compaction output
+  // one allocation, so that one copy fetches them:
+  uint32_t* results_err = nullptr;    // [4]: word 0 takes the device error word
   uint32_t* final_results = nullptr;  // [max_queries]
   uint32_t* match_counters = nullptr; // [max_queries]
   uint32_t* all_matches = nullptr;    // [max_queries][256]
   uint32_t* d_slot_valid = nullptr;
   uint32_t* d_slot_query = nullptr;
-  uint32_t* d_take = nullptr;  // irs_dc_take_rows: row list [max_queries], counts [max_queries], ids [max_queries][256]
+  // irs_dc_take_rows: row list [max_queries], error word [4], counts [max_queries], ids [max_queries][256]
+  uint32_t* d_take = nullptr;
   // distance capture (irs_dc_enable_distance_capture): count, entry, row, code [3], mask [3]
   uint32_t* d_dist = nullptr;
   size_t dist_cap = 0;
@@ -240,13 +243,14 @@ void drop_sums(irs_sharedb* db) {
 // reads; whether there were any.
 bool reclaim_sums(int device) {
   std::lock_guard<std::mutex> lock(sum_holders().mu);
-  const std::vector<irs_sharedb*> all = sum_holders().engines;
+  const auto& held = sum_holders().engines;
   bool any = false;
-  for (irs_sharedb* db : all)
-    if (db->dm->device == device && !db->sums_captured && !db->dm->capturing) {
-      drop_sums_locked(db);
-      any = true;
-    }
+  for (size_t i = held.size(); i-- > 0;) {  // dropping one removes it from the list
+    irs_sharedb* db = held[i];
+    if (db->dm->device != device || db->sums_captured || db->dm->capturing) continue;
+    drop_sums_locked(db);
+    any = true;
+  }
   return any;
 }
 
@@ -396,8 +400,14 @@ void alloc_sums(irs_sharedb* db) {
     drop_sums(db);
     return;
   }
-  std::lock_guard<std::mutex> lock(sum_holders().mu);
-  sum_holders().engines.push_back(db);
+  bool held = true;
+  try {
+    std::lock_guard<std::mutex> lock(sum_holders().mu);
+    sum_holders().engines.push_back(db);
+  } catch (const std::bad_alloc&) {
+    held = false;
+  }
+  if (!held) drop_sums(db);
 }
 
 // Whether a gather of n records leaves the sums behind: for a few records the
@@ -1702,15 +1712,13 @@ int irs_dc_init(irs_device_manager* dm, size_t max_queries, size_t max_db_length
       {(void**)&dc->match_list, dc->match_cap * 8},
       {(void**)&dc->counters, 16},
       {(void**)&dc->partial, max_db_length * 4},
-      {(void**)&dc->final_results, max_queries * 4},
-      {(void**)&dc->match_counters, max_queries * 4},
-      {(void**)&dc->all_matches, max_queries * kMaxMatchesLen * 4},
+      {(void**)&dc->results_err, (4 + max_queries * (2 + kMaxMatchesLen)) * 4},
       {(void**)&dc->d_slot_valid, dc->slot_cap * 4},
       {(void**)&dc->d_slot_query, dc->slot_cap * 4},
       {(void**)&dc->d_seg_start, (dc->slot_cap + 1) * 4},
       {(void**)&dc->d_seg_query, dc->slot_cap * 32 * 4},
       {(void**)&dc->d_seg_mask, dc->slot_cap * 32 * 4},
-      {(void**)&dc->d_take, max_queries * (2 + kMaxMatchesLen) * 4},
+      {(void**)&dc->d_take, (4 + max_queries * (2 + kMaxMatchesLen)) * 4},
   };
   for (auto& a : allocs) {
     cudaError_t e = device_malloc(dm, a.p, a.bytes);
@@ -1720,6 +1728,10 @@ int irs_dc_init(irs_device_manager* dm, size_t max_queries, size_t max_db_length
       return fail(IRS_ERR_NOMEM, "distance comparator allocation of %zu bytes failed", a.bytes);
     }
   }
+  dc->final_results = dc->results_err + 4;
+  dc->match_counters = dc->final_results + max_queries;
+  dc->all_matches = dc->match_counters + max_queries;
+  CU(cudaMemsetAsync(dc->all_matches, 0, max_queries * kMaxMatchesLen * 4, dm->streams[0]));
   int rc = irs_dc_reset(dc, nullptr);
   if (rc) { irs_dc_destroy(dc); return rc; }
   CU(cudaStreamSynchronize(dm->streams[0]));
@@ -1730,8 +1742,8 @@ int irs_dc_init(irs_device_manager* dm, size_t max_queries, size_t max_db_length
 int irs_dc_destroy(irs_distance_comparator* dc) {
   if (!dc) return IRS_OK;
   cudaSetDevice(dc->dm->device);
-  void* ps[] = {dc->bitmap, dc->self_bitmap, dc->match_list, dc->counters, dc->partial, dc->final_results,
-                dc->match_counters, dc->all_matches, dc->d_slot_valid, dc->d_slot_query,
+  void* ps[] = {dc->bitmap, dc->self_bitmap, dc->match_list, dc->counters, dc->partial, dc->results_err,
+                dc->d_slot_valid, dc->d_slot_query,
                 dc->d_seg_start, dc->d_seg_query, dc->d_seg_mask, dc->d_take, dc->d_dist, dc->d_forced,
                 dc->ring};
   for (void* p : ps) if (p) cudaFree(p);
@@ -1742,12 +1754,27 @@ int irs_dc_destroy(irs_distance_comparator* dc) {
 int irs_dc_reset(irs_distance_comparator* dc, void* stream) {
   CHECK(dc, IRS_ERR_INVALID, "dc is NULL");
   cudaStream_t s = party_stream(dc->dm, 0, stream);
-  CU(cudaMemsetAsync(dc->bitmap, 0, dc->max_queries * dc->stride_bits / 8, s));
-  CU(cudaMemsetAsync(dc->self_bitmap, 0, dc->max_queries * dc->self_stride_bits / 8, s));
-  CU(cudaMemsetAsync(dc->counters, 0, 16, s));
-  CU(cudaMemsetAsync(dc->final_results, 0xFF, dc->max_queries * 4, s));
-  CU(cudaMemsetAsync(dc->match_counters, 0, dc->max_queries * 4, s));
+  CU(launch_reset(dc->bitmap, dc->max_queries * dc->stride_bits / 32, dc->self_bitmap,
+                  dc->max_queries * dc->self_stride_bits / 32, dc->counters, dc->final_results, dc->match_counters,
+                  (uint32_t)dc->max_queries, s));
   return IRS_OK;
+}
+
+// Fetches a block of `words` result words behind its four error words in one
+// copy: the device error word joins it on the device.  out[0..words) follows the
+// four; returns the error word's status.
+static int fetch_block(irs_distance_comparator* dc, uint32_t* block, size_t words, std::vector<uint32_t>& out,
+                       cudaStream_t s) {
+  try {
+    out.resize(4 + words);
+  } catch (const std::bad_alloc&) {
+    out.clear();
+    return fail(IRS_ERR_NOMEM, "host buffer of %zu result words failed", words);
+  }
+  CU(cudaMemcpyAsync(block, dc->dm->d_err, 4, cudaMemcpyDeviceToDevice, s));
+  CU(cudaMemcpyAsync(out.data(), block, out.size() * 4, cudaMemcpyDeviceToHost, s));
+  CU(cudaStreamSynchronize(s));
+  return device_error((int)out[0]);
 }
 
 int irs_dc_compare_threshold_open(irs_distance_comparator* dc, irs_circuits* c, irs_sharedb* const code_engines[3],
@@ -2066,16 +2093,22 @@ int irs_dc_take_rows(irs_distance_comparator* dc, const uint32_t* rows, size_t n
   CU(cudaSetDevice(dm->device));
   cudaStream_t s = dm->streams[0];
   uint32_t* d_rows = dc->d_take;
-  uint32_t* d_counts = d_rows + dc->max_queries;
+  uint32_t* d_counts = d_rows + dc->max_queries + 4;
   uint32_t* d_ids = d_counts + dc->max_queries;
   CU(cudaMemcpyAsync(d_rows, rows, n * 4, cudaMemcpyHostToDevice, s));
   CU(launch_take_rows(dc->bitmap, (uint32_t)(dc->stride_bits / 32), d_rows, (uint32_t)n, (uint32_t)db_len, clear,
                       d_counts, d_ids, kMaxMatchesLen, s));
-  CU(cudaMemcpyAsync(counts, d_counts, n * 4, cudaMemcpyDeviceToHost, s));
-  CU(cudaMemcpyAsync(ids, d_ids, n * kMaxMatchesLen * 4, cudaMemcpyDeviceToHost, s));
-  if (!dm->host_sync) return IRS_OK;  // outputs valid once the stream passes the copies
-  CU(cudaStreamSynchronize(s));
-  return check_device_error(dm);
+  if (!dm->host_sync) {  // outputs valid once the stream passes the copies
+    CU(cudaMemcpyAsync(counts, d_counts, n * 4, cudaMemcpyDeviceToHost, s));
+    CU(cudaMemcpyAsync(ids, d_ids, n * kMaxMatchesLen * 4, cudaMemcpyDeviceToHost, s));
+    return IRS_OK;
+  }
+  std::vector<uint32_t> got;
+  const int rc = fetch_block(dc, d_counts - 4, dc->max_queries + n * kMaxMatchesLen, got, s);
+  if (got.empty()) return rc;
+  memcpy(counts, got.data() + 4, n * 4);
+  memcpy(ids, got.data() + 4 + dc->max_queries, n * kMaxMatchesLen * 4);
+  return rc;
 }
 
 static size_t dist_bytes(size_t cap) { return (1 + 2 * cap) * 4 + 6 * cap * 2 + 16; }
@@ -2174,7 +2207,10 @@ int irs_dc_fetch_rows(irs_distance_comparator* dc, size_t first, size_t n, uint3
   if (n) {
     CU(cudaMemcpyAsync(host, dc->bitmap + first * words, n * words * 4, cudaMemcpyDeviceToHost, s));
     if (!dm->host_sync) return IRS_OK;  // rows valid once the stream passes the copy
+    uint32_t err = 0;
+    CU(cudaMemcpyAsync(&err, dm->d_err, 4, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
+    return device_error((int)err);
   }
   return check_device_error(dm);
 }
@@ -2276,13 +2312,22 @@ int irs_dc_fetch_final_results(irs_distance_comparator* dc, size_t n_queries, ui
   irs_device_manager* dm = dc->dm;
   CU(cudaSetDevice(dm->device));
   cudaStream_t s = dm->streams[0];
+  if (dm->host_sync) {
+    const size_t mq = dc->max_queries, words = all_matches ? 2 * mq + n_queries * kMaxMatchesLen : mq + n_queries;
+    std::vector<uint32_t> got;
+    const int rc = fetch_block(dc, dc->results_err, words, got, s);
+    if (got.empty()) return rc;
+    if (final_results) memcpy(final_results, got.data() + 4, n_queries * 4);
+    if (match_counters) memcpy(match_counters, got.data() + 4 + mq, n_queries * 4);
+    if (all_matches) memcpy(all_matches, got.data() + 4 + 2 * mq, n_queries * kMaxMatchesLen * 4);
+    return rc;
+  }
+  // outputs valid once the stream passes the copies
   if (final_results) CU(cudaMemcpyAsync(final_results, dc->final_results, n_queries * 4, cudaMemcpyDeviceToHost, s));
   if (match_counters) CU(cudaMemcpyAsync(match_counters, dc->match_counters, n_queries * 4, cudaMemcpyDeviceToHost, s));
   if (all_matches)
     CU(cudaMemcpyAsync(all_matches, dc->all_matches, n_queries * kMaxMatchesLen * 4, cudaMemcpyDeviceToHost, s));
-  if (!dm->host_sync) return IRS_OK;  // outputs valid once the stream passes the copies
-  CU(cudaStreamSynchronize(s));
-  return check_device_error(dm);
+  return IRS_OK;
 }
 
 }  // extern "C"

@@ -43,7 +43,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>
-#include <vector>
 #include "common.cuh"
 #include "gemm_limb.h"
 #include "quad_gemm.h"
@@ -431,15 +430,17 @@ static double last_done(const uint32_t* tiles, const double* cost, int n_prob, i
     total += tiles[i] * cost[i];
     count += tiles[i];
   }
-  if (count > 16u * (uint32_t)units) return total / units;  // many rounds: the last one does not matter
-  std::vector<double> busy((size_t)units, 0.0);
+  constexpr int kMostUnits = 512;
+  // many rounds: the last one does not matter
+  if (count > 16u * (uint32_t)units || units > kMostUnits) return total / units;
+  double busy[kMostUnits] = {};
   int k = 0, u = 0;
   for (int i = 0; i < n_prob; i++)
     for (uint32_t t = 0; t < tiles[i]; t++) {
       busy[(size_t)((k & 1) ? units - 1 - u : u)] += cost[i];
       if (++u == units) { u = 0; k++; }
     }
-  return *std::max_element(busy.begin(), busy.end());
+  return *std::max_element(busy, busy + units);
 }
 
 // A 128-byte K step takes its MMAs (6 cycles per query column on a pair), or

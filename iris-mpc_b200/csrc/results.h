@@ -7,6 +7,10 @@ namespace irs {
 
 constexpr uint32_t kMaxMatchesLen = 256;
 
+// A comparator's start of a batch: bitmaps (even word counts, 8-byte aligned),
+// counters[4] and match counters zero, final results all ones.
+cudaError_t launch_reset(uint32_t* bitmap, size_t words, uint32_t* self_bitmap, size_t self_words, uint32_t* counters,
+                         uint32_t* final_results, uint32_t* match_counters, uint32_t n_queries, cudaStream_t stream);
 cudaError_t launch_compact(const uint32_t* bitmap, uint32_t n_queries, uint32_t db_len, uint32_t stride_words,
                            uint32_t* out, uint32_t* counter, uint32_t cap, cudaStream_t stream);
 cudaError_t launch_merge_db(const uint32_t* left, const uint32_t* right, const uint32_t* or_policy, uint32_t n_queries,

@@ -168,3 +168,28 @@ def test_small_gather_leaves_the_plain_gemm(dm):
             assert np.array_equal(quad, plain)
     e.close()
     src.close()
+
+
+def test_sums_give_way_to_other_allocations(dm):
+    """The library's own allocations take the room of the derived sums back
+    (unless a captured launch reads them), and results stay the same."""
+    K, n_db = 12800, 200000
+    rng = np.random.default_rng(9)
+    e = _engine(dm, K, 8192, 640, 31)
+    big = irisb200.ShareDB(0, dm, 64, 640, K, W.SEEDS[0])
+    big.alloc_db(n_db)  # 5 GB of records, 6.4 GB of sums
+    base = rng.integers(0, 1 << 16, (20, K), dtype=np.uint16)
+    e.query_upload_slots(base, [(j, 0, 31, j) for j in range(20)])
+    before, plain = _both(e, 0, 8192)
+    assert np.array_equal(before, plain)
+    free, _ = dm.mem_info()
+    taken = [irisb200.DeviceBuffer(dm, free - (3 << 30)), irisb200.DeviceBuffer(dm, 5 << 30)]
+    assert dm.mem_info()[0] < (5 << 30)  # the second one fits only in what the sums held
+    after, _ = _both(e, 0, 8192)
+    assert np.array_equal(after, plain)
+    e.query_upload_slots(base, [(j, 0, 31, j) for j in range(20)])
+    assert np.array_equal(_both(e, 0, 8192)[0], plain)
+    for b in taken:
+        b.free()
+    big.close()
+    e.close()
