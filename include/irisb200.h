@@ -129,7 +129,9 @@ int irs_event_synchronize(void* ev);
 int irs_event_query(void* ev, int* done);
 int irs_event_destroy(void* ev);
 /* Free and total device memory (cudaMemGetInfo), for admission by free HBM
- * (no counterpart: the reference sizes its batches statically). */
+ * (no counterpart: the reference sizes its batches statically).  The derived
+ * layouts that the library gives back when an allocation of its own fails
+ * count as free. */
 int irs_device_manager_mem_info(irs_device_manager* dm, size_t* free_bytes, size_t* total_bytes);
 
 /* Plain device memory helpers for callers that stage their own buffers. */

@@ -239,6 +239,19 @@ void drop_sums(irs_sharedb* db) {
   drop_sums_locked(db);
 }
 
+size_t sums_bytes(size_t cap, size_t K) { return 2 * cap * (K / 2 + 3 * K / 4); }
+size_t forms_bytes(size_t n_cap, size_t K) { return 2 * (kQuadProducts * (n_cap / 4) * (K / 4)); }
+
+// Bytes that reclaim_sums would give back on a device.
+size_t reclaimable_sums(int device) {
+  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  size_t bytes = 0;
+  for (const irs_sharedb* db : sum_holders().engines)
+    if (db->dm->device == device && !db->sums_captured && !db->dm->capturing)
+      bytes += sums_bytes(db->db_cap, db->code_length) + forms_bytes(db->n_cap, db->code_length);
+  return bytes;
+}
+
 // Gives back the sums of every engine on `device` that no captured graph
 // reads; whether there were any.
 bool reclaim_sums(int device) {
@@ -360,21 +373,20 @@ constexpr size_t kQuadMinRows = 576;
 // entries x 2048 rows: 0.19 ms either way; 2,048 entries: 0.35 / 0.52 ms).
 constexpr size_t kQuadMinRecords = 1024;
 
-size_t sums_bytes(size_t cap, size_t K) { return 2 * cap * (K / 2 + 3 * K / 4); }
-size_t forms_bytes(size_t n_cap, size_t K) { return 2 * (kQuadProducts * (n_cap / 4) * (K / 4)); }
-
 // Allocates the derived sums and query forms of an engine whose DB planes have
 // just been allocated (and zeroed, so the sums start at zero too).  Optional:
 // without them the engine runs the plain GEMM.  They are kept out of the way
-// of the program's other allocations: a sixth of the device's memory stays
-// free, and reclaim_sums gives them back when the library needs the room.
+// of the program's other allocations: a twelfth of the device's memory (16 GB)
+// stays free, and reclaim_sums gives them back when the library needs the room.
+// (A sixth left one of six engines of 524,288 records with 5,632 query rows
+// without them: 152 ms for 64 queries instead of 110.)
 void alloc_sums(irs_sharedb* db) {
   irs_device_manager* dm = db->dm;
   const size_t K = db->code_length, cap = db->db_cap;
   if (K % kRowLen || !forms_fit(K) || db->n_cap < kQuadMinRows || cap < kQuadMinRecords || dm->capturing) return;
   const size_t forms = forms_bytes(db->n_cap, K), masks = db->n_cap / kSlotRows * 4 + 4;
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < sums_bytes(cap, K) + forms + total_b / 6) {
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < sums_bytes(cap, K) + forms + total_b / 12) {
     cudaGetLastError();
     return;
   }
@@ -723,6 +735,7 @@ int irs_device_manager_mem_info(irs_device_manager* dm, size_t* free_bytes, size
   CHECK(dm && free_bytes && total_bytes, IRS_ERR_INVALID, "bad arguments");
   CU(cudaSetDevice(dm->device));
   CU(cudaMemGetInfo(free_bytes, total_bytes));
+  *free_bytes += reclaimable_sums(dm->device);
   return IRS_OK;
 }
 
@@ -1265,10 +1278,11 @@ static size_t tiles_128(irs_sharedb* const* engines, int n, size_t len) {
 }
 
 // Whether the plain GEMM of a launch runs on SM pairs.  Six engines x 32,768
-// entries, one-SM against pair: 128 rows 0.86 / 0.87 ms, 192 1.32 / 1.01, 256
+// entries, one-SM against pair: 128 rows 0.86 / 0.87 ms (over 131,072 entries
+// with the threshold between the chunks 3.03 / 2.89), 192 1.32 / 1.01, 256
 // 1.37 / 1.18, 384 1.93 / 1.74, 512 2.46 / 2.10, 768 3.58 / 3.03, 960 4.18 /
 // 4.25, 1024 4.24 / 3.94; at 65,536 entries the last two are 8.6 / 9.0 and 8.4 /
-// 8.0.  So from 192 to 768 rows it is the default, as far as there are more
+// 8.0.  So from 128 to 768 rows it is the default, as far as there are more
 // 128-row tiles than SMs (4,000 entries x 512 rows of one engine: 0.072 / 0.110
 // ms); above, where the caller chose it or the launch is short enough that the
 // clock has not dropped to the power limit (one engine x 32,768 entries, 960
@@ -1279,7 +1293,7 @@ static bool plain_pair(irs_sharedb* const* engines, int n, size_t len) {
   for (int i = 1; i < n; i++)
     if (engines[i]->n_pad != e->n_pad) return false;  // one tile width for the launch
   if (e->n_pad <= 768)
-    return tiles_128(engines, n, len) > (size_t)e->dm->n_sms && (e->pair || e->n_pad >= 192);
+    return tiles_128(engines, n, len) > (size_t)e->dm->n_sms;
   if (e->pair) return true;
   double macs = 0;
   for (int i = 0; i < n; i++) macs += 3.0 * (double)engines[i]->code_length * (double)e->n_pad * (double)len;

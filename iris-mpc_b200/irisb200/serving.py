@@ -128,7 +128,7 @@ class ContinuousServer:
             raise ValueError("row_capacity must exceed max_variants (base pool and row table share the staging)")
         self.dm = dm
         self.ce, self.me = list(code_engines), list(mask_engines)
-        # the DB engines' GEMM: the two-SM kernel where the 256-row tile applies
+        # the DB engines' GEMM: the two-SM kernels where they apply
         # (irs_sharedb_set_pair); close() restores the library's default.  The
         # defaults (two-SM GEMM, 32,768-entry steps) are the measured best of
         # the server on 524,288 entries: higher saturation and lower p99 than
