@@ -445,13 +445,13 @@ def run_ours(args):
     reqs = None
     q_cap = n_rows
     if args.batched_requests and world == 1:
-        from irisb200.batched import centred_rotations, pack
+        from irisb200.batched import centred_rotations, pack_for
         nb = args.batched_requests
         bpl = {j: (int((j * 104729 + 7) % M), (j * 5) % 31 - 15) for j in range(0, nb, 10)}
         bc, bm = irisb200.synth_queries(DB_SEED + rank, Q_SEED + 1, nb, bpl)
         reqs = request_mix(nb, bc, bm, bpl, M, seed=7)
-        lay = pack([list(centred_rotations(r.n_rot)) for r in reqs if r.kind == "uniqueness"
-                    for _ in range(2 if r.mirrored else 1)])
+        lay = pack_for([list(centred_rotations(r.n_rot)) for r in reqs if r.kind == "uniqueness"
+                        for _ in range(2 if r.mirrored else 1)], 1 << 16)
         q_cap = max(n_rows, -(-lay.n_rows // 256) * 256)  # room for the 256-row tile padding
     ce = [irisb200.ShareDB(p, dm, M, q_cap, K_CODE, seeds[p]) for p in range(3)]
     me = [irisb200.ShareDB(p, dm, M, q_cap, K_MASK, seeds[p]) for p in range(3)]
@@ -783,7 +783,7 @@ def run_ours(args):
             # a capture of this launch's own chunk length when the profile has
             # one; else the path's capture scaled by the entries a launch scans
             # (an estimate: the query planes' share of the bytes changes with it)
-            key = {"split": "limb_gemm", "pair": "limb_gemm_pair", "fused": "fused_scan"}[chosen[0]]
+            key = {"split": "limb_gemm", "pair": "quad_gemm", "fused": "fused_scan"}[chosen[0]]
             own = pj.get(key + "_by_chunk", {}).get(str(chunks[0][1]), {})
             lg = pj.get(key, {})
             if own.get("dram_bytes_per_launch"):
@@ -828,7 +828,9 @@ def run_ours(args):
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": None, "unit": "TOPS",
                          "frac": None, "traffic": traffic, "traffic_source": traffic_source,
                          "algorithmic_bytes_per_launch": alg_bytes,
-                         "kernel": {"split": "limb_gemm_kernel<256>", "pair": "limb_gemm_pair_kernel (cta_group::2)",
+                         "kernel": {"split": "limb_gemm_kernel<256>",
+                                    "pair": "quad_gemm_kernel (cta_group::2, 9/16 of the multiplications, counted "
+                                            "in full)",
                                     "fused": "fused_scan_kernel (GEMM and threshold: time includes the threshold)"}
                                    [chosen[0]] + f" (6 engines, one launch per {chunks[0][1]}-entry DB chunk, "
                                    f"{len(chunks)} per batch)",
@@ -1220,7 +1222,7 @@ def run_batched_sweep(args):
     import torch
 
     import irisb200
-    from irisb200.batched import BatchedEngine, centred_rotations, pack, pad_rows
+    from irisb200.batched import BatchedEngine, centred_rotations, pack_for, pad_rows
 
     if int(os.environ.get("RANK", "0")) != 0:
         return
@@ -1232,8 +1234,8 @@ def run_batched_sweep(args):
     pl = {j: (int((j * 104729 + 7) % M), (j * 5) % 31 - 15) for j in range(0, nb, 10)}
     qc, qm = irisb200.synth_queries(DB_SEED, Q_SEED + 1, nb, pl)
     mixes = {b: request_mix(b, qc, qm, pl, M, seed=7 + b) for b in sizes}
-    rows = max(-(-pad_rows(pack([list(centred_rotations(r.n_rot)) for r in mixes[b] if r.kind == "uniqueness"
-                                  for _ in range(2 if r.mirrored else 1)]), 1 << 20).n_rows // 256) * 256
+    rows = max(-(-pad_rows(pack_for([list(centred_rotations(r.n_rot)) for r in mixes[b] if r.kind == "uniqueness"
+                                      for _ in range(2 if r.mirrored else 1)], 1 << 16), 1 << 20).n_rows // 256) * 256
                for b in sizes)
     q_cap = max(2048, rows)
     dm = irisb200.DeviceManager(0)
