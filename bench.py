@@ -844,8 +844,8 @@ def run_ours(args):
             "cublas_limb_gemm_ms_per_batch": cublas_ms,
             "cublas_limb_gemm_clocks": cublas_clk,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-            "gpu_launches": (1 if chosen[0] == "fused" else 2) * len(chunks) * args.steps,
-            "gpu_launches_e2e": ((1 if chosen[0] == "fused" else 2) * len(chunks) + 7) * args.steps,
+            "gpu_launches": ((1 if chosen[0] == "fused" else 2) * len(chunks) + 1) * args.steps,  # + the reset
+            "gpu_launches_e2e": ((1 if chosen[0] == "fused" else 2) * len(chunks) + 8) * args.steps,
             "clocks": clk_value,
             "clocks_e2e": clk_e2e,
             "planted_matches_found": f"{planted_found}/{len(planted)}",

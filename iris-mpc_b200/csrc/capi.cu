@@ -143,12 +143,14 @@ struct irs_sharedb {
   uint8_t* sums = nullptr;
   uint8_t* forms = nullptr;
   uint32_t* row_valid = nullptr;
-  uint32_t* quad_flag = nullptr;  // device copy of quad_rows, for captured launches
-  bool flag_set = false;      // what the last upload left in it
+  uint32_t* quad_flag = nullptr;  // QuadFlags word, for captured launches (kept until destroy)
+  uint32_t flag_rows = 0;     // what the last upload left in it
   bool quad_rows = false;     // the uploaded rows are quads of rotations and the forms hold them
   size_t stale_end = 0;       // records below it have sums that a small gather left behind
   size_t forms_pad = 0;       // padded rows that the form maps are for (0: none)
-  bool sums_captured = false; // a captured launch reads the sums: they stay until alloc_db or destroy
+  bool dot_captured = false;  // a graph of this library reads the sums where quad_flag says so
+  bool sums_pinned = false;   // another capture uses the sums: they stay until alloc_db or destroy
+  bool rows_captured = false; // a captured upload rewrites the rows when it is replayed: no forms
   CUtensorMap tm_sum_lo[2]{}, tm_sum_hi[2]{}, tm_form_lo[kQuadWidths]{},
       tm_form_hi[kQuadWidths]{};
   CUtensorMap tm_db_lo{}, tm_db_hi{}, tm_q_lo{}, tm_q_hi{};
@@ -221,17 +223,25 @@ SumHolders& sum_holders() {
 
 // Frees an engine's sums and forms (the holders' lock is held).  cudaFree
 // waits for the launches that read them.
+// A graph that holds the quad GEMM is told by the flag to run the plain one;
+// replays start under the holders' lock, so that none reads the flag half-way.
 void drop_sums_locked(irs_sharedb* db) {
+  if (db->quad_flag && db->dot_captured) {
+    cudaDeviceSynchronize();
+    cudaMemset(db->quad_flag, 0, 4);
+    cudaDeviceSynchronize();
+    db->flag_rows = 0;
+  }
   auto& v = sum_holders().engines;
   v.erase(std::remove(v.begin(), v.end(), db), v.end());
   if (db->sums) cudaFree(db->sums);
   if (db->forms) cudaFree(db->forms);
   db->sums = db->forms = nullptr;
-  db->row_valid = db->quad_flag = nullptr;
-  db->quad_rows = db->flag_set = false;
+  db->row_valid = nullptr;
+  db->quad_rows = false;
   db->stale_end = 0;
   db->forms_pad = 0;
-  db->sums_captured = false;
+  db->dot_captured = db->sums_pinned = false;
 }
 
 void drop_sums(irs_sharedb* db) {
@@ -247,20 +257,20 @@ size_t reclaimable_sums(int device) {
   std::lock_guard<std::mutex> lock(sum_holders().mu);
   size_t bytes = 0;
   for (const irs_sharedb* db : sum_holders().engines)
-    if (db->dm->device == device && !db->sums_captured && !db->dm->capturing)
+    if (db->dm->device == device && !db->sums_pinned && !db->dm->capturing)
       bytes += sums_bytes(db->db_cap, db->code_length) + forms_bytes(db->n_cap, db->code_length);
   return bytes;
 }
 
-// Gives back the sums of every engine on `device` that no captured graph
-// reads; whether there were any.
+// Gives back the sums of every engine on `device`, except those that a capture
+// other than of this library's own dots uses; whether there were any.
 bool reclaim_sums(int device) {
   std::lock_guard<std::mutex> lock(sum_holders().mu);
   const auto& held = sum_holders().engines;
   bool any = false;
   for (size_t i = held.size(); i-- > 0;) {  // dropping one removes it from the list
     irs_sharedb* db = held[i];
-    if (db->dm->device != device || db->sums_captured || db->dm->capturing) continue;
+    if (db->dm->device != device || db->sums_pinned || db->dm->capturing) continue;
     drop_sums_locked(db);
     any = true;
   }
@@ -384,13 +394,17 @@ void alloc_sums(irs_sharedb* db) {
   irs_device_manager* dm = db->dm;
   const size_t K = db->code_length, cap = db->db_cap;
   if (K % kRowLen || !forms_fit(K) || db->n_cap < kQuadMinRows || cap < kQuadMinRecords || dm->capturing) return;
-  const size_t forms = forms_bytes(db->n_cap, K), masks = db->n_cap / kSlotRows * 4 + 4;
+  const size_t forms = forms_bytes(db->n_cap, K), masks = db->n_cap / kSlotRows * 4;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < sums_bytes(cap, K) + forms + total_b / 12) {
     cudaGetLastError();
     return;
   }
-  void *s = nullptr, *f = nullptr;
+  void *s = nullptr, *f = nullptr, *w = nullptr;
+  if (!db->quad_flag) {
+    if (pool_alloc(dm, db->peer, 4, &w)) return;
+    db->quad_flag = static_cast<uint32_t*>(w);
+  }
   if (cudaMalloc(&s, sums_bytes(cap, K)) != cudaSuccess || cudaMalloc(&f, forms + masks) != cudaSuccess) {
     cudaGetLastError();
     if (s) cudaFree(s);
@@ -399,7 +413,7 @@ void alloc_sums(irs_sharedb* db) {
   db->sums = static_cast<uint8_t*>(s);
   db->forms = static_cast<uint8_t*>(f);
   db->row_valid = reinterpret_cast<uint32_t*>(db->forms + forms);
-  db->quad_flag = db->row_valid + db->n_cap / kSlotRows;
+  db->flag_rows = 0;
   cudaStream_t st = dm->streams[db->peer];
   uint8_t* inner = db->sums + 2 * cap * (K / 2);
   if (make_tmap_plane(&db->tm_sum_lo[0], db->sums, cap, K / 2, 128) ||
@@ -422,15 +436,27 @@ void alloc_sums(irs_sharedb* db) {
   if (!held) drop_sums(db);
 }
 
+bool stream_captures(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return false;
+}
+
 // Whether a gather of n records leaves the sums behind: for a few records the
 // quad GEMM does not run, and the sums would be the larger part of the gather.
-bool gather_skips_sums(const irs_sharedb* db, size_t n) { return n < kQuadMinRecords && !db->sums_captured; }
+// (A captured launch runs it where it was captured, and a captured gather runs
+// whenever it is replayed.)
+bool gather_skips_sums(const irs_sharedb* db, size_t n, cudaStream_t s) {
+  return n < kQuadMinRecords && !db->dot_captured && !db->sums_pinned && !stream_captures(s);
+}
 
 // Brings the sums of records [first, first + n) in line with the planes, on
 // the stream that wrote them.
 cudaError_t update_sums(irs_sharedb* db, size_t first, size_t n, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(sum_holders().mu);
   if (!db->sums || !n) return cudaSuccess;
+  if (stream_captures(s)) db->sums_pinned = true;
   const size_t K = db->code_length, cap = db->db_cap, o = K / 2, i = 3 * K / 4;
   uint8_t* inner = db->sums + 2 * cap * o;
   return launch_derive_sums(db->db_lo + first * K, db->db_hi + first * K, (uint32_t)K, n, db->sums + first * o,
@@ -440,7 +466,7 @@ cudaError_t update_sums(irs_sharedb* db, size_t first, size_t n, cudaStream_t s)
 // Prepares the query forms' tensor maps for the active row count; false where
 // the quad GEMM does not run.
 bool quad_forms_ready(irs_sharedb* db) {
-  if (!db->sums || db->n_pad < kQuadMinRows) return false;
+  if (!db->sums || db->n_pad < kQuadMinRows || db->rows_captured) return false;
   if (db->forms_pad == db->n_pad) return true;
   const size_t K = db->code_length, rows = kQuadProducts * (db->n_pad / 4);
   db->forms_pad = 0;
@@ -478,14 +504,19 @@ uint8_t* forms_hi(irs_sharedb* db) { return db->forms + kQuadProducts * (db->n_p
 
 // Notes whether the rows about to be expanded are quads, and where the
 // expansion puts their forms and (if it changes) the device flag.  The holders'
-// lock is held until the expansion is enqueued.
-QuadForms begin_forms(irs_sharedb* db, bool quads) {
+// lock is held until the expansion is enqueued.  An upload that is captured
+// (on `s`) writes planes alone, and so do the engine's later ones: what the
+// rows are after a replay is not known here.
+QuadForms begin_forms(irs_sharedb* db, bool quads, cudaStream_t s) {
+  if (stream_captures(s)) db->rows_captured = true;
+  quads = quads && !db->rows_captured;
   db->quad_rows = quads;
   QuadForms f{nullptr, nullptr, nullptr, nullptr};
   if (quads) f = {db->forms, forms_hi(db), db->row_valid, nullptr};
-  if (db->sums && db->flag_set != quads) {
+  const uint32_t rows = quads ? (uint32_t)db->n_pad : 0u;
+  if (db->quad_flag && (db->flag_rows != rows || db->rows_captured)) {
     f.flag = db->quad_flag;
-    db->flag_set = quads;
+    db->flag_rows = rows;
   }
   return f;
 }
@@ -493,7 +524,7 @@ QuadForms begin_forms(irs_sharedb* db, bool quads) {
 // Planes and forms of a row table whose bases and table are in the staging.
 int expand_row_table(irs_sharedb* db, const uint32_t* desc, size_t n_rows, const uint32_t* d_desc, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(sum_holders().mu);
-  const QuadForms f = begin_forms(db, quad_forms_ready(db) && rows_are_quads(desc, n_rows));
+  const QuadForms f = begin_forms(db, quad_forms_ready(db) && rows_are_quads(desc, n_rows), s);
   CU(launch_expand_rows(db->q_stage, (uint32_t)db->code_length, d_desc, (uint32_t)n_rows, (uint32_t)db->n_pad, db->q_lo,
                         db->q_hi, f, s));
   return IRS_OK;
@@ -849,6 +880,7 @@ int irs_sharedb_destroy(irs_sharedb* db) {
   if (!db) return IRS_OK;
   irs_device_manager* dm = db->dm;
   cudaSetDevice(dm->device);
+  db->dot_captured = false;  // no graph over the engine is launched any more
   drop_sums(db);
   pool_free(dm, db->peer, db->db_lo);
   pool_free(dm, db->peer, db->db_hi);
@@ -857,6 +889,7 @@ int irs_sharedb_destroy(irs_sharedb* db) {
   pool_free(dm, db->peer, db->q_stage);
   pool_free(dm, db->peer, db->d_slots);
   pool_free(dm, db->peer, db->results);
+  pool_free(dm, db->peer, db->quad_flag);
   cudaStreamSynchronize(dm->streams[db->peer]);
   if (db->done) cudaEventDestroy(db->done);
   if (db->copied) cudaEventDestroy(db->copied);
@@ -1064,7 +1097,7 @@ int irs_sharedb_query_upload(irs_sharedb* db, const uint16_t* rows, size_t n_row
   CU(launch_split_limbs(db->q_stage, (uint32_t)K, db->q_lo, db->q_hi, db->n_pad * K, s));
   {
     std::lock_guard<std::mutex> lock(sum_holders().mu);
-    if (begin_forms(db, false).flag) CU(cudaMemsetAsync(db->quad_flag, 0, 4, s));  // rows of no known structure
+    if (begin_forms(db, false, s).flag) CU(cudaMemsetAsync(db->quad_flag, 0, 4, s));  // rows of no known structure
   }
   db->have_query = true;
   return IRS_OK;
@@ -1095,7 +1128,7 @@ int irs_sharedb_query_upload_slots(irs_sharedb* db, const uint16_t* base, size_t
   CU(cudaEventRecord(db->copied, s));
   {
     std::lock_guard<std::mutex> lock(sum_holders().mu);
-    const QuadForms f = begin_forms(db, quad_forms_ready(db));  // a slot's rows are consecutive rotations
+    const QuadForms f = begin_forms(db, quad_forms_ready(db), s);  // a slot's rows are consecutive rotations
     CU(launch_expand_slots(db->q_stage, (uint32_t)K, db->d_slots, (uint32_t)n_slots, (uint32_t)db->n_pad, db->q_lo,
                            db->q_hi, f, s));
   }
@@ -1191,7 +1224,7 @@ int irs_sharedb_gather_records(irs_sharedb* dst, irs_sharedb* src, const uint32_
   if (dm->host_sync) CU(cudaEventRecord(dst->copied, s));
   CU(launch_gather_rows(src->db_lo, src->db_hi, reinterpret_cast<const uint32_t*>(dst->q_stage), (uint32_t)n,
                         (uint32_t)K, dst->db_lo, dst->db_hi, s));
-  if (dst->sums && gather_skips_sums(dst, n)) {
+  if (dst->sums && gather_skips_sums(dst, n, s)) {
     dst->stale_end = std::max(dst->stale_end, n);
   } else {
     CU(update_sums(dst, 0, n, s));
@@ -1375,9 +1408,7 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
     }
     StageTimer timer(dm, s, "dot");
     std::lock_guard<std::mutex> lock(sum_holders().mu);
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    CU(cudaStreamIsCapturing(s, &st));
-    const bool captured = st != cudaStreamCaptureStatusNone;
+    const bool captured = stream_captures(s);
     const int width = stall ? -1 : quad_width(engines, n, offset, len, pair);
     bool quads = width >= 0;
     for (int i = 0; i < n && !captured; i++) quads = quads && engines[i]->quad_rows;
@@ -1390,9 +1421,10 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
       for (int i = 0; i < n; i++) {
         fill_quad_problem(engines[i], P.prob[i], width, Q.prob[i]);
         if (!captured) continue;
-        engines[i]->sums_captured = true;
+        (dm->capturing ? engines[i]->dot_captured : engines[i]->sums_pinned) = true;
         Q.run.word[i] = engines[i]->quad_flag;
         Q.run.n = n;
+        Q.run.rows = (uint32_t)engines[i]->n_pad;
       }
       P.skip = Q.run;
       CU(launch_quad_gemm(Q, dm->n_sms, s));
@@ -2081,7 +2113,10 @@ int irs_graph_launch(irs_graph* g, void* stream) {
       CU(cudaEventRecord(g->dm->uploads[p], g->dm->streams[p]));
       CU(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), g->dm->uploads[p], 0));
     }
-  CU(cudaGraphLaunch(g->exec, static_cast<cudaStream_t>(stream)));
+  {
+    std::lock_guard<std::mutex> lock(sum_holders().mu);
+    CU(cudaGraphLaunch(g->exec, static_cast<cudaStream_t>(stream)));
+  }
   // later query uploads on other party streams wait for the graph's GEMMs
   CU(cudaEventRecord(g->dm->graph_done, static_cast<cudaStream_t>(stream)));
   return IRS_OK;

@@ -31,17 +31,18 @@ struct alignas(64) GemmProblem {
 };
 
 constexpr int kMaxGemmProblems = 6;
-// Device words that are nonzero while an engine's uploaded rows are quads of
-// rotations.  A captured launch holds both GEMMs, since later uploads decide
-// which one a replay needs: the quad GEMM runs when all words are set, the
-// plain one when not.
+// Device words that hold the padded row count while an engine's uploaded rows
+// are quads of rotations, else 0.  A captured launch holds both GEMMs, since
+// later uploads decide which one a replay needs: the quad GEMM runs when all
+// words are the row count it was captured for, the plain one when not.
 struct QuadFlags {
   const uint32_t* word[kMaxGemmProblems];
   int n;  // 0: not captured, no check
+  uint32_t rows;
 #ifdef __CUDACC__
   __device__ __forceinline__ bool all_set() const {
     bool all = true;
-    for (int i = 0; i < n; i++) all = all && *word[i] != 0;
+    for (int i = 0; i < n; i++) all = all && *word[i] == rows;
     return all;
   }
 #endif

@@ -190,7 +190,7 @@ __global__ void expand_kernel(const uint16_t* __restrict__ base, uint32_t K, Row
                               uint8_t* __restrict__ lo, uint8_t* __restrict__ hi, QuadForms quads) {
   const uint32_t per_quarter = K / 32;
   if (blockIdx.x < n_pad) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && quads.flag) *quads.flag = quads.lo ? 1u : 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && quads.flag) *quads.flag = quads.lo ? n_pad : 0u;
     const uint32_t row = blockIdx.x;
     const RowSource src = rows(row);
     for (uint32_t o = threadIdx.x; o < 4 * per_quarter; o += blockDim.x) {

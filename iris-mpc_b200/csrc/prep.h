@@ -19,7 +19,7 @@ struct QuadForms {
   uint8_t* lo;      // [9][n_pad/4][K/4], NULL: none
   uint8_t* hi;
   uint32_t* valid;  // [n_pad/32] rows of each slot that hold a query row
-  uint32_t* flag;   // set to whether there are forms (NULL: left alone)
+  uint32_t* flag;   // set to the padded rows the forms are for, 0 without forms (NULL: left alone)
 };
 
 struct SynthOut {

@@ -18,7 +18,7 @@ struct alignas(64) QuadProblem {
   // sums [rows][K/2], [2] the inner sums [rows][3K/4] (derive_sums_kernel)
   CUtensorMap tm_a_lo[3];
   CUtensorMap tm_a_hi[3];
-  CUtensorMap tm_b_lo;  // query forms [9][n_pad/4][K/4] (expand_quads kernels)
+  CUtensorMap tm_b_lo;  // query forms [9][n_pad/4][K/4] (expand_kernel)
   CUtensorMap tm_b_hi;
   uint16_t* out;        // [m_len][n_pad]
   const uint32_t* row_valid;  // [n_pad/32] rows of each slot that hold a query row

@@ -152,6 +152,33 @@ def test_captured_launch_follows_the_uploads(dm):
     e.close()
 
 
+def test_captured_launch_keeps_its_row_count(dm):
+    """A graph captured at one padded row count replays on those rows of a
+    longer upload, whose forms lie elsewhere."""
+    K, n_db = 6400, 4100
+    rng = np.random.default_rng(12)
+    e = irisb200.ShareDB(0, dm, n_db, 1024, K, W.SEEDS[0])
+    e.alloc_db(n_db)
+    e.fill_random(3, n_db)
+    base = rng.integers(0, 1 << 16, (32, K), dtype=np.uint16)
+    slots = [(j, 0, 31, j) for j in range(32)]
+    e.query_upload_slots(base[:20], slots[:20])
+    plain = _both(e, 0, n_db)[1]
+    dm.synchronize()
+    g = irisb200.Graph.capture(dm, lambda: e.dot(0, n_db, 1, dm.stream(0)))
+    e.query_upload_slots(base, slots)  # 1024 rows, the first 640 as before
+    g.launch(dm.stream(0))
+    dm.synchronize()
+    e.query_upload_slots(base[20:], slots[:12])
+    e.query_upload_slots(base[:20], slots[:20])  # 640 rows again: the replay's result stride
+    assert np.array_equal(e.fetch_results(n_db), plain)
+    g.launch(dm.stream(0))
+    assert np.array_equal(e.fetch_results(n_db), plain)
+    dm.synchronize()
+    g.close()
+    e.close()
+
+
 def test_small_gather_leaves_the_plain_gemm(dm):
     """A gather of a few records, then of many, then a write: results follow the records."""
     K, n_db = 6400, 8300
@@ -170,9 +197,11 @@ def test_small_gather_leaves_the_plain_gemm(dm):
     src.close()
 
 
-def test_sums_give_way_to_other_allocations(dm):
-    """The library's own allocations take the room of the derived sums back
-    (unless a captured launch reads them), and results stay the same."""
+@pytest.mark.parametrize("captured", [False, True])
+def test_sums_give_way_to_other_allocations(dm, captured):
+    """The library's own allocations take the room of the derived sums back,
+    and results stay the same, those of a graph that was captured with them
+    included."""
     K, n_db = 12800, 200000
     rng = np.random.default_rng(9)
     e = _engine(dm, K, 8192, 640, 31)
@@ -182,11 +211,20 @@ def test_sums_give_way_to_other_allocations(dm):
     e.query_upload_slots(base, [(j, 0, 31, j) for j in range(20)])
     before, plain = _both(e, 0, 8192)
     assert np.array_equal(before, plain)
-    free, _ = dm.mem_info()  # counts what the sums hold as free
-    taken = [irisb200.DeviceBuffer(dm, free - (3 << 30))]
-    assert dm.mem_info()[0] < (4 << 30)  # it fitted only in what the sums held
+    dm.synchronize()
+    g = irisb200.Graph.capture(dm, lambda: e.dot(0, 8192, 1, dm.stream(0))) if captured else None
+    taken = []  # mem_info counts what the sums hold as free (the driver may find more in its pools)
+    while dm.mem_info()[0] > (4 << 30):
+        taken.append(irisb200.DeviceBuffer(dm, dm.mem_info()[0] - (3 << 30)))
     after, _ = _both(e, 0, 8192)
     assert np.array_equal(after, plain)
+    if captured:
+        for _ in range(2):
+            g.launch(dm.stream(0))
+            assert np.array_equal(e.fetch_results(8192), plain)
+            e.query_upload_slots(base, [(j, 0, 31, j) for j in range(20)])
+        dm.synchronize()
+        g.close()
     e.query_upload_slots(base, [(j, 0, 31, j) for j in range(20)])
     assert np.array_equal(_both(e, 0, 8192)[0], plain)
     for b in taken:
