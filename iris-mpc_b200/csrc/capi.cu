@@ -2107,14 +2107,18 @@ int irs_graph_end_capture(irs_device_manager* dm, irs_graph** out) {
 
 int irs_graph_launch(irs_graph* g, void* stream) {
   CHECK(g && g->exec, IRS_ERR_INVALID, "graph is NULL");
-  // the graph's GEMMs read what the parties' streams have uploaded
-  for (int p = 0; p < 3; p++)
+  // the graph's GEMMs read what the parties' streams have uploaded (a launch
+  // that is captured itself cannot wait for work outside its capture)
+  const bool captured = stream_captures(static_cast<cudaStream_t>(stream));
+  for (int p = 0; p < 3 && !captured; p++)
     if (g->dm->streams[p] != static_cast<cudaStream_t>(stream)) {
       CU(cudaEventRecord(g->dm->uploads[p], g->dm->streams[p]));
       CU(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), g->dm->uploads[p], 0));
     }
   {
     std::lock_guard<std::mutex> lock(sum_holders().mu);
+    for (irs_sharedb* db : sum_holders().engines)
+      if (captured && db->dm == g->dm && db->dot_captured) db->sums_pinned = true;  // replays outside this lock
     CU(cudaGraphLaunch(g->exec, static_cast<cudaStream_t>(stream)));
   }
   // later query uploads on other party streams wait for the graph's GEMMs

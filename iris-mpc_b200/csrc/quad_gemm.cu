@@ -18,13 +18,13 @@
 // columns divide by both, and rows i, i+2, i+4, i+6 of a slot form a quad.
 // The additions run in Z_2^16 before the limb split: on the DB side once per
 // record (derive_sums_kernel), on the query side once per upload
-// (expand_quads_kernel), on the products in the epilogue.
+// (expand_kernel), on the products in the epilogue.
 //
 // Every term is exact modulo 2^16, so the dot shares equal the limb GEMM's
 // (gemm_limb.cu) bit for bit; the limbs, the keystream positions and the
 // result layout are the same.
 //
-// What bounds it: the board's power limit, with the tensor pipe 79% active at
+// What bounds it: the board's power limit, with the tensor pipe 78% active at
 // the clock that leaves (ncu, 16,384 entries x 2048 rows; 92% of the rounds of
 // tiles are full there).  Six engines over 131,072 entries x 2048 rows: 18.4 ms
 // at 1530 MHz, against 30.7 ms at 1400 MHz for the two-SM limb GEMM.  The sums
