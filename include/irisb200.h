@@ -274,6 +274,10 @@ int irs_sharedb_set_tile(irs_sharedb* db, int block_n);
  * rows trade clock for MAC rate, so the batch autotuner decides there (no
  * counterpart in the reference). */
 int irs_sharedb_set_pair(irs_sharedb* db, int on);
+/* *on = 1 while the engine holds the derived sums of its records that the
+ * rotation-structured GEMM needs (see alloc_db), for callers that place query
+ * rows themselves (no counterpart in the reference). */
+int irs_sharedb_has_sums(irs_sharedb* db, int* on);
 int irs_sharedb_use_batch_counter(irs_sharedb* db, int on);
 /* Starts a new batch: the zero-share mask and circuit keystreams are drawn at
  * ChaCha counter (batch_id << 40) | position (ChaChaCtx counter,

@@ -93,6 +93,7 @@ extern "C" {
     pub fn irs_mirror_query_share(coefs: *mut u16, n: usize, flip_imaginary: c_int) -> c_int;
     pub fn irs_sharedb_set_tile(db: *mut IrsShareDb, block_n: c_int) -> c_int;
     pub fn irs_sharedb_set_pair(db: *mut IrsShareDb, on: c_int) -> c_int;
+    pub fn irs_sharedb_has_sums(db: *mut IrsShareDb, on: *mut c_int) -> c_int;
     pub fn irs_sharedb_use_batch_counter(db: *mut IrsShareDb, on: c_int) -> c_int;
     pub fn irs_sharedb_set_batch(db: *mut IrsShareDb, batch_id: u64) -> c_int;
     pub fn irs_sharedb_dot(db: *mut IrsShareDb, offset: usize, len: usize, multiplier: u16,

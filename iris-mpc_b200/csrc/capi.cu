@@ -1250,6 +1250,13 @@ int irs_sharedb_set_pair(irs_sharedb* db, int on) {
   return IRS_OK;
 }
 
+int irs_sharedb_has_sums(irs_sharedb* db, int* on) {
+  CHECK(db && on, IRS_ERR_INVALID, "bad arguments");
+  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  *on = db->sums != nullptr;
+  return IRS_OK;
+}
+
 int irs_sharedb_set_batch(irs_sharedb* db, uint64_t batch_id) {
   CHECK(db, IRS_ERR_INVALID, "db is NULL");
   CHECK(batch_id < (1ull << 24), IRS_ERR_INVALID, "batch id must be below 2^24");

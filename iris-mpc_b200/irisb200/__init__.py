@@ -113,6 +113,7 @@ _SIGS = {
     "irs_sharedb_set_batch": [_vp, _u64],
     "irs_sharedb_set_tile": [_vp, _i],
     "irs_sharedb_set_pair": [_vp, _i],
+    "irs_sharedb_has_sums": [_vp, C.POINTER(_i)],
     "irs_sharedb_use_batch_counter": [_vp, _i],
     "irs_circuits_use_batch_counter": [_vp, _i],
     "irs_device_manager_set_batch_counter": [_vp, _u64, _vp],
@@ -536,6 +537,12 @@ class ShareDB:
     def set_pair(self, on: bool) -> None:
         """The GEMM on SM pairs wherever it can run so (irs_sharedb_set_pair)."""
         _check(lib().irs_sharedb_set_pair(self.h, int(on)))
+
+    def has_sums(self) -> bool:
+        """Whether the engine holds what the quad GEMM needs (irs_sharedb_has_sums)."""
+        on = _i()
+        _check(lib().irs_sharedb_has_sums(self.h, C.byref(on)))
+        return bool(on.value)
 
     def set_tile(self, block_n: int) -> None:
         _check(lib().irs_sharedb_set_tile(self.h, block_n))

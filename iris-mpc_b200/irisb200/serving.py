@@ -121,6 +121,9 @@ class ContinuousServer:
     results, with the library in its asynchronous host mode and every host
     buffer it reads or writes page-locked and double-buffered."""
 
+    quads = True      # the engines hold what the library's quad GEMM needs
+    slots_in_use = 0  # words that held rows when the layout was last made
+
     def __init__(self, dm, code_engines, mask_engines, circuits, chunk: int = 32768, row_capacity: int = 2048,
                  max_variants: int = 512, max_reauth: int = 64, threshold_a: int = 16384, seeds=None,
                  db_capacity: int | None = None, gemm_pair: bool = True):
@@ -136,6 +139,7 @@ class ContinuousServer:
         # 16,384- or 8,192-entry steps
         for e in self.ce + self.me:
             e.set_pair(gemm_pair)
+        self.quads = all(e.has_sums() for e in self.ce + self.me)
         self.c = circuits
         self.A = threshold_a
         self.chunk = max(32, chunk // 32 * 32)
@@ -206,12 +210,14 @@ class ContinuousServer:
     def _place(self, n: int):
         """First free run of n rows: once as many words are in use as the
         library's quad GEMM takes (words fill from the front), with its quads
-        of rows to itself where there is such a run; else any."""
-        if self.row_capacity >= QUAD_MIN_ROWS and self.slot_occ[QUAD_MIN_ROWS // 32 - 3]:
+        of rows to itself, or none until others complete; else any."""
+        busy = QUAD_MIN_ROWS // 32 - 3
+        if self.quads and self.n_slot_cap > busy + 2 and (self.slot_occ[busy] or self.slots_in_use > busy):
             for s in range(self.n_slot_cap):
                 q = first_quads(_quads_of(self.slot_occ[s]), n)
                 if q >= 0:
                     return s, q // 2 * 8 + q % 2
+            return None
         for s in range(self.n_slot_cap):
             f = _first_run(self.slot_occ[s], n)
             if f >= 0:
@@ -274,6 +280,7 @@ class ContinuousServer:
         """Row table and segment table of the current placement."""
         used = [s for s in range(self.n_slot_cap) if self.slot_occ[s]]
         n_slots = used[-1] + 1 if used else 1
+        self.slots_in_use = len(used)
         # empty rows pad the table for the GEMM's widest tile (padded_rows); the
         # threshold kernel only visits the slots that carry segments
         n_rows = min(padded_rows(n_slots * 32, self.row_capacity), self.row_capacity)

@@ -230,8 +230,11 @@ def test_placement_in_a_large_server_keeps_quads_apart():
         vs.append((v, pure))
         if len(vs) > 20 and rng.random() < 0.5:
             s._release(vs.pop(int(rng.integers(len(vs))))[0])
-    first_mixed = next((i for i, (_, pure) in enumerate(vs) if not pure), len(vs))
-    assert first_mixed > 20  # quads are shared only once the server is nearly full
+    assert len(vs) > 20 and all(pure for _, pure in vs)
+    s.quads = False  # engines without the sums: any row
+    while s._place(1) is not None:
+        s._occupy(_Variant(-1, False, [0]), *s._place(1))
+    assert all(o == 0xFFFFFFFF for o in s.slot_occ)
     for q in range(8):  # the quads of a word, row by row
         for r in range(32):
             assert bool(_quads_of(1 << r) >> (r // 8 * 2 + r % 2) & 1)
