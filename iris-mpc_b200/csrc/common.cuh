@@ -150,11 +150,15 @@ IRS_HD void chacha12_block_prepared(const uint32_t* pre, uint32_t ctr_lo, uint32
 
 // Packed 16-bit lane arithmetic (two u16 per u32, no carry across lanes).
 IRS_HD uint32_t add2(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+  uint32_t d;
+  asm("add.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+#else
   return ((a & 0x7fff7fffu) + (b & 0x7fff7fffu)) ^ ((a ^ b) & 0x80008000u);
+#endif
 }
-IRS_HD uint32_t sub2(uint32_t a, uint32_t b) {
-  return ((a | 0x80008000u) - (b & 0x7fff7fffu)) ^ ((a ^ ~b) & 0x80008000u);
-}
+IRS_HD uint32_t sub2(uint32_t a, uint32_t b) { return ~add2(~a, b); }
 
 #ifdef __CUDACC__
 __device__ __forceinline__ uint64_t globaltimer_ns() {
