@@ -916,7 +916,7 @@ def threshold_roofline(thr_ms: float, words: int, n_sm: int, sm_mhz, chunks) -> 
         out["counters_source"] = pj.get("source")
         if pj.get("alu_pipe_pct") is not None:
             # the binding pipe: the integer ALU pipe is busier than the issue
-            # slots (87.5% against 71.3% in the capture), so it sets the limit
+            # slots (87.1% against 71.9% in the capture), so it sets the limit
             out["binding_pipe"] = {"pipe": "alu", "frac": pj["alu_pipe_pct"] / 100.0,
                                    "issue_frac": pj.get("issue_active_pct", 0.0) / 100.0,
                                    "source": "ncu sm__inst_executed_pipe_alu (pct of peak sustained active), "

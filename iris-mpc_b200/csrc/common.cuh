@@ -148,7 +148,9 @@ IRS_HD void chacha12_block_prepared(const uint32_t* pre, uint32_t ctr_lo, uint32
 #undef IRS_ROT16
 #undef IRS_ROT8
 
-// Packed 16-bit lane arithmetic (two u16 per u32, no carry across lanes).
+// Packed 16-bit lane arithmetic (two u16 per u32, no carry across lanes).  One
+// instruction for the add, in place of the five of the form below: it counts
+// where the integer pipe is the limit (2^24 comparisons 411 -> 403 us).
 IRS_HD uint32_t add2(uint32_t a, uint32_t b) {
 #ifdef __CUDA_ARCH__
   uint32_t d;

@@ -26,7 +26,7 @@
 //
 // What bounds it: the board's power limit, with the tensor pipe 78% active at
 // the clock that leaves (ncu, 16,384 entries x 2048 rows; 92% of the rounds of
-// tiles are full there).  Six engines over 131,072 entries x 2048 rows: 18.4 ms
+// tiles are full there).  Six engines over 131,072 entries x 2048 rows: 18.1 ms
 // at 1530 MHz, against 30.7 ms at 1400 MHz for the two-SM limb GEMM.  The sums
 // make 2.25x the DB bytes (5.5 GB read per 16,384-entry launch), which is why
 // few query rows keep the plain kernel.
