@@ -68,7 +68,9 @@ struct irs_device_manager {
   int* d_err = nullptr;
   uint64_t* d_batch = nullptr;  // device batch counter (irs_device_manager_set_batch_counter)
   bool capturing = false;  // a graph capture on streams[0] is open
-  cudaEvent_t graph_done = nullptr;  // recorded after each graph launch
+  cudaEvent_t graph_done = nullptr;  // complete when every graph launched so far has run
+  cudaStream_t graph_join = nullptr;  // the graphs' streams meet here, and graph_done follows them
+  cudaEvent_t graph_ran = nullptr;    // recorded after each graph launch, on its stream
   cudaEvent_t uploads[3] = {nullptr, nullptr, nullptr};  // recorded on the parties' streams before one
   bool host_sync = true;  // false: host-buffer calls return once enqueued (irs_device_manager_set_host_sync)
   // stage timers (irs_device_manager_set_timing): event pairs per label, resolved on read
@@ -584,6 +586,8 @@ int irs_device_manager_init(int device, irs_device_manager** out) {
   CU(cudaMalloc(&dm->d_batch, sizeof(uint64_t)));
   CU(cudaMemset(dm->d_batch, 0, sizeof(uint64_t)));
   CU(cudaEventCreateWithFlags(&dm->graph_done, cudaEventDisableTiming));
+  CU(cudaEventCreateWithFlags(&dm->graph_ran, cudaEventDisableTiming));
+  CU(cudaStreamCreateWithFlags(&dm->graph_join, cudaStreamNonBlocking));
   for (cudaEvent_t& e : dm->uploads) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   *out = dm;
   return IRS_OK;
@@ -596,6 +600,8 @@ int irs_device_manager_destroy(irs_device_manager* dm) {
   cudaFree(dm->d_err);
   cudaFree(dm->d_batch);
   if (dm->graph_done) cudaEventDestroy(dm->graph_done);
+  if (dm->graph_ran) cudaEventDestroy(dm->graph_ran);
+  if (dm->graph_join) cudaStreamDestroy(dm->graph_join);
   for (cudaEvent_t e : dm->uploads)
     if (e) cudaEventDestroy(e);
   for (auto& t : dm->timers) {
@@ -1052,7 +1058,7 @@ int irs_sharedb_synth_db(irs_sharedb* const code_engines[3], irs_sharedb* const 
 }
 
 // Orders a write to an engine's query rows or records on stream s after the
-// last GEMM that read them (a direct launch, or a graph launch).
+// last GEMMs that read them (a direct launch, and every graph launch).
 static cudaError_t wait_last_dot(irs_sharedb* db, cudaStream_t s) {
   cudaError_t e = cudaStreamWaitEvent(s, db->done, 0);
   if (e != cudaSuccess) return e;
@@ -2128,8 +2134,16 @@ int irs_graph_launch(irs_graph* g, void* stream) {
       if (captured && db->dm == g->dm && db->dot_captured) db->sums_pinned = true;  // replays outside this lock
     CU(cudaGraphLaunch(g->exec, static_cast<cudaStream_t>(stream)));
   }
-  // later query uploads on other party streams wait for the graph's GEMMs
-  CU(cudaEventRecord(g->dm->graph_done, static_cast<cudaStream_t>(stream)));
+  // Later query uploads on other party streams wait for the graph's GEMMs, and
+  // for those of every graph before it: graphs over different engines may run
+  // on different streams, and an upload knows only the engine it writes.
+  if (captured) {  // part of another capture: the event belongs to it
+    CU(cudaEventRecord(g->dm->graph_done, static_cast<cudaStream_t>(stream)));
+    return IRS_OK;
+  }
+  CU(cudaEventRecord(g->dm->graph_ran, static_cast<cudaStream_t>(stream)));
+  CU(cudaStreamWaitEvent(g->dm->graph_join, g->dm->graph_ran, 0));
+  CU(cudaEventRecord(g->dm->graph_done, g->dm->graph_join));
   return IRS_OK;
 }
 

@@ -71,7 +71,7 @@ __device__ __forceinline__ bool tile_of(const GemmParams& P, int t, Tile& out) {
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1) limb_gemm_kernel(const __grid_constant__ GemmParams P) {
   using C = Cfg<BN>;
-  if (P.skip.n && P.skip.all_set()) return;  // the quad GEMM runs; the same words for every CTA
+  if (P.skip.n && P.skip.all_set()) return;  // the quad GEMM runs
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* a_lo = smem;
@@ -292,7 +292,6 @@ constexpr int pair_stage_bytes(int bn) { return 2 * 128 * kBK + 2 * (bn / 2) * k
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     limb_gemm_pair_kernel(const __grid_constant__ GemmParams P) {
-  if (P.skip.n && P.skip.all_set()) return;  // the quad GEMM runs; the same words for every CTA
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int n_stages = P.pair_stages;
@@ -324,6 +323,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   int* err = P.err;
   const uint64_t lim = P.wait_timeout_ns, lim2 = 2 * P.wait_timeout_ns;
 
+  if (P.skip.n && cluster_reads(P.skip, tmem_slot)) return;  // the quad GEMM runs
   if (threadIdx.x == 0) {
     for (int s = 0; s < n_stages; s++) {
       mbar_init(&full_bar[s], 1);
@@ -536,6 +536,7 @@ __global__ void __cluster_dims__(S, 1, 1) __launch_bounds__(kThreads, 1)
   const GemmProblem& pr = P.prob[tl.prob];
   const uint32_t k_begin = pr.k_iters * (uint32_t)rank / S, k_end = pr.k_iters * (uint32_t)(rank + 1) / S;
 
+  if (P.skip.n && cluster_reads(P.skip, tmem_slot)) return;  // the quad GEMM runs
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; s++) {
       mbar_init(&full_bar[s], 1);

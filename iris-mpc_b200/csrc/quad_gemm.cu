@@ -143,7 +143,6 @@ __device__ __noinline__ void put_slot(const QuadProblem& pr, uint32_t m_local, u
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     quad_gemm_kernel(const __grid_constant__ QuadParams P) {
-  if (P.run.n && !P.run.all_set()) return;  // the same words for every CTA
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int bn = P.tile_n, half_n = bn / 2;
@@ -170,6 +169,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
   int* err = P.err;
   const uint64_t lim = P.wait_timeout_ns, lim2 = 2 * P.wait_timeout_ns;
 
+  if (P.run.n && !cluster_reads(P.run, tmem_slot)) return;
   if (threadIdx.x == 0) {
     for (int s = 0; s < n_stages; s++) {
       mbar_init(&full_bar[s], 1);

@@ -3,6 +3,7 @@
 // barrier, the paired MMA and its multicast commit.  Used by the two-SM limb
 // GEMM (gemm_limb.cu) and the rotation-structured GEMM (quad_gemm.cu).
 #pragma once
+#include "gemm_limb.h"
 #include "tc_sm100.cuh"
 
 namespace irs {
@@ -22,8 +23,28 @@ __device__ __forceinline__ uint32_t map_to_rank(const void* p, uint32_t rank) {
   return r;
 }
 
+__device__ __forceinline__ uint32_t ld_cluster(uint32_t cluster_addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// QuadFlags::all_set as the cluster's first CTA reads it, for every thread of
+// the cluster.  Its CTAs share barriers and tensor memory, so none may work
+// where another has left; and the words can change between two readings, where
+// the program writes an engine's rows while a graph over it runs.  `slot` is a
+// word of shared memory at the same offset in every CTA.
+__device__ __forceinline__ bool cluster_reads(const QuadFlags& flags, uint32_t* slot) {
+  if (threadIdx.x == 0) *slot = flags.all_set();
+  __syncthreads();
+  cluster_sync_all();
+  const bool all = ld_cluster(map_to_rank(slot, 0)) != 0;
+  cluster_sync_all();  // the first CTA stays until the others have read its word
+  return all;
 }
 
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
