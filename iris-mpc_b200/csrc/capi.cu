@@ -71,7 +71,7 @@ struct irs_device_manager {
   cudaEvent_t graph_done = nullptr;  // complete when every graph launched so far has run
   cudaStream_t graph_join = nullptr;  // the graphs' streams meet here, and graph_done follows them
   cudaEvent_t graph_ran = nullptr;    // recorded after each graph launch, on its stream
-  cudaEvent_t uploads[3] = {nullptr, nullptr, nullptr};  // recorded on the parties' streams before one
+  cudaEvent_t uploads[3] = {nullptr, nullptr, nullptr};  // recorded on the parties' streams before one (and before a capture)
   bool host_sync = true;  // false: host-buffer calls return once enqueued (irs_device_manager_set_host_sync)
   // stage timers (irs_device_manager_set_timing): event pairs per label, resolved on read
   bool timing = false;
@@ -2089,6 +2089,7 @@ int irs_graph_begin_capture(irs_device_manager* dm) {
   CHECK(dm, IRS_ERR_INVALID, "dm is NULL");
   CHECK(!dm->capturing, IRS_ERR_STATE, "a capture is already open");
   CU(cudaSetDevice(dm->device));
+  CU(cudaEventRecord(dm->uploads[0], dm->streams[0]));  // for graph launches beside the capture
   CU(cudaStreamBeginCapture(dm->streams[0], cudaStreamCaptureModeThreadLocal));
   dm->capturing = true;
   return IRS_OK;
@@ -2125,7 +2126,9 @@ int irs_graph_launch(irs_graph* g, void* stream) {
   const bool captured = stream_captures(static_cast<cudaStream_t>(stream));
   for (int p = 0; p < 3 && !captured; p++)
     if (g->dm->streams[p] != static_cast<cudaStream_t>(stream)) {
-      CU(cudaEventRecord(g->dm->uploads[p], g->dm->streams[p]));
+      // (a party's stream that is being captured: its uploads ended with the
+      // event that irs_graph_begin_capture recorded)
+      if (!stream_captures(g->dm->streams[p])) CU(cudaEventRecord(g->dm->uploads[p], g->dm->streams[p]));
       CU(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), g->dm->uploads[p], 0));
     }
   {
