@@ -278,6 +278,18 @@ int irs_sharedb_set_pair(irs_sharedb* db, int on);
  * rotation-structured GEMM needs (see alloc_db), for callers that place query
  * rows themselves (no counterpart in the reference). */
 int irs_sharedb_has_sums(irs_sharedb* db, int* on);
+/* The GEMM that the engine's last dot launched (no counterpart in the
+ * reference): IRS_GEMM_ONE_SM, IRS_GEMM_PAIR (on SM pairs), IRS_GEMM_QUAD (the
+ * rotation-structured one), or IRS_GEMM_CAPTURED for a captured dot that holds
+ * IRS_GEMM_QUAD and a plain one, of which every replay takes the one that the
+ * rows uploaded by then need.  *quad_rows: the padded row count for which a
+ * replay after the last upload takes IRS_GEMM_QUAD, 0 for none. */
+#define IRS_GEMM_NONE 0
+#define IRS_GEMM_ONE_SM 1
+#define IRS_GEMM_PAIR 2
+#define IRS_GEMM_QUAD 3
+#define IRS_GEMM_CAPTURED 4
+int irs_sharedb_last_gemm(irs_sharedb* db, int* gemm, size_t* quad_rows);
 int irs_sharedb_use_batch_counter(irs_sharedb* db, int on);
 /* Starts a new batch: the zero-share mask and circuit keystreams are drawn at
  * ChaCha counter (batch_id << 40) | position (ChaChaCtx counter,

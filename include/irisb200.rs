@@ -19,6 +19,12 @@ pub struct IrsQuerySlot { pub src: u32, pub rot_lo: u32, pub n_rot: u32, pub que
 pub const IRS_SCAN_SPLIT: i32 = 0;
 pub const IRS_SCAN_PAIR: i32 = 1;
 pub const IRS_SCAN_FUSED: i32 = 2;
+
+pub const IRS_GEMM_NONE: i32 = 0;
+pub const IRS_GEMM_ONE_SM: i32 = 1;
+pub const IRS_GEMM_PAIR: i32 = 2;
+pub const IRS_GEMM_QUAD: i32 = 3;
+pub const IRS_GEMM_CAPTURED: i32 = 4;
 #[repr(C)] #[derive(Clone, Copy)]
 pub struct IrsScanCandidate { pub path: i32, pub tile: i32, pub chunk: u64 }
 #[repr(C)] #[derive(Clone, Copy)]
@@ -94,6 +100,7 @@ extern "C" {
     pub fn irs_sharedb_set_tile(db: *mut IrsShareDb, block_n: c_int) -> c_int;
     pub fn irs_sharedb_set_pair(db: *mut IrsShareDb, on: c_int) -> c_int;
     pub fn irs_sharedb_has_sums(db: *mut IrsShareDb, on: *mut c_int) -> c_int;
+    pub fn irs_sharedb_last_gemm(db: *mut IrsShareDb, gemm: *mut c_int, quad_rows: *mut usize) -> c_int;
     pub fn irs_sharedb_use_batch_counter(db: *mut IrsShareDb, on: c_int) -> c_int;
     pub fn irs_sharedb_set_batch(db: *mut IrsShareDb, batch_id: u64) -> c_int;
     pub fn irs_sharedb_dot(db: *mut IrsShareDb, offset: usize, len: usize, multiplier: u16,

@@ -138,6 +138,7 @@ struct irs_sharedb {
   // results [max_db][n_pad] u16 (entry-major)
   uint16_t* results = nullptr;
   size_t res_offset = 0, res_len = 0;
+  int last_gemm = IRS_GEMM_NONE;
   uint64_t batch = 0;
   // rotation-structured GEMM (quad_gemm.cu): the records' derived sums, one
   // allocation (outer lo, hi [db_cap][K/2], inner lo, hi [db_cap][3K/4]), and
@@ -1263,6 +1264,14 @@ int irs_sharedb_has_sums(irs_sharedb* db, int* on) {
   return IRS_OK;
 }
 
+int irs_sharedb_last_gemm(irs_sharedb* db, int* gemm, size_t* quad_rows) {
+  CHECK(db && gemm && quad_rows, IRS_ERR_INVALID, "bad arguments");
+  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  *gemm = db->last_gemm;
+  *quad_rows = db->sums ? db->flag_rows : 0;
+  return IRS_OK;
+}
+
 int irs_sharedb_set_batch(irs_sharedb* db, uint64_t batch_id) {
   CHECK(db, IRS_ERR_INVALID, "db is NULL");
   CHECK(batch_id < (1ull << 24), IRS_ERR_INVALID, "batch id must be below 2^24");
@@ -1443,6 +1452,9 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
       CU(launch_quad_gemm(Q, dm->n_sms, s));
     }
     if (!quads || captured) CU(launch_limb_gemm(P, few ? 128 : engines[0]->block_n, pair, dm->n_sms, s));
+    for (int i = 0; i < n; i++)
+      engines[i]->last_gemm =
+          quads ? (captured ? IRS_GEMM_CAPTURED : IRS_GEMM_QUAD) : pair ? IRS_GEMM_PAIR : IRS_GEMM_ONE_SM;
   }
   for (int i = 0; i < n; i++) {
     engines[i]->res_offset = offset;

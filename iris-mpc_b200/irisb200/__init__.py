@@ -114,6 +114,7 @@ _SIGS = {
     "irs_sharedb_set_tile": [_vp, _i],
     "irs_sharedb_set_pair": [_vp, _i],
     "irs_sharedb_has_sums": [_vp, C.POINTER(_i)],
+    "irs_sharedb_last_gemm": [_vp, C.POINTER(_i), C.POINTER(_sz)],
     "irs_sharedb_use_batch_counter": [_vp, _i],
     "irs_circuits_use_batch_counter": [_vp, _i],
     "irs_device_manager_set_batch_counter": [_vp, _u64, _vp],
@@ -482,6 +483,9 @@ class DeviceManager:
             self.h = None
 
 
+GEMMS = ("none", "one_sm", "pair", "quad", "captured")  # IRS_GEMM_*
+
+
 class ShareDB:
     """ShareDB (iris-mpc-gpu/src/dot/share_db.rs:448-1070) of one party."""
 
@@ -543,6 +547,13 @@ class ShareDB:
         on = _i()
         _check(lib().irs_sharedb_has_sums(self.h, C.byref(on)))
         return bool(on.value)
+
+    def last_gemm(self):
+        """(name in GEMMS of what the last dot launched, padded rows that a
+        replay of a captured one takes as quads) (irs_sharedb_last_gemm)."""
+        gemm, rows = _i(), _sz()
+        _check(lib().irs_sharedb_last_gemm(self.h, C.byref(gemm), C.byref(rows)))
+        return GEMMS[gemm.value], rows.value
 
     def set_tile(self, block_n: int) -> None:
         _check(lib().irs_sharedb_set_tile(self.h, block_n))
