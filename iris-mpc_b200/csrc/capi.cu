@@ -316,6 +316,7 @@ void pool_free(irs_device_manager* dm, int party, void* p) {
 // cudaFreeAsync): unlike pool_alloc it does not wait for the stream.
 int scratch_alloc(irs_device_manager* dm, cudaStream_t s, size_t bytes, void** out) {
   *out = nullptr;
+  if (!bytes) return IRS_OK;
   cudaError_t e = cudaMallocFromPoolAsync(out, bytes, dm->pools[0], s);
   if (e == cudaErrorMemoryAllocation && !dm->capturing) {
     cudaGetLastError();
@@ -1551,6 +1552,20 @@ __global__ void scatter_views_kernel(const uint32_t* comp, size_t n_words32, uin
   if (opened) opened[i] = c0 ^ c1 ^ c2;
 }
 
+// Begins a call over flat share vectors on stream s.  Work of party 0's stream
+// comes first, whichever stream the caller chose: the shares may be dot results
+// that it is still writing.  Such calls take scratch memory and may wait, so
+// they are not captured (irs_circuits_compare_threshold_masked_many_noalloc is).
+static int begin_flat(irs_device_manager* dm, cudaStream_t s) {
+  CU(cudaSetDevice(dm->device));
+  CHECK(!dm->capturing && !stream_captures(s), IRS_ERR_CUDA,
+        "a call over flat shares cannot be captured; the no-allocation entry point can");
+  if (s == dm->streams[0] || stream_captures(dm->streams[0])) return IRS_OK;
+  CU(cudaEventRecord(dm->uploads[0], dm->streams[0]));
+  CU(cudaStreamWaitEvent(s, dm->uploads[0], 0));
+  return IRS_OK;
+}
+
 // Whether a result array of a flat call shares memory with an input: the kernel
 // then may not write results while other words' shares are still to be read.
 static bool results_overlap_shares(const ThresholdParams& P, int stage, uint64_t* const res_a[3],
@@ -1579,8 +1594,9 @@ static int run_flat(irs_circuits* c, const uint16_t* const code_a[3], const uint
           IRS_ERR_INVALID, "share pointers must be 16-byte aligned");
   }
   irs_device_manager* dm = c->dm;
-  CU(cudaSetDevice(dm->device));
   cudaStream_t s = party_stream(dm, 0, stream);
+  int rc = begin_flat(dm, s);
+  if (rc) return rc;
   ThresholdParams P;
   base_params(c, P);
   for (int p = 0; p < 3; p++) {
@@ -1602,7 +1618,7 @@ static int run_flat(irs_circuits* c, const uint16_t* const code_a[3], const uint
   // (or results over the shares: every share is read before the first is written)
   uint32_t* comp = nullptr;
   void* p;
-  int rc = scratch_alloc(dm, s, 3 * P.n_words * 4, &p);
+  rc = scratch_alloc(dm, s, 3 * P.n_words * 4, &p);
   if (rc) return rc;
   comp = (uint32_t*)p;
   P.res_comp = comp;
@@ -1658,12 +1674,13 @@ int irs_circuits_or_reduce(irs_circuits* c, const uint64_t* const res_a[3], size
   CHECK(n > 0 && n % 64 == 0, IRS_ERR_INVALID, "n = %zu must be a positive multiple of 64", n);
   for (int p = 0; p < 3; p++) CHECK(res_a[p], IRS_ERR_INVALID, "share pointer missing");
   irs_device_manager* dm = c->dm;
-  CU(cudaSetDevice(dm->device));
   cudaStream_t s = party_stream(dm, 0, stream);
+  int rc = begin_flat(dm, s);
+  if (rc) return rc;
   const size_t n_words = n / 32;
   // gather the three a-shares (u64 words = pairs of u32 words) into one [3][n_words] vector
   void* p;
-  int rc = scratch_alloc(dm, s, 3 * n_words * 4, &p);
+  rc = scratch_alloc(dm, s, 3 * n_words * 4, &p);
   if (rc) return rc;
   uint32_t* comp = static_cast<uint32_t*>(p);
   cudaError_t e = cudaSuccess;
@@ -1685,8 +1702,9 @@ int irs_circuits_compare_threshold_masked_many_with_or_tree(irs_circuits* c, con
           "share pointers must be 16-byte aligned");
   }
   irs_device_manager* dm = c->dm;
-  CU(cudaSetDevice(dm->device));
   cudaStream_t s = party_stream(dm, 0, stream);
+  int rc = begin_flat(dm, s);
+  if (rc) return rc;
   ThresholdParams P;
   base_params(c, P);
   for (int p = 0; p < 3; p++) {
@@ -1696,7 +1714,7 @@ int irs_circuits_compare_threshold_masked_many_with_or_tree(irs_circuits* c, con
   P.threshold_a = threshold_a;
   P.n_words = n / 32;
   void* p;
-  int rc = scratch_alloc(dm, s, 3 * P.n_words * 4, &p);
+  rc = scratch_alloc(dm, s, 3 * P.n_words * 4, &p);
   if (rc) return rc;
   P.res_comp = static_cast<uint32_t*>(p);
   cudaError_t e = launch_threshold_flat(P, kStageFull, s);
@@ -1717,8 +1735,9 @@ int irs_circuits_lift_mpc(irs_circuits* c, const uint16_t* const mask_a[3], size
   CHECK(c && mask_a && corr, IRS_ERR_INVALID, "bad arguments");
   CHECK(n % 64 == 0, IRS_ERR_INVALID, "n = %zu must be a multiple of 64", n);
   irs_device_manager* dm = c->dm;
-  CU(cudaSetDevice(dm->device));
   cudaStream_t s = party_stream(dm, 0, stream);
+  int rc = begin_flat(dm, s);
+  if (rc) return rc;
   ThresholdParams P;
   base_params(c, P);
   for (int p = 0; p < 3; p++) {
@@ -1728,7 +1747,7 @@ int irs_circuits_lift_mpc(irs_circuits* c, const uint16_t* const mask_a[3], size
   }
   P.n_words = n / 32;
   void* p;
-  int rc = scratch_alloc(dm, s, 6 * n * 2, &p);
+  rc = scratch_alloc(dm, s, 6 * n * 2, &p);
   if (rc) return rc;
   uint16_t* tmp = (uint16_t*)p;
   cudaError_t e = launch_lift_flat(P, tmp, s);
