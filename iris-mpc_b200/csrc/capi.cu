@@ -965,27 +965,28 @@ int irs_sharedb_load_records_i8(irs_sharedb* db, size_t first, size_t n, const u
   CU(cudaSetDevice(dm->device));
   cudaStream_t s = dm->streams[db->peer];
   const size_t K = db->code_length;
-  // through a bounded staging buffer of its own (the query staging may hold a
-  // server's resident bases)
-  const size_t per = std::min<size_t>(n, std::max<size_t>(1, (64u << 20) / K));
-  void* stage = nullptr;
-  int rc = n ? pool_alloc(dm, db->peer, 2 * per * K, &stage) : IRS_OK;
-  if (rc) return rc;
-  uint8_t* st = static_cast<uint8_t*>(stage);
-  cudaError_t e = cudaSuccess;
-  for (size_t done = 0; done < n && e == cudaSuccess;) {
-    const size_t c = std::min(per, n - done), at = (first + done) * K;
-    e = cudaMemcpyAsync(st, limb0 + done * K, c * K, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(st + per * K, limb1 + done * K, c * K, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = launch_i8_plane(st, (uint32_t)K, db->db_lo + at, c * K, s);
-    if (e == cudaSuccess) e = launch_i8_plane(st + per * K, (uint32_t)K, db->db_hi + at, c * K, s);
-    if (e == cudaSuccess) e = update_sums(db, first + done, c, s);
-    done += c;
+  uint8_t* planes[2] = {db->db_lo + first * K, db->db_hi + first * K};
+  const uint8_t* limbs[2] = {limb0, limb1};
+  if (i8_plane_in_place(K)) {
+    for (int l = 0; l < 2; l++) {
+      CU(cudaMemcpyAsync(planes[l], limbs[l], n * K, cudaMemcpyHostToDevice, s));
+      CU(launch_i8_plane(planes[l], (uint32_t)K, planes[l], n, s));
+    }
+  } else {  // a row at a time (the query staging may hold a server's resident bases)
+    void* stage = nullptr;
+    int rc = n ? pool_alloc(dm, db->peer, K, &stage) : IRS_OK;
+    if (rc) return rc;
+    cudaError_t e = cudaSuccess;
+    for (size_t r = 0; r < 2 * n && e == cudaSuccess; r++) {
+      e = cudaMemcpyAsync(stage, limbs[r & 1] + r / 2 * K, K, cudaMemcpyHostToDevice, s);
+      if (e == cudaSuccess)
+        e = launch_i8_plane(static_cast<uint8_t*>(stage), (uint32_t)K, planes[r & 1] + r / 2 * K, 1, s);
+    }
+    pool_free(dm, db->peer, stage);
+    CU(e);
   }
-  if (stage) pool_free(dm, db->peer, stage);
-  const cudaError_t sync = cudaStreamSynchronize(s);
-  CU(e);
-  CU(sync);
+  CU(update_sums(db, first, n, s));
+  CU(cudaStreamSynchronize(s));
   db->db_len = std::max(db->db_len, first + n);
   return IRS_OK;
 }

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "common.cuh"
+#include "launch_attr.cuh"
 #include "prep.h"
 
 namespace irs {
@@ -48,15 +49,26 @@ __global__ void split_limbs_kernel(const uint16_t* __restrict__ in, uint32_t K, 
   reinterpret_cast<uint2*>(hi)[d] = make_uint2(high_bytes(a), high_bytes(b));
 }
 
-// Stored i8 limbs (byte - 128) in record order to a plane, one thread per octet.
-__global__ void i8_plane_kernel(const uint8_t* __restrict__ in, uint32_t K, uint8_t* __restrict__ out, size_t n8) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n8) return;
-  const uint2 v = reinterpret_cast<const uint2*>(in)[i];
+// Stored i8 limbs (byte - 128) in record order to a plane, one block per row.
+// With `in_place` (in == out) the row passes through shared memory, so that
+// records are written without scratch memory however full the device is.
+__global__ void i8_plane_kernel(const uint8_t* in, uint32_t K, uint8_t* out, bool in_place) {
+  extern __shared__ uint2 record[];
   const uint32_t per = K / 8;
-  reinterpret_cast<uint2*>(out)[i / per * per + plane_octet((uint32_t)(i % per), K)] =
-      make_uint2(v.x ^ 0x80808080u, v.y ^ 0x80808080u);
+  const uint2* src = reinterpret_cast<const uint2*>(in) + (size_t)blockIdx.x * per;
+  uint2* dst = reinterpret_cast<uint2*>(out) + (size_t)blockIdx.x * per;
+  if (in_place) {
+    for (uint32_t o = threadIdx.x; o < per; o += blockDim.x) record[o] = src[o];
+    __syncthreads();
+    src = record;
+  }
+  for (uint32_t o = threadIdx.x; o < per; o += blockDim.x) {
+    const uint2 v = src[o];
+    dst[plane_octet(o, K)] = make_uint2(v.x ^ 0x80808080u, v.y ^ 0x80808080u);
+  }
 }
+
+constexpr int kI8RowMost = 227 * 1024;  // a row of i8 limbs in shared memory
 
 // Bytewise sums of two u16 vectors given as limb words: (al, ah) + (bl, bh).
 __device__ __forceinline__ void add_limbs(uint32_t al, uint32_t ah, uint32_t bl, uint32_t bh, uint32_t& sl,
@@ -375,11 +387,16 @@ cudaError_t launch_split_limbs(const uint16_t* in, uint32_t K, uint8_t* lo, uint
   return cudaGetLastError();
 }
 
+bool i8_plane_in_place(size_t K) { return K <= kI8RowMost; }
+
 cudaError_t launch_i8_plane(const uint8_t* in, uint32_t K, uint8_t* out, size_t n, cudaStream_t stream) {
-  if (n % 8) return cudaErrorInvalidValue;
-  const size_t n8 = n / 8;
-  if (!n8) return cudaSuccess;
-  i8_plane_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, stream>>>(in, K, out, n8);
+  if (!n) return cudaSuccess;
+  const bool in_place = in == out;
+  if (in_place && !i8_plane_in_place(K)) return cudaErrorInvalidValue;
+  static std::atomic<uint64_t> attr_done{0};
+  const cudaError_t e = smem_limit_once(i8_plane_kernel, kI8RowMost, attr_done);
+  if (e != cudaSuccess) return e;
+  i8_plane_kernel<<<(unsigned)n, 256, in_place ? K : 0, stream>>>(in, K, out, in_place);
   return cudaGetLastError();
 }
 

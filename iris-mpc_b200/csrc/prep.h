@@ -32,6 +32,8 @@ struct SynthOut {
 // n = rows x K coefficients; planes in quarter order (prep.cu)
 cudaError_t launch_split_limbs(const uint16_t* in, uint32_t K, uint8_t* lo, uint8_t* hi, size_t n,
                                cudaStream_t stream);
+// n rows of K i8 limbs to a plane; in == out where i8_plane_in_place(K)
+bool i8_plane_in_place(size_t K);
 cudaError_t launch_i8_plane(const uint8_t* in, uint32_t K, uint8_t* out, size_t n, cudaStream_t stream);
 cudaError_t launch_derive_sums(const uint8_t* lo, const uint8_t* hi, uint32_t K, size_t n, uint8_t* outer_lo,
                                uint8_t* outer_hi, uint8_t* inner_lo, uint8_t* inner_hi, cudaStream_t stream);

@@ -61,3 +61,45 @@ def test_update_and_delete(dm, oracle):
         c.close()
         for e in ce + me:
             e.close()
+
+
+def _limbs(rec):
+    return ((rec & 0xFF).astype(np.uint8) ^ 0x80).view(np.int8), ((rec >> 8).astype(np.uint8) ^ 0x80).view(np.int8)
+
+
+# the shortest code, the longest whose limbs fit a block's shared memory, and one that does not
+@pytest.mark.parametrize("K", [128, 232448, 232576])
+def test_stored_limbs_of_any_length(dm, K):
+    rng = np.random.default_rng(K)
+    e = irisb200.ShareDB(0, dm, 64, 64, K, W.SEEDS[0])
+    e.alloc_db(64)
+    rec = rng.integers(0, 1 << 16, (7, K), dtype=np.uint16)
+    e.load_records_i8(20, *_limbs(rec))
+    assert np.array_equal(e.fetch_records(20, 7), rec)
+    assert not e.fetch_records(19, 1).any() and not e.fetch_records(27, 1).any()
+    e.load_records(40, rec)
+    assert np.array_equal(e.fetch_records(40, 7), rec)
+    e.close()
+
+
+def test_stored_limbs_need_no_free_memory():
+    """Records go into the resident database however full the device is."""
+    K, n = 6400, 8192
+    rng = np.random.default_rng(1)
+    rec = rng.integers(0, 1 << 16, (n, K), dtype=np.uint16)
+    dm = irisb200.DeviceManager(0)
+    e = irisb200.ShareDB(0, dm, 64, 64, K, W.SEEDS[0])
+    e.alloc_db(n)
+    e.load_records_i8(0, *_limbs(rec[:1]))  # the kernels are loaded
+    taken = []
+    for step in (1 << 30, 1 << 25):  # less than 64 MB stay free
+        while dm.mem_info()[0] > 2 * step:
+            taken.append(irisb200.DeviceBuffer(dm, max(step, dm.mem_info()[0] - 2 * step)))
+    try:
+        e.load_records_i8(0, *_limbs(rec))
+        assert np.array_equal(e.fetch_records(0, n), rec)
+    finally:
+        for b in taken:
+            b.free()
+        e.close()
+        dm.close()
