@@ -1005,9 +1005,11 @@ int irs_sharedb_fetch_records(irs_sharedb* db, size_t first, size_t n, uint16_t*
   CU(cudaStreamSynchronize(s));
   // planes are in quarter order (prep.cu): octet o of a row sits in quarter o % 4
   for (size_t r = 0; r < n; r++)
-    for (size_t k = 0; k < K; k++) {
-      const size_t o = k / 8, at = r * K + (o % 4) * (K / 4) + o / 4 * 8 + k % 8;
-      records[r * K + k] = (uint16_t)(lo[at] | (hi[at] << 8));
+    for (size_t q = 0; q < 4; q++) {
+      const uint8_t *l = &lo[r * K + q * (K / 4)], *h = &hi[r * K + q * (K / 4)];
+      uint16_t* out = records + r * K + 8 * q;
+      for (size_t o = 0; o < K / 32; o++, l += 8, h += 8, out += 32)
+        for (int k = 0; k < 8; k++) out[k] = (uint16_t)(l[k] | (h[k] << 8));
     }
   return IRS_OK;
 }
