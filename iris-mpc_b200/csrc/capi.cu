@@ -16,6 +16,7 @@
 #include <new>
 #include <map>
 #include <mutex>
+#include <shared_mutex>
 #include <string>
 #include <vector>
 
@@ -211,73 +212,110 @@ cudaStream_t party_stream(irs_device_manager* dm, int party, void* s) {
   return s ? static_cast<cudaStream_t>(s) : dm->streams[party];
 }
 
-// Engines that hold derived sums, over all device managers of the process.
-// The sums are an extra layout of records that are resident anyway, so they
-// give way when an allocation of the library fails.  The lock covers every
-// read of an engine's sums up to the launch that uses them.
+// Engines of a device that hold derived sums, over all device managers of the
+// process.  The sums are an extra layout of records that are resident anyway, so
+// they give way when an allocation of the library fails.  A launch that may read
+// an engine's sums holds the lock shared from the look at them until it is
+// enqueued, so that launches do not wait for one another; whoever takes sums away
+// holds it alone.  Each device has its own: a thread that waits for a full launch
+// queue, or frees memory, does not hold up those that drive other devices.
 struct SumHolders {
-  std::mutex mu;
+  std::shared_mutex mu;
   std::vector<irs_sharedb*> engines;
 };
-SumHolders& sum_holders() {
-  static SumHolders h;
-  return h;
+using SumReader = std::shared_lock<std::shared_mutex>;
+using SumWriter = std::lock_guard<std::shared_mutex>;
+SumHolders& sum_holders(int device) {
+  static SumHolders h[64];
+  return h[device & 63];
 }
+SumHolders& sum_holders(const irs_sharedb* db) { return sum_holders(db->dm->device); }
 
-// Frees an engine's sums and forms (the holders' lock is held).  cudaFree
-// waits for the launches that read them.
+// Memory of an engine's sums and forms that nothing new can reach.
+struct DroppedSums {
+  uint8_t* sums = nullptr;
+  uint8_t* forms = nullptr;
+};
+
+// Takes an engine's sums and forms away from it (its device's lock is held
+// alone); the caller frees them once it has released the lock: cudaFree waits
+// for the launches that read them.
 // A graph that holds the quad GEMM is told by the flag to run the plain one;
-// replays start under the holders' lock, so that none reads the flag half-way.
-void drop_sums_locked(irs_sharedb* db) {
+// replays start under the lock, so that none reads the flag half-way.
+DroppedSums take_sums(irs_sharedb* db) {
   if (db->quad_flag && db->dot_captured) {
-    cudaDeviceSynchronize();
-    cudaMemset(db->quad_flag, 0, 4);
-    cudaDeviceSynchronize();
+    if (cudaEventSynchronize(db->dm->graph_done) != cudaSuccess) {
+      cudaGetLastError();
+      cudaDeviceSynchronize();
+    }
+    cudaMemsetAsync(db->quad_flag, 0, 4, db->dm->streams[db->peer]);
+    cudaStreamSynchronize(db->dm->streams[db->peer]);
     db->flag_rows = 0;
   }
-  auto& v = sum_holders().engines;
+  auto& v = sum_holders(db).engines;
   v.erase(std::remove(v.begin(), v.end(), db), v.end());
-  if (db->sums) cudaFree(db->sums);
-  if (db->forms) cudaFree(db->forms);
+  const DroppedSums d{db->sums, db->forms};
   db->sums = db->forms = nullptr;
   db->row_valid = nullptr;
   db->quad_rows = false;
   db->stale_end = 0;
   db->forms_pad = 0;
   db->dot_captured = db->sums_pinned = false;
+  return d;
+}
+
+void free_sums(const DroppedSums& d) {
+  if (d.sums) cudaFree(d.sums);
+  if (d.forms) cudaFree(d.forms);
 }
 
 void drop_sums(irs_sharedb* db) {
-  std::lock_guard<std::mutex> lock(sum_holders().mu);
-  drop_sums_locked(db);
+  {
+    SumReader lock(sum_holders(db).mu);
+    if (!db->sums) return;
+  }
+  DroppedSums d;
+  {
+    SumWriter lock(sum_holders(db).mu);
+    d = take_sums(db);
+  }
+  free_sums(d);
 }
 
 size_t sums_bytes(size_t cap, size_t K) { return 2 * cap * (K / 2 + 3 * K / 4); }
 size_t forms_bytes(size_t n_cap, size_t K) { return 2 * (kQuadProducts * (n_cap / 4) * (K / 4)); }
 
+// Whether reclaim_sums may take an engine's sums (the lock is held): not those
+// that a capture other than of this library's own dots uses.
+bool sums_reclaimable(const irs_sharedb* db, int device) {
+  return db->dm->device == device && !db->sums_pinned && !db->dm->capturing;
+}
+
 // Bytes that reclaim_sums would give back on a device.
 size_t reclaimable_sums(int device) {
-  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  SumReader lock(sum_holders(device).mu);
   size_t bytes = 0;
-  for (const irs_sharedb* db : sum_holders().engines)
-    if (db->dm->device == device && !db->sums_pinned && !db->dm->capturing)
+  for (const irs_sharedb* db : sum_holders(device).engines)
+    if (sums_reclaimable(db, device))
       bytes += sums_bytes(db->db_cap, db->code_length) + forms_bytes(db->n_cap, db->code_length);
   return bytes;
 }
 
-// Gives back the sums of every engine on `device`, except those that a capture
-// other than of this library's own dots uses; whether there were any.
+// Gives back the sums of every engine on `device` that may lose them; whether
+// there were any.
 bool reclaim_sums(int device) {
-  std::lock_guard<std::mutex> lock(sum_holders().mu);
-  const auto& held = sum_holders().engines;
   bool any = false;
-  for (size_t i = held.size(); i-- > 0;) {  // dropping one removes it from the list
-    irs_sharedb* db = held[i];
-    if (db->dm->device != device || db->sums_pinned || db->dm->capturing) continue;
-    drop_sums_locked(db);
-    any = true;
+  for (DroppedSums d;; any = true) {
+    {
+      SumWriter lock(sum_holders(device).mu);
+      const auto& held = sum_holders(device).engines;
+      const auto it = std::find_if(held.rbegin(), held.rend(),
+                                   [&](const irs_sharedb* db) { return sums_reclaimable(db, device); });
+      if (it == held.rend()) return any;
+      d = take_sums(*it);
+    }
+    free_sums(d);
   }
-  return any;
 }
 
 // cudaMalloc that gives the derived sums back before it fails.
@@ -432,8 +470,8 @@ void alloc_sums(irs_sharedb* db) {
   }
   bool held = true;
   try {
-    std::lock_guard<std::mutex> lock(sum_holders().mu);
-    sum_holders().engines.push_back(db);
+    SumWriter lock(sum_holders(db).mu);
+    sum_holders(db).engines.push_back(db);
   } catch (const std::bad_alloc&) {
     held = false;
   }
@@ -458,7 +496,7 @@ bool gather_skips_sums(const irs_sharedb* db, size_t n, cudaStream_t s) {
 // Brings the sums of records [first, first + n) in line with the planes, on
 // the stream that wrote them.
 cudaError_t update_sums(irs_sharedb* db, size_t first, size_t n, cudaStream_t s) {
-  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  SumReader lock(sum_holders(db).mu);
   if (!db->sums || !n) return cudaSuccess;
   if (stream_captures(s)) db->sums_pinned = true;
   const size_t K = db->code_length, cap = db->db_cap, o = K / 2, i = 3 * K / 4;
@@ -507,7 +545,7 @@ bool rows_are_quads(const uint32_t* desc, size_t n_rows) {
 uint8_t* forms_hi(irs_sharedb* db) { return db->forms + kQuadProducts * (db->n_pad / 4) * (db->code_length / 4); }
 
 // Notes whether the rows about to be expanded are quads, and where the
-// expansion puts their forms and (if it changes) the device flag.  The holders'
+// expansion puts their forms and (if it changes) the device flag.  The sums'
 // lock is held until the expansion is enqueued.  An upload that is captured
 // (on `s`) writes planes alone, and so do the engine's later ones: what the
 // rows are after a replay is not known here.
@@ -527,7 +565,7 @@ QuadForms begin_forms(irs_sharedb* db, bool quads, cudaStream_t s) {
 
 // Planes and forms of a row table whose bases and table are in the staging.
 int expand_row_table(irs_sharedb* db, const uint32_t* desc, size_t n_rows, const uint32_t* d_desc, cudaStream_t s) {
-  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  SumReader lock(sum_holders(db).mu);
   const QuadForms f = begin_forms(db, quad_forms_ready(db) && rows_are_quads(desc, n_rows), s);
   CU(launch_expand_rows(db->q_stage, (uint32_t)db->code_length, d_desc, (uint32_t)n_rows, (uint32_t)db->n_pad, db->q_lo,
                         db->q_hi, f, s));
@@ -1107,7 +1145,7 @@ int irs_sharedb_query_upload(irs_sharedb* db, const uint16_t* rows, size_t n_row
   if (n_rows) CU(cudaMemcpyAsync(db->q_stage, rows, n_rows * K * 2, cudaMemcpyHostToDevice, s));
   CU(launch_split_limbs(db->q_stage, (uint32_t)K, db->q_lo, db->q_hi, db->n_pad * K, s));
   {
-    std::lock_guard<std::mutex> lock(sum_holders().mu);
+    SumReader lock(sum_holders(db).mu);
     if (begin_forms(db, false, s).flag) CU(cudaMemsetAsync(db->quad_flag, 0, 4, s));  // rows of no known structure
   }
   db->have_query = true;
@@ -1138,7 +1176,7 @@ int irs_sharedb_query_upload_slots(irs_sharedb* db, const uint16_t* base, size_t
   CU(cudaMemcpyAsync(db->d_slots, slots, n_slots * sizeof(QuerySlot), cudaMemcpyHostToDevice, s));
   CU(cudaEventRecord(db->copied, s));
   {
-    std::lock_guard<std::mutex> lock(sum_holders().mu);
+    SumReader lock(sum_holders(db).mu);
     const QuadForms f = begin_forms(db, quad_forms_ready(db), s);  // a slot's rows are consecutive rotations
     CU(launch_expand_slots(db->q_stage, (uint32_t)K, db->d_slots, (uint32_t)n_slots, (uint32_t)db->n_pad, db->q_lo,
                            db->q_hi, f, s));
@@ -1263,14 +1301,14 @@ int irs_sharedb_set_pair(irs_sharedb* db, int on) {
 
 int irs_sharedb_has_sums(irs_sharedb* db, int* on) {
   CHECK(db && on, IRS_ERR_INVALID, "bad arguments");
-  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  SumReader lock(sum_holders(db).mu);
   *on = db->sums != nullptr;
   return IRS_OK;
 }
 
 int irs_sharedb_last_gemm(irs_sharedb* db, int* gemm, size_t* quad_rows) {
   CHECK(db && gemm && quad_rows, IRS_ERR_INVALID, "bad arguments");
-  std::lock_guard<std::mutex> lock(sum_holders().mu);
+  SumReader lock(sum_holders(db).mu);
   *gemm = db->last_gemm;
   *quad_rows = db->sums ? db->flag_rows : 0;
   return IRS_OK;
@@ -1433,7 +1471,7 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
       dm->stall_limit_ns = 0;
     }
     StageTimer timer(dm, s, "dot");
-    std::lock_guard<std::mutex> lock(sum_holders().mu);
+    SumReader lock(sum_holders(dm->device).mu);
     const bool captured = stream_captures(s);
     const int width = stall ? -1 : quad_width(engines, n, offset, len, pair);
     bool quads = width >= 0;
@@ -2165,10 +2203,13 @@ int irs_graph_launch(irs_graph* g, void* stream) {
       if (!stream_captures(g->dm->streams[p])) CU(cudaEventRecord(g->dm->uploads[p], g->dm->streams[p]));
       CU(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), g->dm->uploads[p], 0));
     }
+  if (captured) {  // replays start outside the lock
+    SumWriter lock(sum_holders(g->dm->device).mu);
+    for (irs_sharedb* db : sum_holders(g->dm->device).engines)
+      if (db->dm == g->dm && db->dot_captured) db->sums_pinned = true;
+  }
   {
-    std::lock_guard<std::mutex> lock(sum_holders().mu);
-    for (irs_sharedb* db : sum_holders().engines)
-      if (captured && db->dm == g->dm && db->dot_captured) db->sums_pinned = true;  // replays outside this lock
+    SumReader lock(sum_holders(g->dm->device).mu);
     CU(cudaGraphLaunch(g->exec, static_cast<cudaStream_t>(stream)));
   }
   // Later query uploads on other party streams wait for the graph's GEMMs, and
