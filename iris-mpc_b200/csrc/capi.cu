@@ -222,6 +222,7 @@ cudaStream_t party_stream(irs_device_manager* dm, int party, void* s) {
 struct SumHolders {
   std::shared_mutex mu;
   std::vector<irs_sharedb*> engines;
+  std::vector<irs_device_manager*> managers;  // all of the device
 };
 using SumReader = std::shared_lock<std::shared_mutex>;
 using SumWriter = std::lock_guard<std::shared_mutex>;
@@ -301,41 +302,62 @@ size_t reclaimable_sums(int device) {
   return bytes;
 }
 
-// Gives back the sums of every engine on `device` that may lose them; whether
-// there were any.
+// Gives back the sums of one engine on `device` that may lose them, the last
+// to have got them; whether there was one.
 bool reclaim_sums(int device) {
-  bool any = false;
-  for (DroppedSums d;; any = true) {
-    {
-      SumWriter lock(sum_holders(device).mu);
-      const auto& held = sum_holders(device).engines;
-      const auto it = std::find_if(held.rbegin(), held.rend(),
-                                   [&](const irs_sharedb* db) { return sums_reclaimable(db, device); });
-      if (it == held.rend()) return any;
-      d = take_sums(*it);
-    }
-    free_sums(d);
+  DroppedSums d;
+  {
+    SumWriter lock(sum_holders(device).mu);
+    const auto& held = sum_holders(device).engines;
+    const auto it = std::find_if(held.rbegin(), held.rend(),
+                                 [&](const irs_sharedb* db) { return sums_reclaimable(db, device); });
+    if (it == held.rend()) return false;
+    d = take_sums(*it);
   }
+  free_sums(d);
+  return true;
 }
 
-// cudaMalloc that gives the derived sums back before it fails.
-cudaError_t device_malloc(irs_device_manager* dm, void** p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation) {
+// Whether `bytes` can be had on a device once all sums are given back: with
+// what is free and what the managers' pools hold unused.
+bool fits_without_sums(int device, size_t bytes) {
+  size_t room = reclaimable_sums(device), free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) room += free_b;
+  SumReader lock(sum_holders(device).mu);
+  for (const irs_device_manager* dm : sum_holders(device).managers)
+    for (cudaMemPool_t pool : dm->pools) {
+      uint64_t reserved = 0, used = 0;
+      if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+          cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+        room += reserved - used;
+    }
+  cudaGetLastError();
+  return bytes <= room;
+}
+
+// An allocation (`take`) that gives derived sums back, an engine's at a time,
+// before it fails; none where that cannot help.
+template <class Take>
+cudaError_t alloc_or_reclaim(irs_device_manager* dm, size_t bytes, Take take) {
+  cudaError_t e = take();
+  for (bool asked = false; e == cudaErrorMemoryAllocation && !dm->capturing; e = take()) {
     cudaGetLastError();
-    if (!dm->capturing && reclaim_sums(dm->device)) e = cudaMalloc(p, bytes);
+    if (!asked && !fits_without_sums(dm->device, bytes)) return e;
+    asked = true;
+    if (!reclaim_sums(dm->device)) return e;
   }
   return e;
+}
+
+cudaError_t device_malloc(irs_device_manager* dm, void** p, size_t bytes) {
+  return alloc_or_reclaim(dm, bytes, [&] { return cudaMalloc(p, bytes); });
 }
 
 int pool_alloc(irs_device_manager* dm, int party, size_t bytes, void** out) {
   *out = nullptr;
   if (!bytes) return IRS_OK;
-  cudaError_t e = cudaMallocFromPoolAsync(out, bytes, dm->pools[party], dm->streams[party]);
-  if (e == cudaErrorMemoryAllocation && !dm->capturing) {
-    cudaGetLastError();
-    if (reclaim_sums(dm->device)) e = cudaMallocFromPoolAsync(out, bytes, dm->pools[party], dm->streams[party]);
-  }
+  cudaError_t e = alloc_or_reclaim(
+      dm, bytes, [&] { return cudaMallocFromPoolAsync(out, bytes, dm->pools[party], dm->streams[party]); });
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(IRS_ERR_NOMEM, "device allocation of %zu bytes for party %d failed: %s", bytes, party,
@@ -355,11 +377,8 @@ void pool_free(irs_device_manager* dm, int party, void* p) {
 int scratch_alloc(irs_device_manager* dm, cudaStream_t s, size_t bytes, void** out) {
   *out = nullptr;
   if (!bytes) return IRS_OK;
-  cudaError_t e = cudaMallocFromPoolAsync(out, bytes, dm->pools[0], s);
-  if (e == cudaErrorMemoryAllocation && !dm->capturing) {
-    cudaGetLastError();
-    if (reclaim_sums(dm->device)) e = cudaMallocFromPoolAsync(out, bytes, dm->pools[0], s);
-  }
+  const cudaError_t e =
+      alloc_or_reclaim(dm, bytes, [&] { return cudaMallocFromPoolAsync(out, bytes, dm->pools[0], s); });
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(IRS_ERR_NOMEM, "device scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
@@ -629,6 +648,13 @@ int irs_device_manager_init(int device, irs_device_manager** out) {
   CU(cudaEventCreateWithFlags(&dm->graph_ran, cudaEventDisableTiming));
   CU(cudaStreamCreateWithFlags(&dm->graph_join, cudaStreamNonBlocking));
   for (cudaEvent_t& e : dm->uploads) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  try {
+    SumWriter lock(sum_holders(device).mu);
+    sum_holders(device).managers.push_back(dm);
+  } catch (const std::bad_alloc&) {
+    irs_device_manager_destroy(dm);
+    return fail(IRS_ERR_NOMEM, "host allocation failed");
+  }
   *out = dm;
   return IRS_OK;
 }
@@ -636,6 +662,11 @@ int irs_device_manager_init(int device, irs_device_manager** out) {
 int irs_device_manager_destroy(irs_device_manager* dm) {
   if (!dm) return IRS_OK;
   cudaSetDevice(dm->device);
+  {
+    SumWriter lock(sum_holders(dm->device).mu);
+    auto& v = sum_holders(dm->device).managers;
+    v.erase(std::remove(v.begin(), v.end(), dm), v.end());
+  }
   for (int p = 0; p < 3; p++) if (dm->streams[p]) cudaStreamSynchronize(dm->streams[p]);
   cudaFree(dm->d_err);
   cudaFree(dm->d_batch);

@@ -75,3 +75,31 @@ def test_launches_beside_a_thread_that_takes_sums():
         dm.close()
     assert not failed and not any(t.is_alive() for t in threads)
     assert "quad" in ran
+
+
+def test_sums_give_way_one_engine_at_a_time():
+    """An allocation takes no more sums than it needs, and none where all of
+    them would not do."""
+    dm = irisb200.DeviceManager(0)
+    engines = [irisb200.ShareDB(0, dm, 64, 640, 6400, W.SEEDS[0]) for _ in range(3)]
+    for e in engines:
+        e.alloc_db(40000)  # 640 MB of sums each
+    total = dm.mem_info()[1]
+    with pytest.raises(irisb200.IrisError):
+        irisb200.DeviceBuffer(dm, total)
+    assert all(e.has_sums() for e in engines)
+    taken = []
+    while all(e.has_sums() for e in engines):
+        taken.append(irisb200.DeviceBuffer(dm, max(1 << 28, dm.mem_info()[0] - (6 << 30))))
+    assert sorted(e.has_sums() for e in engines) == [False, True, True]
+    with pytest.raises(irisb200.IrisError):
+        irisb200.DeviceBuffer(dm, total // 2)
+    assert sorted(e.has_sums() for e in engines) == [False, True, True]
+    while sum(e.has_sums() for e in engines) == 2:
+        taken.append(irisb200.DeviceBuffer(dm, 1 << 28))
+    assert sorted(e.has_sums() for e in engines) == [False, False, True]
+    for b in taken:
+        b.free()
+    for e in engines:
+        e.close()
+    dm.close()
