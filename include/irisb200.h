@@ -129,10 +129,15 @@ int irs_event_synchronize(void* ev);
 int irs_event_query(void* ev, int* done);
 int irs_event_destroy(void* ev);
 /* Free and total device memory (cudaMemGetInfo), for admission by free HBM
- * (no counterpart: the reference sizes its batches statically).  The derived
- * layouts that the library gives back when an allocation of its own fails
- * count as free. */
+ * (no counterpart: the reference sizes its batches statically). */
 int irs_device_manager_mem_info(irs_device_manager* dm, size_t* free_bytes, size_t* total_bytes);
+/* Memory of the layouts that the library derives from resident records (the
+ * sums of irs_sharedb_alloc_db), over all engines of the device.  The library
+ * gives it back, an engine's at a time, when an allocation of its own would
+ * fail; to any other allocator it is not free.  give_back != 0 frees it now
+ * (*bytes: what is left): the engines then run without it until their records
+ * are allocated anew. */
+int irs_device_manager_derived(irs_device_manager* dm, int give_back, size_t* bytes);
 
 /* Plain device memory helpers for callers that stage their own buffers. */
 int irs_device_alloc(irs_device_manager* dm, size_t bytes, void** ptr);
@@ -159,7 +164,12 @@ int irs_sharedb_init(irs_device_manager* dm, int peer_id, size_t max_db_length, 
                      size_t code_length, const uint32_t seed0[8], const uint32_t seed1[8], int is_remote,
                      irs_sharedb** out);
 int irs_sharedb_destroy(irs_sharedb* db);
-/* ShareDB::alloc_db (share_db.rs:575-618); the DB lives in HBM. */
+/* ShareDB::alloc_db (share_db.rs:575-618); the DB lives in HBM.  An engine of
+ * at least 576 query rows, 1,024 records and a code_length in whole 800s also
+ * allocates 1.25 times the records' memory for their derived sums, which the
+ * rotation-structured GEMM reads, if a twelfth of the device's memory stays
+ * free beside them: see irs_device_manager_derived.  It is never an error that
+ * there is no room for them, and every write to the records keeps them up. */
 int irs_sharedb_alloc_db(irs_sharedb* db, size_t max_db_length);
 /* ShareDB::load_single_record_from_db for records first..first+n-1
  * (share_db.rs:620-655): u16 share coefficients [n][code_length]. */

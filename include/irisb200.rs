@@ -58,6 +58,7 @@ extern "C" {
     pub fn irs_event_destroy(ev: *mut c_void) -> c_int;
     pub fn irs_device_manager_mem_info(dm: *mut IrsDeviceManager, free_bytes: *mut usize,
         total_bytes: *mut usize) -> c_int;
+    pub fn irs_device_manager_derived(dm: *mut IrsDeviceManager, give_back: c_int, bytes: *mut usize) -> c_int;
     pub fn irs_device_alloc(dm: *mut IrsDeviceManager, bytes: usize, ptr: *mut *mut c_void) -> c_int;
     pub fn irs_host_alloc_pinned(bytes: usize, ptr: *mut *mut c_void) -> c_int;
     pub fn irs_host_free_pinned(ptr: *mut c_void) -> c_int;

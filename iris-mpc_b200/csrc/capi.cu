@@ -843,7 +843,14 @@ int irs_device_manager_mem_info(irs_device_manager* dm, size_t* free_bytes, size
   CHECK(dm && free_bytes && total_bytes, IRS_ERR_INVALID, "bad arguments");
   CU(cudaSetDevice(dm->device));
   CU(cudaMemGetInfo(free_bytes, total_bytes));
-  *free_bytes += reclaimable_sums(dm->device);
+  return IRS_OK;
+}
+
+int irs_device_manager_derived(irs_device_manager* dm, int give_back, size_t* bytes) {
+  CHECK(dm && bytes, IRS_ERR_INVALID, "bad arguments");
+  CU(cudaSetDevice(dm->device));
+  while (give_back && reclaim_sums(dm->device)) {}
+  *bytes = reclaimable_sums(dm->device);
   return IRS_OK;
 }
 

@@ -77,6 +77,7 @@ _SIGS = {
     "irs_device_manager_test_stall_next_dot": [_vp, _u64],
     "irs_device_manager_sm_count": [_vp, C.POINTER(_i)],
     "irs_device_manager_mem_info": [_vp, C.POINTER(_sz), C.POINTER(_sz)],
+    "irs_device_manager_derived": [_vp, _i, C.POINTER(_sz)],
     "irs_device_manager_set_host_sync": [_vp, _i],
     "irs_event_create": [C.POINTER(_vp)],
     "irs_event_record": [_vp, _vp],
@@ -471,6 +472,14 @@ class DeviceManager:
         f, t = _sz(), _sz()
         _check(lib().irs_device_manager_mem_info(self.h, C.byref(f), C.byref(t)))
         return f.value, t.value
+
+    def derived_bytes(self, give_back: bool = False) -> int:
+        """Memory of the engines' derived layouts, which the library's own
+        allocations can have and others cannot; give_back frees it
+        (irs_device_manager_derived)."""
+        n = _sz()
+        _check(lib().irs_device_manager_derived(self.h, int(give_back), C.byref(n)))
+        return n.value
 
     def sm_count(self) -> int:
         c = C.c_int()

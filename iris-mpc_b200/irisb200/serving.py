@@ -47,7 +47,7 @@ def plan_row_capacity(dm, chunk: int, reserve_bytes: int = 8 << 30, cap: int = 8
     """Query rows the server can keep in flight, from the free HBM: each row
     costs a u16 result per chunk entry for the six engines plus its limb
     planes and staging (admission by free HBM)."""
-    free, _ = dm.mem_info()
+    free = dm.mem_info()[0] + dm.derived_bytes()  # the library's allocations can have both
     per_row = chunk * RESULT_BYTES_PER_ROW_ENTRY + 6 * 4 * IRIS_CODE_LENGTH
     rows = max(64, (max(free - reserve_bytes, 0) // per_row) // 64 * 64)
     return int(min(rows, cap))

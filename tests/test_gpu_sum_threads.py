@@ -103,3 +103,20 @@ def test_sums_give_way_one_engine_at_a_time():
     for e in engines:
         e.close()
     dm.close()
+
+
+def test_free_memory_is_what_any_allocator_can_have():
+    """mem_info is the device's free memory; the sums count apart, and are given
+    back on demand."""
+    import torch
+    dm = irisb200.DeviceManager(0)
+    e = irisb200.ShareDB(0, dm, 64, 640, 6400, W.SEEDS[0])
+    e.alloc_db(40000)
+    sums = 2 * -(-40000 // 128) * 128 * 8000
+    assert e.has_sums() and dm.mem_info() == torch.cuda.mem_get_info(0)
+    before, held = dm.mem_info()[0], dm.derived_bytes()
+    assert sums <= held < sums * 1.1
+    assert dm.derived_bytes(give_back=True) == 0 and not e.has_sums()
+    assert dm.mem_info()[0] >= before + sums
+    e.close()
+    dm.close()
