@@ -288,6 +288,12 @@ int irs_sharedb_set_pair(irs_sharedb* db, int on);
  * rotation-structured GEMM needs (see alloc_db), for callers that place query
  * rows themselves (no counterpart in the reference). */
 int irs_sharedb_has_sums(irs_sharedb* db, int* on);
+/* *on = 1 if a dot over `len` entries of the n engines, with `rows` uploaded
+ * rows that are quads (rows i, i + 2, i + 4, i + 6 of each octet hold rotations
+ * of one base, that far apart, or nothing), runs the rotation-structured GEMM;
+ * `pair` as in irs_sharedb_set_pair, the tile width left to the library.  For
+ * callers that weigh such a placement of rows against a denser one. */
+int irs_sharedb_runs_quads(irs_sharedb* const* engines, int n, size_t rows, size_t len, int pair, int* on);
 /* The GEMM that the engine's last dot launched (no counterpart in the
  * reference): IRS_GEMM_ONE_SM, IRS_GEMM_PAIR (on SM pairs), IRS_GEMM_QUAD (the
  * rotation-structured one), or IRS_GEMM_CAPTURED for a captured dot that holds

@@ -101,6 +101,8 @@ extern "C" {
     pub fn irs_sharedb_set_tile(db: *mut IrsShareDb, block_n: c_int) -> c_int;
     pub fn irs_sharedb_set_pair(db: *mut IrsShareDb, on: c_int) -> c_int;
     pub fn irs_sharedb_has_sums(db: *mut IrsShareDb, on: *mut c_int) -> c_int;
+    pub fn irs_sharedb_runs_quads(engines: *const *mut IrsShareDb, n: c_int, rows: usize, len: usize, pair: c_int,
+        on: *mut c_int) -> c_int;
     pub fn irs_sharedb_last_gemm(db: *mut IrsShareDb, gemm: *mut c_int, quad_rows: *mut usize) -> c_int;
     pub fn irs_sharedb_use_batch_counter(db: *mut IrsShareDb, on: c_int) -> c_int;
     pub fn irs_sharedb_set_batch(db: *mut IrsShareDb, batch_id: u64) -> c_int;

@@ -1408,9 +1408,7 @@ static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t 
 }
 
 // Tiles of 128 entries x 128 query rows of a launch.
-static size_t tiles_128(irs_sharedb* const* engines, int n, size_t len) {
-  return (size_t)n * ((len + 127) / 128) * ((engines[0]->n_pad + 127) / 128);
-}
+static size_t tiles_128(int n, size_t len, size_t n_pad) { return (size_t)n * ((len + 127) / 128) * ((n_pad + 127) / 128); }
 
 // Whether the plain GEMM of a launch runs on SM pairs.  Six engines x 32,768
 // entries, one-SM against pair: 128 rows 0.86 / 0.87 ms (over 131,072 entries
@@ -1422,28 +1420,38 @@ static size_t tiles_128(irs_sharedb* const* engines, int n, size_t len) {
 // ms); above, where the caller chose it or the launch is short enough that the
 // clock has not dropped to the power limit (one engine x 32,768 entries, 960
 // rows 0.94 / 0.89, 1984 rows 1.60 / 1.51).
+static bool plain_pair_for(irs_sharedb* const* engines, int n, size_t len, size_t n_pad, bool pair) {
+  if (!gemm_pair_applies(true, (uint32_t)n_pad)) return false;
+  if (n_pad <= 768) return tiles_128(n, len, n_pad) > (size_t)engines[0]->dm->n_sms;
+  if (pair) return true;
+  double macs = 0;
+  for (int i = 0; i < n; i++) macs += 3.0 * (double)engines[i]->code_length * (double)n_pad * (double)len;
+  return macs < 3e12;  // about 2 ms
+}
+
 static bool plain_pair(irs_sharedb* const* engines, int n, size_t len) {
   const irs_sharedb* e = engines[0];
-  if (!gemm_pair_applies(true, (uint32_t)e->n_pad) || (e->tile_override && !e->pair)) return false;
+  if (e->tile_override && !e->pair) return false;
   for (int i = 1; i < n; i++)
     if (engines[i]->n_pad != e->n_pad) return false;  // one tile width for the launch
-  if (e->n_pad <= 768)
-    return tiles_128(engines, n, len) > (size_t)e->dm->n_sms;
-  if (e->pair) return true;
-  double macs = 0;
-  for (int i = 0; i < n; i++) macs += 3.0 * (double)engines[i]->code_length * (double)e->n_pad * (double)len;
-  return macs < 3e12;  // about 2 ms
+  return plain_pair_for(engines, n, len, e->n_pad, e->pair);
 }
 
 // Whether a launch of 256-row tiles with the GEMM left open has so few tiles
 // that it runs 128-row ones with their K loop shared (gemm_k_split): 64 entries
 // x 2048 rows, six engines, 81 us against 112.
+static bool few_tiles_for(irs_sharedb* const* engines, int n, size_t len, size_t n_pad) {
+  for (int i = 0; i < n; i++)
+    if (engines[i]->code_length < 8 * 128) return false;
+  return 3 * tiles_128(n, len, n_pad) <= 2 * (size_t)engines[0]->dm->n_sms;
+}
+
 static bool few_tiles(irs_sharedb* const* engines, int n, size_t len) {
   const irs_sharedb* e = engines[0];
   if (e->pair || e->tile_override || e->block_n != 256) return false;
   for (int i = 0; i < n; i++)
-    if (engines[i]->n_pad != e->n_pad || engines[i]->code_length < 8 * 128) return false;
-  return 3 * tiles_128(engines, n, len) <= 2 * (size_t)e->dm->n_sms;
+    if (engines[i]->n_pad != e->n_pad) return false;
+  return few_tiles_for(engines, n, len, e->n_pad);
 }
 
 static void fill_quad_problem(const irs_sharedb* db, const GemmProblem& g, int width, QuadProblem& pr) {
@@ -1468,6 +1476,27 @@ static void fill_quad_problem(const irs_sharedb* db, const GemmProblem& g, int w
   pr.nonce = g.nonce;
   pr.batch = g.batch;
   pr.batch_dev = g.batch_dev;
+}
+
+int irs_sharedb_runs_quads(irs_sharedb* const* engines, int n, size_t rows, size_t len, int pair, int* on) {
+  CHECK(engines && on && n > 0 && n <= kMaxGemmProblems, IRS_ERR_INVALID, "1..6 engines per launch");
+  *on = 0;
+  uint32_t K[kMaxGemmProblems];
+  for (int i = 0; i < n; i++) {
+    CHECK(engines[i] && engines[i]->dm == engines[0]->dm, IRS_ERR_INVALID, "engine %d missing or on another device", i);
+    K[i] = (uint32_t)engines[i]->code_length;
+  }
+  const size_t n_pad = padded_query_rows(rows, engines[0]->n_cap);
+  SumReader lock(sum_holders(engines[0]).mu);
+  for (int i = 0; i < n; i++)
+    if (!engines[i]->sums || padded_query_rows(rows, engines[i]->n_cap) != n_pad || n_pad > engines[i]->n_cap)
+      return IRS_OK;
+  if (n_pad < kQuadMinRows || !len) return IRS_OK;
+  const int bn = gemm_block_n_for((uint32_t)n_pad);
+  const bool few = !pair && bn == 256 && few_tiles_for(engines, n, len, n_pad);
+  const bool on_pairs = !few && plain_pair_for(engines, n, len, n_pad, pair != 0);
+  *on = quad_width_for(K, n, (uint32_t)len, (uint32_t)n_pad, bn, on_pairs, engines[0]->dm->n_sms) >= 0;
+  return IRS_OK;
 }
 
 int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multipliers, int n, size_t offset, size_t len,

@@ -115,6 +115,7 @@ _SIGS = {
     "irs_sharedb_set_tile": [_vp, _i],
     "irs_sharedb_set_pair": [_vp, _i],
     "irs_sharedb_has_sums": [_vp, C.POINTER(_i)],
+    "irs_sharedb_runs_quads": [_vp, _i, _sz, _sz, _i, C.POINTER(_i)],
     "irs_sharedb_last_gemm": [_vp, C.POINTER(_i), C.POINTER(_sz)],
     "irs_sharedb_use_batch_counter": [_vp, _i],
     "irs_circuits_use_batch_counter": [_vp, _i],
@@ -555,6 +556,15 @@ class ShareDB:
         """Whether the engine holds what the quad GEMM needs (irs_sharedb_has_sums)."""
         on = _i()
         _check(lib().irs_sharedb_has_sums(self.h, C.byref(on)))
+        return bool(on.value)
+
+    @staticmethod
+    def runs_quads(engines, n_rows: int, length: int, pair: bool) -> bool:
+        """Whether a dot of the engines over `length` entries runs the quad GEMM
+        on n_rows rows that are quads (irs_sharedb_runs_quads)."""
+        hs = (_vp * len(engines))(*[e.h for e in engines])
+        on = _i()
+        _check(lib().irs_sharedb_runs_quads(C.cast(hs, _vp), len(engines), n_rows, length, int(pair), C.byref(on)))
         return bool(on.value)
 
     def last_gemm(self):

@@ -146,7 +146,7 @@ def first_quads(occupied: int, n: int) -> int:
     """Lowest quad of a word (8 of them: rows i, i + 2, i + 4, i + 6 of each
     octet of rows) where a run of n rows has its quads to itself, or -1.  A run
     starts at an octet (an even quad), a single row takes any one quad."""
-    need = (1 << (n // 8 * 2 + min(n % 8, 2))) - 1
+    need = (1 << quads_of(n)) - 1
     for q in range(0, 8, 1 if n == 1 else 2):
         if need << q < 1 << 8 and not occupied & need << q:
             return q
@@ -174,18 +174,41 @@ def pack_quads(variant_rows: list) -> Layout:
             fill.append(0)
         start = s
         slots[s].append((v, q // 2 * 8 + q % 2, n))
-        fill[s] |= (1 << (n // 8 * 2 + min(n % 8, 2))) - 1 << q
+        fill[s] |= (1 << quads_of(n)) - 1 << q
     return _layout_of(slots, variant_rows)
 
 
-def pack_for(variant_rows: list, cap: int) -> Layout:
-    """pack_quads where its rows fit the capacity and the quad GEMM then takes
-    less than the plain one over pack()'s rows (0.75 of the time per padded row:
-    six engines x 32,768 entries, 1024 rows 2.8 against 3.7 ms, 640 rows 2.2
-    against 2.6), else pack."""
-    quads = sum(len(r) // 8 * 2 + min(len(r) % 8, 2) for r in variant_rows)
-    rows, before = padded_rows(-(-quads // 8) * 32, cap), padded_rows(sum(len(r) for r in variant_rows), cap)
-    if QUAD_MIN_ROWS <= rows <= cap and rows * 0.75 < before:
+# One pass (GEMM and threshold) of six engines over 32,768 entries by padded
+# query rows, in ms, the mean of launches of 32,768 and 65,536 entries: quads of
+# rotations on the quad GEMM, any rows on the two-SM one.
+_QUAD_MS = ((576, 640, 768, 1024, 1280, 1536, 1792, 2048), (2.5, 2.55, 2.85, 3.47, 4.65, 5.13, 5.92, 6.55))
+_PLAIN_MS = ((128, 256, 384, 512, 640, 768, 1024, 1280, 1536, 1792, 2048),
+             (0.82, 1.43, 1.87, 2.37, 3.2, 3.6, 4.7, 5.95, 7.24, 8.4, 9.7))
+
+
+def _pass_ms(n_rows: int, cap: int, table) -> float:
+    rows = padded_rows(n_rows, cap)
+    return float(np.interp(rows, *table)) * max(1.0, rows / table[0][-1])
+
+
+def quads_of(n: int) -> int:
+    """Quads that a run of n rows takes (first_quads)."""
+    return n // 8 * 2 + min(n % 8, 2)
+
+
+def quads_pay(rows: int, quads: int, cap: int) -> bool:
+    """Whether `quads` quads kept apart on the quad GEMM take less than their
+    `rows` live rows packed densely on the two-SM one."""
+    n = -(-quads // 8) * 32
+    return QUAD_MIN_ROWS <= padded_rows(n, cap) <= cap and _pass_ms(n, cap, _QUAD_MS) < _pass_ms(rows, cap, _PLAIN_MS)
+
+
+def pack_for(variant_rows: list, cap: int, runs_quads=None) -> Layout:
+    """pack_quads where its rows fit the capacity, the quad GEMM then runs
+    (runs_quads(rows), where the caller can tell) and the pass takes less than
+    over pack()'s rows (quads_pay); else pack."""
+    quads, rows = sum(quads_of(len(r)) for r in variant_rows), sum(len(r) for r in variant_rows)
+    if quads_pay(rows, quads, cap) and (runs_quads is None or runs_quads(padded_rows(-(-quads // 8) * 32, cap))):
         layout = pack_quads(variant_rows)
         if layout.n_rows <= cap:
             return layout
@@ -312,6 +335,30 @@ class BatchedEngine:
             out += [("fused", 128, ch) for ch in chunks[:3]]
         return out
 
+    def _pass_candidates(self, n_rows: int):
+        """The candidates that _tune chooses from: _candidates on the fixed path,
+        where it can run the rows (the two-SM GEMM: from 128 on)."""
+        cands = self._candidates(n_rows, self.db_len)
+        if self.fixed is None:
+            return cands
+        fixed = [c for c in cands if c[0] == self.fixed]
+        if self.fixed == "pair" and not fixed and n_rows >= 128:
+            fixed = [("pair", 256, ch) for ch in sorted({c[2] for c in cands}, reverse=True)]
+        return fixed or cands
+
+    def _quads_run(self, n_rows: int) -> bool:
+        """Whether a pass over n_rows padded rows that are quads runs the quad
+        GEMM: on the candidate chosen for that many rows, or (to be tuned) on the
+        two-SM path."""
+        cand = self.tuned.get((n_rows + 63) // 64 * 64)
+        if cand is None:
+            tunes = self.autotune and self.fixed in (None, "pair")
+            cand = ("pair", 256, 32768) if tunes else self._pass_candidates(n_rows)[0]
+        path, tile, chunk = cand
+        if path == "fused" or (path == "split" and tile):
+            return False
+        return bool(self.ce[0].runs_quads(self.ce + self.me, n_rows, min(chunk, self.db_len), path == "pair"))
+
     def _run_db_pass(self, layout: Layout, cand) -> None:
         path, tile, chunk = cand
         key = (layout.n_slots, path, tile, chunk, self.db_len)
@@ -334,14 +381,12 @@ class BatchedEngine:
         n_pad = (layout.n_rows + 63) // 64 * 64
         if n_pad in self.tuned:
             return self.tuned[n_pad]
-        cands = self._candidates(layout.n_rows, self.db_len)
-        if self.fixed is not None:
-            cands = [c for c in cands if c[0] == self.fixed] or cands
+        cands = self._pass_candidates(layout.n_rows)
         if not self.autotune or len(cands) == 1:
             self.tuned[n_pad] = cands[0]
             return cands[0]
         self.scan.set_rows(layout.n_rows, True)
-        only = self.fixed if any(c[0] == self.fixed for c in cands) else None
+        only = self.fixed if any(c[0] == self.fixed for c in self._candidates(layout.n_rows, self.db_len)) else None
         best = self.scan.tune(only_path=only)
         self.tune_log[n_pad] = list(self.scan.tune_log)
         self.tuned[n_pad] = best
@@ -407,7 +452,7 @@ class BatchedEngine:
         buffers; returns (layout, bases, rows used, segments used)."""
         nb, base_of, mirrored = self._fill_bases(requests, variants, code, mask)
         rows_of = [list(centred_rotations(requests[i].n_rot)) for i, _ in variants]
-        layout = attach_bases(pack_for(rows_of, cap) if pad else pack(rows_of), base_of, mirrored)
+        layout = attach_bases(pack_for(rows_of, cap, self._quads_run) if pad else pack(rows_of), base_of, mirrored)
         if pad:
             layout = pad_rows(layout, cap)
         if layout.n_rows > rows.size:

@@ -249,3 +249,87 @@ def test_pack_quads_keeps_quads_apart_and_every_row():
         assert small.n_rows <= cap
         if lay.n_rows < QUAD_MIN_ROWS - 64:
             assert np.array_equal(pack_for(rows, 1 << 16).row_desc, pack(rows).row_desc)
+
+
+def _mix(rng, n):
+    """Requests of 1, 16 or 31 rotations, half of them mirrored."""
+    from irisb200.batched import Request
+    z = np.zeros((3, 12800), np.uint16), np.zeros((3, 6400), np.uint16)
+    return [Request(code=z[0], mask=z[1], n_rot=int(rng.choice([1, 16, 31])), mirrored=bool(rng.random() < 0.5))
+            for _ in range(n)]
+
+
+def test_rows_are_packed_by_quads_only_where_the_pass_runs_them(monkeypatch):
+    """An engine whose pass cannot run the quad GEMM (no sums, a path with a
+    tile of its own, launches too short) packs densely; one that can, and gains
+    by it, packs by quads."""
+    e, _ = _fake_engine(monkeypatch)
+    e.max_variants = 128
+    asked = []
+
+    class Engine(_Obj):
+        runs = True
+
+        def runs_quads(self, engines, n_rows, length, pair):
+            asked.append((len(engines), n_rows, length, pair))
+            return Engine.runs
+    e.ce = [Engine(query_length=4096) for _ in range(3)]
+    e.me = [Engine(query_length=4096) for _ in range(3)]
+    reqs = _mix(np.random.default_rng(4), 48)
+    uniq, _ = e._variants(reqs)
+    dense = pack([list(centred_rotations(reqs[i].n_rot)) for i, _ in uniq])
+
+    def rows(path, autotune=False):
+        e.fixed, e.autotune = path, autotune
+        buf = np.zeros(4096, np.uint32)
+        seg = (np.zeros(129, np.uint32), np.zeros(128, np.uint32), np.zeros(128, np.uint32))
+        code, mask = np.zeros((3, 128, 12800), np.uint16), np.zeros((3, 128, 6400), np.uint16)
+        return e._stage(reqs, uniq, code, mask, buf, seg, 4096, pad=True)[0]
+    live = lambda lay: int((lay.row_desc != 0xFFFFFFFF).sum())  # noqa: E731
+    for path, autotune in (("pair", False), (None, True), ("pair", True)):
+        lay = rows(path, autotune)
+        assert _quad_pure(lay.row_desc) and live(lay) == live(dense)
+        assert asked[-1][0] == 6 and asked[-1][2] <= e.db_len and asked[-1][3]
+    for path, autotune in (("split", False), ("fused", False), (None, False), ("split", True)):
+        n = len(asked)
+        lay = rows(path, autotune)  # a tile width of its own: not even asked
+        assert lay.n_slots == dense.n_slots and not _quad_pure(lay.row_desc) and len(asked) == n
+    e.tuned = {k: ("split", 256, 32768) for k in range(64, 4097, 64)}  # what the tuner chose
+    assert not _quad_pure(rows(None, True).row_desc)
+    e.tuned = {k: ("split", 0, 32768) for k in range(64, 4097, 64)}  # the library's own choice
+    assert _quad_pure(rows(None, True).row_desc)
+    e.tuned = {}
+    Engine.runs = False
+    assert not _quad_pure(rows("pair").row_desc)
+
+
+def test_packing_takes_the_cheaper_pass():
+    """Quads kept apart cost padded rows: they are taken where the measured time
+    of that many on the quad GEMM is below that of the dense rows."""
+    from irisb200.batched import pack_for, pack_quads, padded_rows
+    rng = np.random.default_rng(8)
+    quad = dict(zip((640, 768, 1024, 1280, 2048), (2.55, 2.85, 3.47, 4.65, 6.55)))
+    plain = dict(zip((512, 640, 768, 1024, 1280, 2048), (2.37, 3.2, 3.6, 4.7, 5.95, 9.7)))
+    both = set()
+    for n in range(17, 60):
+        rows = [list(centred_rotations(r.n_rot)) for r in _mix(rng, n) for _ in range(2 if r.mirrored else 1)]
+        got = pack_for(rows, 4096)
+        dense, apart = pack(rows), pack_quads(rows)
+        p, q = padded_rows(dense.n_rows, 4096), padded_rows(apart.n_rows, 4096)
+        if p not in plain or q not in quad or dense.n_rows != -(-sum(map(len, rows)) // 32) * 32:
+            continue
+        pays = quad[q] < plain[p]
+        assert np.array_equal(got.row_desc, (apart if pays else dense).row_desc)
+        both.add((p, q, pays))
+    assert (512, 640, False) in both and any(pays for _, _, pays in both)
+
+
+def test_the_two_sm_path_takes_every_row_count_it_can_run():
+    from irisb200.batched import BatchedEngine
+    e = BatchedEngine.__new__(BatchedEngine)
+    e.db_len, e.fixed = 65536, "pair"
+    assert e._pass_candidates(640) == [("pair", 256, c) for c in (65536, 32768, 16384, 8192)]
+    assert e._pass_candidates(2048) == [c for c in BatchedEngine._candidates(2048, 65536) if c[0] == "pair"]
+    assert e._pass_candidates(64) == BatchedEngine._candidates(64, 65536)  # no two-SM GEMM there
+    e.fixed = None
+    assert e._pass_candidates(640) == BatchedEngine._candidates(640, 65536)

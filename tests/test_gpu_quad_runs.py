@@ -199,3 +199,31 @@ def test_six_engines_and_sums_that_give_way(dm):
         x.free()
     for e in engines:
         e.close()
+
+
+def test_runs_quads_tells_what_a_launch_does(dm):
+    n_db = 9500
+    rng = np.random.default_rng(10)
+    engines = [irisb200.ShareDB(p % 3, dm, n_db, 1000, 6400, W.SEEDS[p % 3]) for p in range(6)]
+    for e in engines:
+        e.alloc_db(n_db)
+    seen = set()
+    for n_q in (16, 18, 20, 25, 30):
+        for e in engines:
+            e.query_upload_slots(rng.integers(0, 1 << 16, (n_q, 6400), dtype=np.uint16),
+                                 [(j, 0, 31, j) for j in range(n_q)])
+        for pair in (False, True):
+            for e in engines:
+                e.set_pair(pair)
+            for some in (engines[:1], engines[:3], engines):
+                for length in (96, 1024, 3000, n_db):
+                    irisb200.dot_many(some, [1] * len(some), 0, length)
+                    ran = some[0].last_gemm()[0] == "quad"
+                    assert irisb200.ShareDB.runs_quads(some, 32 * n_q, length, pair) == ran
+                    seen.add((n_q, ran))
+    assert {q for q, ran in seen if ran} == {18, 20, 25, 30} and (16, False) in seen
+    assert not irisb200.ShareDB.runs_quads(engines, 2048, n_db, False)  # above the capacity
+    dm.derived_bytes(give_back=True)
+    assert not irisb200.ShareDB.runs_quads(engines, 640, n_db, False)
+    for e in engines:
+        e.close()
