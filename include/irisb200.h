@@ -582,7 +582,9 @@ int irs_scan_set_timing(irs_scan* s, size_t max_passes);
 int irs_scan_timings(irs_scan* s, double* gemm_ms, double* threshold_ms, double* pass_ms, size_t cap, size_t* n,
                      int reset);
 /* Times `passes` consecutive passes of every candidate (only those on path
- * `only_path` when >= 0) after a warm one (comparator reset before each),
+ * `only_path` when >= 0; without that restriction, where the list has no
+ * IRS_SCAN_PAIR and the uploaded rows pad to 128 or more, the two-SM GEMM and
+ * the library's own choice, tile 0, as well) after a warm one (comparator reset before each),
  * re-times the `finalists` fastest interleaved for `rounds` rounds and
  * configures the best mean; `log` receives the first-round times, then each
  * finalist's mean (*n_log = the count; at most log_cap written). */

@@ -99,7 +99,7 @@ class PlainScan:
         `only_path` restricts the candidates to one path.
         tune_log: (candidate, ms per pass) of the first round, then
         (candidate, mean ms over the interleaved rounds) per finalist."""
-        cap = len(self.candidates()) + max(0, finalists)
+        cap = len(self.candidates()) + 6 + max(0, finalists)  # (up to 6 that tune() adds to the list)
         log = (ScanTiming * cap)()
         chosen, n = ScanCandidate(), C.c_size_t()
         op = -1 if only_path is None else SCAN_PATHS.index(only_path)
