@@ -28,6 +28,7 @@ admitted afterwards scan it.  The device batch counter advances every step
 from __future__ import annotations
 
 import collections
+import functools
 import heapq
 import math
 import time
@@ -38,7 +39,7 @@ import numpy as np
 from . import (IRIS_CODE_LENGTH, MASK_CODE_LENGTH, MAX_MATCHES_LEN, DistanceComparator, Event, IrisError,
                PinnedArray, ShareDB, dot_many, mirror_query_share)
 from .batched import (MULTS, QUAD_MIN_ROWS, Request, Result, attach_bases, centred_rotations, first_quads, pack,
-                      padded_rows)
+                      padded_rows, quads_of)
 
 RESULT_BYTES_PER_ROW_ENTRY = 2 * 6  # u16 dot share per (row, entry) for 6 engines
 
@@ -62,6 +63,12 @@ def split_record_i8(record: np.ndarray):
     return lo, hi
 
 
+# Placement looks at every word for every waiting request of a step, and most
+# words are as they were for the one before: 64 words in 5 us instead of 50 to 140.
+_remembered = functools.lru_cache(maxsize=1 << 14)
+
+
+@_remembered
 def _first_run(occupied: int, n: int) -> int:
     """Lowest bit position f with bits f..f+n-1 clear in a 32-bit word, or -1."""
     free = ~occupied & 0xFFFFFFFF
@@ -79,6 +86,19 @@ def _quads_of(occupied: int) -> int:
     x = occupied | occupied >> 2
     x = (x | x >> 4) & 0x03030303
     return x & 3 | x >> 6 & 12 | x >> 12 & 48 | x >> 18 & 192
+
+
+@_remembered
+def _first_quad_row(occupied: int, n: int) -> int:
+    """First row of a word where a run of n rows has its quads to itself, or -1."""
+    q = first_quads(_quads_of(occupied), n)
+    return q // 2 * 8 + q % 2 if q >= 0 else -1
+
+
+def _dense_rows(n: int) -> int:
+    """Rows of a word that a run of n rows takes among its like, as many of them
+    as fit (11 rows: two runs, 16 each); not more than its quads."""
+    return min(4 * quads_of(n), 32 // (32 // n))
 
 
 @dataclass
@@ -121,8 +141,9 @@ class ContinuousServer:
     results, with the library in its asynchronous host mode and every host
     buffer it reads or writes page-locked and double-buffered."""
 
-    quads = True      # the engines hold what the library's quad GEMM needs
+    quads = True      # the steps run the library's quad GEMM where their rows are quads
     slots_in_use = 0  # words that held rows when the layout was last made
+    mix_rows = mix_quads = 0.0  # what the last few hundred runs take: rows (_dense_rows), and quads when kept apart
 
     def __init__(self, dm, code_engines, mask_engines, circuits, chunk: int = 32768, row_capacity: int = 2048,
                  max_variants: int = 512, max_reauth: int = 64, threshold_a: int = 16384, seeds=None,
@@ -139,7 +160,7 @@ class ContinuousServer:
         # 16,384- or 8,192-entry steps
         for e in self.ce + self.me:
             e.set_pair(gemm_pair)
-        self.quads = all(e.has_sums() for e in self.ce + self.me)
+        self.gemm_pair = gemm_pair
         self.c = circuits
         self.A = threshold_a
         self.chunk = max(32, chunk // 32 * 32)
@@ -167,6 +188,7 @@ class ContinuousServer:
         circuits.use_batch_counter(True)
         dm.set_batch_counter(1)
         self._alloc_host(nsub)
+        self._check_quads(0)
         self.flight = []
         self.layout_dirty = False
         self.next_chunk = 0
@@ -207,16 +229,29 @@ class ContinuousServer:
         n = self.db_len if db_len is None else db_len
         return max(1, math.ceil(n / self.chunk))
 
+    def _check_quads(self, n_rows: int) -> None:
+        """Whether steps over n_rows rows run the quad GEMM if the rows are quads:
+        asked with every layout, since the library may have given the memory of
+        the engines' sums to another allocation."""
+        self.quads = bool(self.ce[0].runs_quads(self.ce + self.me, max(n_rows, QUAD_MIN_ROWS),
+                                                min(self.chunk, self.db_len), getattr(self, "gemm_pair", True)))
+
     def _place(self, n: int):
         """First free run of n rows: once as many words are in use as the
         library's quad GEMM takes (words fill from the front), with its quads
-        of rows to itself, or none until others complete; else any."""
+        of rows to itself, or none until others complete; else any.  Runs of few
+        rows fill their quads badly (one of 3 rows takes the room of 8), so the
+        quads of the requests' mix must cost less than its rows alone: a full
+        row table takes 0.69 of the time on the quad GEMM at 2,048 rows, 0.80 at
+        640, so they may be at most four thirds of the rows."""
         busy = QUAD_MIN_ROWS // 32 - 3
-        if self.quads and self.n_slot_cap > busy + 2 and (self.slot_occ[busy] or self.slots_in_use > busy):
+        apart = 3 * (self.mix_quads + quads_of(n)) < self.mix_rows + _dense_rows(n)
+        if (self.quads and apart and self.n_slot_cap > busy + 2
+                and (self.slot_occ[busy] or self.slots_in_use > busy)):
             for s in range(self.n_slot_cap):
-                q = first_quads(_quads_of(self.slot_occ[s]), n)
-                if q >= 0:
-                    return s, q // 2 * 8 + q % 2
+                f = _first_quad_row(self.slot_occ[s], n)
+                if f >= 0:
+                    return s, f
             return None
         for s in range(self.n_slot_cap):
             f = _first_run(self.slot_occ[s], n)
@@ -227,6 +262,8 @@ class ContinuousServer:
     def _occupy(self, v: _Variant, s: int, f: int) -> None:
         n = len(v.rots)
         self.slot_occ[s] |= ((1 << n) - 1) << f
+        self.mix_rows = self.mix_rows * 0.996 + _dense_rows(n)
+        self.mix_quads = self.mix_quads * 0.996 + quads_of(n)
         self.slot_vars[s].append(v)
         v.slot, v.first = s, f
 
@@ -323,6 +360,7 @@ class ContinuousServer:
         for e in self.ce + self.me:
             e.query_expand_rows(self.max_variants, rt)
         self.dc.set_segments(ss[: seg_start.size], sq[: seg_query.size], sm[: seg_mask.size])
+        self._check_quads(row_desc.size)
         self.rows_active = row_desc.size
         self.layout_dirty = False
 

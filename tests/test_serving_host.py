@@ -238,3 +238,55 @@ def test_placement_in_a_large_server_keeps_quads_apart():
     for q in range(8):  # the quads of a word, row by row
         for r in range(32):
             assert bool(_quads_of(1 << r) >> (r // 8 * 2 + r % 2) & 1)
+
+
+def _busy(s):
+    for slot in range(16):
+        s._occupy(_Variant(0, False, list(range(31))), slot, 0)
+
+
+def test_runs_of_few_rows_fill_a_busy_server():
+    """Quads kept apart would leave most of their rows empty: they are placed
+    densely, as many as the free words hold."""
+    for n, per_word in ((1, 32), (3, 10), (11, 2)):
+        s = _placer(40)
+        for slot in range(16):
+            s._occupy(_Variant(0, False, list(range(n))), slot, 0)
+        placed = 0
+        while (where := s._place(n)) is not None:
+            s._occupy(_Variant(0, False, list(range(n))), *where)
+            placed += 1
+        assert placed == 40 * per_word - 16
+    s = _placer(40)
+    _busy(s)
+    assert s._place(16) == (16, 0)
+    s._occupy(_Variant(0, False, list(range(16))), 16, 0)
+    for k in range(16):  # among long runs, short ones keep their quads
+        where = s._place(5)
+        s._occupy(_Variant(k + 1, False, list(range(5))), *where)
+        assert where == (16 + (k + 2) // 4, (k + 2) % 4 * 8)
+
+
+def test_placement_follows_the_sums(monkeypatch):
+    """The library is asked with every layout whether the steps run the quad
+    GEMM; once it has taken the sums back, any free rows will do."""
+    s, _ = _fake_server(monkeypatch, db_len=100_000, chunk=32768, rows=40 * 32, max_variants=64)
+    asked = []
+
+    def runs_quads(engines, n_rows, length, pair):
+        asked.append((len(engines), n_rows, length, pair))
+        return Held.sums
+
+    class Held:
+        sums = True
+    s.ce[0].runs_quads = runs_quads
+    _busy(s)
+    s.pending_bases = set()
+    s._upload_layout()
+    assert asked == [(6, 576, 32768, True)] and s.quads
+    for slot in range(16, 40):
+        s._occupy(_Variant(0, False, list(range(31))), slot, 0)
+    assert s._place(1) is None  # rows are free, quads are not
+    Held.sums = False
+    s._upload_layout()
+    assert not s.quads and s._place(1) == (0, 31)
