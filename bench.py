@@ -528,6 +528,7 @@ def run_ours(args):
     dm.synchronize()
     clk_value = clk.summary(clk.windows[-1])
     total_ms = begin.elapsed_time(end)
+    gemm = gemm_kernel_of(chosen[0], ce[0].last_gemm()[0])
     gemm_ms, thr_ms, batch_ms = ps.timings()  # per step, summed over its chunks
     ps.set_timing(0)
     if dist:
@@ -770,7 +771,8 @@ def run_ours(args):
         ops = 3 * 6 * (K_CODE + K_MASK) * (NQ * 31) * M  # algorithmic int8 ops per batch (all chunks)
         ops_launch = ops * chunks[0][1] / M  # per GEMM launch (one chunk)
         gemm_avg = statistics.mean(gemm_ms)  # per batch = sum over its chunk launches
-        achieved = ops / (gemm_avg * 1e-3) / 1e12  # = ops per launch / mean launch duration
+        equivalent = ops / (gemm_avg * 1e-3) / 1e12  # = ops per launch / mean launch duration
+        achieved = equivalent * gemm["multiplications"]  # those that the kernel carries out
         traffic = traffic_source = None
         # algorithmic DRAM bytes of one launch: the six engines' DB limb planes
         # once, their query planes once, the u16 dot shares written
@@ -783,7 +785,7 @@ def run_ours(args):
             # a capture of this launch's own chunk length when the profile has
             # one; else the path's capture scaled by the entries a launch scans
             # (an estimate: the query planes' share of the bytes changes with it)
-            key = {"split": "limb_gemm", "pair": "quad_gemm", "fused": "fused_scan"}[chosen[0]]
+            key = gemm["profile"]
             own = pj.get(key + "_by_chunk", {}).get(str(chunks[0][1]), {})
             lg = pj.get(key, {})
             if own.get("dram_bytes_per_launch"):
@@ -828,13 +830,12 @@ def run_ours(args):
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": None, "unit": "TOPS",
                          "frac": None, "traffic": traffic, "traffic_source": traffic_source,
                          "algorithmic_bytes_per_launch": alg_bytes,
-                         "kernel": {"split": "limb_gemm_kernel<256>",
-                                    "pair": "quad_gemm_kernel (cta_group::2, 9/16 of the multiplications, counted "
-                                            "in full)",
-                                    "fused": "fused_scan_kernel (GEMM and threshold: time includes the threshold)"}
-                                   [chosen[0]] + f" (6 engines, one launch per {chunks[0][1]}-entry DB chunk, "
+                         "kernel": gemm["kernel"] + f" (6 engines, one launch per {chunks[0][1]}-entry DB chunk, "
                                    f"{len(chunks)} per batch)",
-                         "ops_per_launch": ops_launch,
+                         "ops_per_launch": ops_launch * gemm["multiplications"],
+                         "equivalent_tops": equivalent,
+                         "equivalent_ops_per_launch": ops_launch,
+                         "equivalent": "the multiplications of the plain limb GEMM for the same dot shares",
                          "peak_source": "2 x measured dense bf16, sustained (MEASURED_PEAKS.json "
                                         "bf16_tflops_sustained; dense int8 issues at twice the bf16 rate on "
                                         "B200): the GEMM is timed over back-to-back steps",
@@ -892,6 +893,19 @@ def run_ours(args):
         dist.barrier()
         dist.destroy_process_group()
     return result
+
+
+def gemm_kernel_of(path: str, ran: str) -> dict:
+    """The GEMM kernel of a pass on `path` whose last dot launched `ran`
+    (ShareDB.last_gemm): its name, its key in the traffic profile, and the share
+    of the plain limb GEMM's multiplications that it carries out."""
+    name, profile, share = {
+        "fused": ("fused_scan_kernel (GEMM and threshold: time includes the threshold)", "fused_scan", 1.0),
+        "one_sm": ("limb_gemm_kernel<256>", "limb_gemm", 1.0),
+        "pair": ("limb_gemm_pair_kernel (cta_group::2)", "limb_gemm_pair", 1.0),
+        "quad": ("quad_gemm_kernel (cta_group::2, nine products of K/4 in place of sixteen)", "quad_gemm", 9 / 16),
+    }["fused" if path == "fused" else ran]
+    return {"kernel": name, "profile": profile, "multiplications": share}
 
 
 def threshold_roofline(thr_ms: float, words: int, n_sm: int, sm_mhz, chunks) -> dict:

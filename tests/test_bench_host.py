@@ -100,3 +100,15 @@ def test_cpu_mpc_simulation_matches_plaintext():
     assert out["equal_to_plaintext"]
     assert out["matches"] >= 1
     assert out["value"] > 0 and out["kind"] == "port"
+
+
+def test_roofline_names_the_gemm_that_ran():
+    """The two-SM path runs the rotation-structured GEMM only where the engines
+    hold its sums; the roofline counts the multiplications that were carried out."""
+    of = bench.gemm_kernel_of
+    assert of("pair", "quad")["profile"] == "quad_gemm" and of("pair", "quad")["multiplications"] == 9 / 16
+    assert of("split", "quad") == of("pair", "quad")  # the library's own choice
+    for path, ran, profile in (("pair", "pair", "limb_gemm_pair"), ("split", "one_sm", "limb_gemm"),
+                               ("fused", "pair", "fused_scan")):
+        k = of(path, ran)
+        assert k["profile"] == profile and k["multiplications"] == 1.0 and profile in k["kernel"]
