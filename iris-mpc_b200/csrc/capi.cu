@@ -645,8 +645,6 @@ int irs_device_manager_init(int device, irs_device_manager** out) {
   CU(cudaMalloc(&dm->d_batch, sizeof(uint64_t)));
   CU(cudaMemset(dm->d_batch, 0, sizeof(uint64_t)));
   CU(cudaEventCreateWithFlags(&dm->graph_done, cudaEventDisableTiming));
-  CU(cudaEventCreateWithFlags(&dm->graph_ran, cudaEventDisableTiming));
-  CU(cudaStreamCreateWithFlags(&dm->graph_join, cudaStreamNonBlocking));
   for (cudaEvent_t& e : dm->uploads) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   try {
     SumWriter lock(sum_holders(device).mu);
@@ -2241,6 +2239,13 @@ int irs_graph_end_capture(irs_device_manager* dm, irs_graph** out) {
   dm->capturing = false;
   cudaGraph_t g = nullptr;
   CU(cudaStreamEndCapture(dm->streams[0], &g));
+  cudaError_t made = cudaSuccess;  // with the first graph: most managers have none
+  if (!dm->graph_ran) made = cudaEventCreateWithFlags(&dm->graph_ran, cudaEventDisableTiming);
+  if (made == cudaSuccess && !dm->graph_join) made = cudaStreamCreateWithFlags(&dm->graph_join, cudaStreamNonBlocking);
+  if (made != cudaSuccess) {
+    cudaGraphDestroy(g);
+    return fail(IRS_ERR_CUDA, "stream or event of the graphs: %s", cudaGetErrorString(made));
+  }
   auto* gr = new (std::nothrow) irs_graph();
   if (!gr) {
     cudaGraphDestroy(g);
