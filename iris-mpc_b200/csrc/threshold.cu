@@ -334,8 +334,9 @@ cudaError_t launch_threshold_flat(const ThresholdParams& P, int stage, cudaStrea
   const uint64_t n_warps = (P.n_words + 31) / 32;
   if (n_warps <= kSplitMost) {
     static std::atomic<uint64_t> split_full{0}, split_msb{0};
-    cudaError_t e = smem_limit_once(threshold_flat_split_kernel<kStageFull>, kSplitSmem, split_full);
-    if (e == cudaSuccess) e = smem_limit_once(threshold_flat_split_kernel<kStageMsbOnly>, kSplitSmem, split_msb);
+    const cudaError_t e = stage == kStageFull
+                              ? smem_limit_once(threshold_flat_split_kernel<kStageFull>, kSplitSmem, split_full)
+                              : smem_limit_once(threshold_flat_split_kernel<kStageMsbOnly>, kSplitSmem, split_msb);
     if (e != cudaSuccess) return e;
     if (stage == kStageFull)
       threshold_flat_split_kernel<kStageFull><<<(unsigned)n_warps, kSplitThreads, kSplitSmem, stream>>>(P);
