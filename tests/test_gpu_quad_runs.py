@@ -227,3 +227,31 @@ def test_runs_quads_tells_what_a_launch_does(dm):
     assert not irisb200.ShareDB.runs_quads(engines, 640, n_db, False)
     for e in engines:
         e.close()
+
+
+def test_a_program_s_own_capture_keeps_the_sums(dm):
+    """A dot captured by the program itself, on the engine's own party stream,
+    replays on the sums it was captured with: they are not given back."""
+    import torch
+    K, n_db, n_q = 6400, 16384, 20
+    rng = np.random.default_rng(14)
+    e = irisb200.ShareDB(0, dm, n_db, n_q * 32, K, W.SEEDS[0])
+    e.alloc_db(n_db)
+    e.fill_random(6, n_db)
+    e.query_upload_slots(rng.integers(0, 1 << 16, (n_q, K), dtype=np.uint16), [(j, 0, 31, j) for j in range(n_q)])
+    want = _quad(e, 0, n_db)
+    dm.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(dm.stream(0)), capture_error_mode="thread_local"):
+        e.dot(0, n_db, 1)
+    assert e.last_gemm() == ("captured", n_q * 32)
+    dm.derived_bytes(give_back=True)
+    assert e.has_sums()
+    ptr, stride = e.result_view()
+    for _ in range(2):
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(e.fetch_results(n_db), want)
+    del g
+    torch.cuda.synchronize()
+    e.close()
