@@ -837,8 +837,12 @@ cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair, int n_sms, c
   if (pair) {
     P.pair_n = gemm_pair_n(P.prob[0].n_pad);
     const int units = (int)P.prob[0].n_pad / 64, tiles = (int)(P.prob[0].n_pad + kPairMaxN - 1) / kPairMaxN;
-    // 960 rows as 4 x 256: 0.73 ms (one engine x 32,768 entries), as 256 x 3 +
-    // 192 0.77: tiles of unequal length drift apart and share less of L2
+    // Tiles of unequal length drift apart and share less of L2, equal ones pad
+    // the rows.  32,768 entries, unequal / equal, one engine and six: 704 rows
+    // (padded by 1/11) 0.622 / 0.623 and 2.60 / 2.63 ms, 896 (2/14) 0.709 / 0.753
+    // and 3.09 / 3.37, 960 (1/15) 0.798 / 0.763 and 3.72 / 3.62, 1216 (1/19) 0.972
+    // / 0.962 and 4.36 / 4.61, 1984 (1/31) 1.503 / 1.467 and 7.59 / 8.16, in long
+    // runs 8.50 / 7.96.  From a fifteenth down they are as good or better.
     const int spare = P.pair_n / 64 * tiles - units;  // units of padding if all tiles were as wide
     P.pair_wider = 15 * spare <= units ? tiles : units % tiles;
     block_n = kPairMaxN;  // the tiles of a problem: as many as 256-row ones

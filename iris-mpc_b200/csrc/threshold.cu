@@ -322,10 +322,10 @@ static cudaError_t allow_rand_smem(K kernel, std::atomic<uint64_t>& done) {
 }
 
 // Most warps' worth of words (32 each) that run in the split kernels: two rounds
-// of the three blocks that fit an SM.  Flat calls, split against one thread per
+// of the three blocks that fit an SM, of a B200's 148.  Flat calls, split against one thread per
 // word: 4,096 elements 10.5 / 25 us (cold), 454,656 18.5 / 23.5, 699,968 24.7 /
 // 34.9, 1,048,576 34.0 / 34.4, 2,097,152 66 / 64, 4,194,304 123 / 104.
-constexpr uint64_t kSplitMost = 888;
+constexpr uint64_t kSplitMost = 2 * 3 * 148;
 
 bool threshold_writes_shares(uint64_t n_words) { return (n_words + 31) / 32 <= kSplitMost; }
 

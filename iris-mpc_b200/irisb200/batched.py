@@ -139,7 +139,7 @@ def _layout_of(slots, variant_rows) -> Layout:
                   np.array(seg_mask, np.uint32), n_slots * 32, n_slots)
 
 
-QUAD_MIN_ROWS = 576  # padded query rows from which the library's quad GEMM runs
+QUAD_MIN_ROWS = 576  # padded query rows from which the library's quad GEMM can run (runs_quads: whether it does)
 
 
 def first_quads(occupied: int, n: int) -> int:
