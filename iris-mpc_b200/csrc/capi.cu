@@ -147,7 +147,8 @@ struct irs_sharedb {
   uint8_t* sums = nullptr;
   uint8_t* forms = nullptr;
   uint32_t* row_valid = nullptr;
-  uint32_t* quad_flag = nullptr;  // QuadFlags word, for captured launches (kept until destroy)
+  uint32_t* quad_flag = nullptr;  // QuadFlags word, for captured launches
+  std::vector<uint32_t*> old_flags;  // words of graphs over sums that are gone: zero, kept until destroy
   uint32_t flag_rows = 0;     // what the last upload left in it
   bool quad_rows = false;     // the uploaded rows are quads of rotations and the forms hold them
   size_t stale_end = 0;       // records below it have sums that a small gather left behind
@@ -241,16 +242,22 @@ struct DroppedSums {
 // Takes an engine's sums and forms away from it (its device's lock is held
 // alone); the caller frees them once it has released the lock: cudaFree waits
 // for the launches that read them.
-// A graph that holds the quad GEMM is told by the flag to run the plain one;
-// replays start under the lock, so that none reads the flag half-way.
+// A graph that holds the quad GEMM is told by the flag to run the plain one, for
+// good: the word is its own from here on, and whatever sums the engine gets next
+// have another.  Replays start under the lock, so that none reads it half-way.
 DroppedSums take_sums(irs_sharedb* db) {
-  if (db->quad_flag && db->dot_captured) {
+  if (db->quad_flag && (db->dot_captured || db->sums_pinned)) {
     if (cudaEventSynchronize(db->dm->graph_done) != cudaSuccess) {
       cudaGetLastError();
       cudaDeviceSynchronize();
     }
     cudaMemsetAsync(db->quad_flag, 0, 4, db->dm->streams[db->peer]);
     cudaStreamSynchronize(db->dm->streams[db->peer]);
+    try {
+      db->old_flags.push_back(db->quad_flag);
+    } catch (const std::bad_alloc&) {  // four bytes of the pool stay with the device manager
+    }
+    db->quad_flag = nullptr;
     db->flag_rows = 0;
   }
   auto& v = sum_holders(db).engines;
@@ -475,6 +482,7 @@ void alloc_sums(irs_sharedb* db) {
   db->forms = static_cast<uint8_t*>(f);
   db->row_valid = reinterpret_cast<uint32_t*>(db->forms + forms);
   db->flag_rows = 0;
+  db->stale_end = 0;
   cudaStream_t st = dm->streams[db->peer];
   uint8_t* inner = db->sums + 2 * cap * (K / 2);
   if (make_tmap_plane(&db->tm_sum_lo[0], db->sums, cap, K / 2, 128) ||
@@ -972,6 +980,7 @@ int irs_sharedb_destroy(irs_sharedb* db) {
   pool_free(dm, db->peer, db->d_slots);
   pool_free(dm, db->peer, db->results);
   pool_free(dm, db->peer, db->quad_flag);
+  for (uint32_t* w : db->old_flags) pool_free(dm, db->peer, w);
   cudaStreamSynchronize(dm->streams[db->peer]);
   if (db->done) cudaEventDestroy(db->done);
   if (db->copied) cudaEventDestroy(db->copied);

@@ -255,3 +255,33 @@ def test_a_program_s_own_capture_keeps_the_sums(dm):
     del g
     torch.cuda.synchronize()
     e.close()
+
+
+def test_records_allocated_anew_start_a_new_generation_of_sums(dm):
+    """Records allocated anew have sums and a device word of their own: a graph
+    over the first ones (not launched again) keeps a word that no upload writes,
+    and one captured over the new ones follows the uploads and the sums."""
+    K, n_q = 6400, 20
+    rng = np.random.default_rng(15)
+    e = irisb200.ShareDB(0, dm, 16384, n_q * 32, K, W.SEEDS[0])
+    base = rng.integers(0, 1 << 16, (n_q, K), dtype=np.uint16)
+    slots = [(j, 0, 31, j) for j in range(n_q)]
+    graphs, want = [], None
+    for n_db in (16384, 16000, 16384):
+        e.alloc_db(n_db)
+        e.fill_random(n_db, n_db)
+        e.query_upload_slots(base, slots)
+        want = _quad(e, 0, n_db)
+        assert np.array_equal(want, _plain(e, 0, n_db))
+        dm.synchronize()
+        graphs.append(irisb200.Graph.capture(dm, lambda: e.dot(0, n_db, 1, dm.stream(0))))
+        assert e.last_gemm() == ("captured", n_q * 32)
+        for held in (True, False):
+            graphs[-1].launch(dm.stream(0))
+            dm.synchronize()
+            assert np.array_equal(e.fetch_results(n_db), want)
+            dm.derived_bytes(give_back=True)
+            assert not e.has_sums() and e.last_gemm()[1] == 0
+    for g in graphs:
+        g.close()
+    e.close()
