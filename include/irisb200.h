@@ -275,11 +275,14 @@ int irs_mirror_query_share(uint16_t* coefs, size_t n, int flip_imaginary);
  * Default: the 64-row tile for 64 padded rows, up to 768 the two-SM GEMM (or
  * 128-row tiles in launches of few tiles), above that the 256-row tile, and the
  * rotation-structured GEMM where the uploaded rows and the launch suit it; a
- * width given here runs the one-SM GEMM.  The dot shares do not depend on it. */
+ * width given here that divides the padded rows runs the one-SM GEMM (with
+ * set_pair, the two-SM GEMMs).  The dot shares do not depend on it. */
 int irs_sharedb_set_tile(irs_sharedb* db, int block_n);
-/* on != 0: the GEMM runs on SM pairs wherever it can (a cluster of two CTAs with
+/* on != 0: the GEMM runs on SM pairs (a cluster of two CTAs with
  * tcgen05.mma.cta_group::2 on a tile of 256 entries and up to 256 rows; same
- * results), the rotation-structured GEMM included.  Off by default, which leaves
+ * results) from 128 padded rows on, the rotation-structured GEMM included; a
+ * launch of few rounds still takes one-SM tiles where those are expected to take
+ * less, unless its rows are whole 256-row tiles.  Off by default, which leaves
  * the choice to the library: under the B200's power cap long launches of many
  * rows trade clock for MAC rate, so the batch autotuner decides there (no
  * counterpart in the reference). */

@@ -160,7 +160,7 @@ struct irs_sharedb {
       tm_form_hi[kQuadWidths]{};
   CUtensorMap tm_db_lo{}, tm_db_hi{}, tm_q_lo{}, tm_q_hi{};
   CUtensorMap tm_qp_lo{}, tm_qp_hi{};    // half a tile of the two-SM GEMM
-  CUtensorMap tm_q128_lo{}, tm_q128_hi{};  // 128 rows, for launches of few tiles
+  CUtensorMap tm_qf_lo[2]{}, tm_qf_hi[2]{};  // 64 and 128 rows, for launches of few rounds
   int block_n = 0;
   cudaEvent_t done = nullptr;  // recorded after the engine's last dot launch
   cudaEvent_t copied = nullptr;  // recorded after an upload's last read of host memory
@@ -420,8 +420,10 @@ int rebuild_query_maps(irs_sharedb* db) {
       make_tmap_u8(&db->tm_q_hi, db->q_hi, db->n_cap, db->code_length, box) ||
       make_tmap_u8(&db->tm_qp_lo, db->q_lo, db->n_cap, db->code_length, half) ||
       make_tmap_u8(&db->tm_qp_hi, db->q_hi, db->n_cap, db->code_length, half) ||
-      make_tmap_u8(&db->tm_q128_lo, db->q_lo, db->n_cap, db->code_length, 128) ||
-      make_tmap_u8(&db->tm_q128_hi, db->q_hi, db->n_cap, db->code_length, 128))
+      make_tmap_u8(&db->tm_qf_lo[0], db->q_lo, db->n_cap, db->code_length, 64) ||
+      make_tmap_u8(&db->tm_qf_hi[0], db->q_hi, db->n_cap, db->code_length, 64) ||
+      make_tmap_u8(&db->tm_qf_lo[1], db->q_lo, db->n_cap, db->code_length, 128) ||
+      make_tmap_u8(&db->tm_qf_hi[1], db->q_hi, db->n_cap, db->code_length, 128))
     return fail(IRS_ERR_CUDA, "tensor map for the query planes failed");
   return IRS_OK;
 }
@@ -1366,8 +1368,9 @@ int irs_sharedb_set_batch(irs_sharedb* db, uint64_t batch_id) {
   return IRS_OK;
 }
 
-// The GEMM that a launch's query maps are for.
-enum class Gemm { kOneSm, kPair, kFewTiles };
+// The GEMM that a launch's query maps are for: the one-SM kernel on the engine's
+// own tiles, the two-SM one, or the one-SM kernel on 64- or 128-row tiles.
+enum class Gemm { kOneSm, kPair, k64, k128 };
 
 static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t len, Gemm gemm, GemmProblem& pr) {
   CHECK(db->db_lo, IRS_ERR_STATE, "alloc_db not called");
@@ -1379,8 +1382,9 @@ static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t le
   memset(&pr, 0, sizeof pr);
   pr.tm_a_lo = db->tm_db_lo;
   pr.tm_a_hi = db->tm_db_hi;
-  pr.tm_b_lo = gemm == Gemm::kPair ? db->tm_qp_lo : gemm == Gemm::kFewTiles ? db->tm_q128_lo : db->tm_q_lo;
-  pr.tm_b_hi = gemm == Gemm::kPair ? db->tm_qp_hi : gemm == Gemm::kFewTiles ? db->tm_q128_hi : db->tm_q_hi;
+  const int f = gemm == Gemm::k128;
+  pr.tm_b_lo = gemm == Gemm::kPair ? db->tm_qp_lo : gemm == Gemm::kOneSm ? db->tm_q_lo : db->tm_qf_lo[f];
+  pr.tm_b_hi = gemm == Gemm::kPair ? db->tm_qp_hi : gemm == Gemm::kOneSm ? db->tm_q_hi : db->tm_qf_hi[f];
   pr.out = db->results;
   pr.m0 = (uint32_t)offset;
   pr.m_len = (uint32_t)len;
@@ -1397,68 +1401,71 @@ static int fill_problem(irs_sharedb* db, uint16_t mult, size_t offset, size_t le
   return IRS_OK;
 }
 
-// The tile width with which a launch over `len` entries can run as the
-// rotation-structured GEMM, or -1: every engine holds sums and form maps, the
-// caller left the GEMM open (no tile width asked for) or chose the two-SM one,
-// and the quad GEMM is expected to take less.  Whether it does run depends on
-// the uploaded rows.
-static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t len, bool pair) {
-  uint32_t K[kMaxGemmProblems];
-  for (int i = 0; i < n; i++) {
-    const irs_sharedb* e = engines[i];
-    if (!e->sums || e->n_pad != engines[0]->n_pad || e->forms_pad != e->n_pad || offset < e->stale_end) return -1;
-    if (e->tile_override && !gemm_pair_applies(e->pair, (uint32_t)e->n_pad)) return -1;
-    K[i] = (uint32_t)e->code_length;
-  }
-  const irs_sharedb* e = engines[0];
-  return quad_width_for(K, n, (uint32_t)len, (uint32_t)e->n_pad, e->block_n, pair, e->dm->n_sms);
+// Whether a launch takes less than about 2 ms.
+static bool short_launch(irs_sharedb* const* engines, int n, size_t len, size_t n_pad) {
+  double macs = 0;
+  for (int i = 0; i < n; i++) macs += 3.0 * (double)engines[i]->code_length * (double)n_pad * (double)len;
+  return macs < 3e12;
 }
-
-// Tiles of 128 entries x 128 query rows of a launch.
-static size_t tiles_128(int n, size_t len, size_t n_pad) { return (size_t)n * ((len + 127) / 128) * ((n_pad + 127) / 128); }
 
 // Whether the plain GEMM of a launch runs on SM pairs.  Six engines x 32,768
 // entries, one-SM against pair: 128 rows 0.86 / 0.87 ms (over 131,072 entries
 // with the threshold between the chunks 3.03 / 2.89), 192 1.32 / 1.01, 256
 // 1.37 / 1.18, 384 1.93 / 1.74, 512 2.46 / 2.10, 768 3.58 / 3.03, 960 4.18 /
 // 4.25, 1024 4.24 / 3.94; at 65,536 entries the last two are 8.6 / 9.0 and 8.4 /
-// 8.0.  So from 128 to 768 rows it is the default, as far as there are more
-// 128-row tiles than SMs (4,000 entries x 512 rows of one engine: 0.072 / 0.110
-// ms); above, where the caller chose it or the launch is short enough that the
-// clock has not dropped to the power limit (one engine x 32,768 entries, 960
-// rows 0.94 / 0.89, 1984 rows 1.60 / 1.51).
-static bool plain_pair_for(irs_sharedb* const* engines, int n, size_t len, size_t n_pad, bool pair) {
-  if (!gemm_pair_applies(true, (uint32_t)n_pad)) return false;
-  if (n_pad <= 768) return tiles_128(n, len, n_pad) > (size_t)engines[0]->dm->n_sms;
-  if (pair) return true;
-  double macs = 0;
-  for (int i = 0; i < n; i++) macs += 3.0 * (double)engines[i]->code_length * (double)n_pad * (double)len;
-  return macs < 3e12;  // about 2 ms
+// 8.0.  So from 128 to 768 rows it is the default; above, where the caller chose
+// it or the launch is short enough that the clock has not dropped to the power
+// limit (one engine x 32,768 entries, 960 rows 0.94 / 0.89, 1984 rows 1.60 /
+// 1.51); and in launches of a few rounds where it fills them as well as smaller
+// tiles would (few_rounds_tile), unless the caller chose it for whole 256-row
+// tiles.  Those run also where the engine's own tiles are wider (64 entries x 2048
+// rows, six engines, 128-row tiles 81 us, 256-row ones 112).
+struct PlainGemm {
+  bool pair;
+  int block_n;
+};
+static PlainGemm plain_gemm_for(irs_sharedb* const* engines, int n, size_t len, size_t n_pad, bool pair,
+                                bool narrow_tile = false) {
+  const int bn = gemm_block_n_for((uint32_t)n_pad);
+  const bool applies = gemm_pair_applies(true, (uint32_t)n_pad);
+  if (applies && pair && !narrow_tile && n_pad > 768 && n_pad % 256 == 0) return {true, bn};
+  uint32_t K[kMaxGemmProblems];
+  for (int i = 0; i < n; i++) K[i] = (uint32_t)engines[i]->code_length;
+  const int few = few_rounds_tile(K, n, (uint32_t)len, (uint32_t)n_pad, engines[0]->dm->n_sms);
+  if (few) return {false, std::min(bn, few)};
+  return {applies && (pair || n_pad <= 768 || short_launch(engines, n, len, n_pad)), bn};
 }
 
-static bool plain_pair(irs_sharedb* const* engines, int n, size_t len) {
+// Whether the engine runs one-SM tiles of a width that the caller gave (one that
+// divides the rows) rather than two-SM ones.
+static bool own_tiles(const irs_sharedb* e) {
+  return e->tile_override && e->n_pad % (size_t)e->tile_override == 0 && !e->pair;
+}
+
+static PlainGemm plain_gemm(irs_sharedb* const* engines, int n, size_t len) {
   const irs_sharedb* e = engines[0];
-  if (e->tile_override && !e->pair) return false;
+  const PlainGemm own{false, e->block_n};
+  if (!len || own_tiles(e)) return own;
   for (int i = 1; i < n; i++)
-    if (engines[i]->n_pad != e->n_pad) return false;  // one tile width for the launch
-  return plain_pair_for(engines, n, len, e->n_pad, e->pair);
+    if (engines[i]->n_pad != e->n_pad) return own;  // one tile width for the launch
+  return plain_gemm_for(engines, n, len, e->n_pad, e->pair, e->tile_override && e->tile_override < 256);
 }
 
-// Whether a launch of 256-row tiles with the GEMM left open has so few tiles
-// that it runs 128-row ones with their K loop shared (gemm_k_split): 64 entries
-// x 2048 rows, six engines, 81 us against 112.
-static bool few_tiles_for(irs_sharedb* const* engines, int n, size_t len, size_t n_pad) {
-  for (int i = 0; i < n; i++)
-    if (engines[i]->code_length < 8 * 128) return false;
-  return 3 * tiles_128(n, len, n_pad) <= 2 * (size_t)engines[0]->dm->n_sms;
-}
-
-static bool few_tiles(irs_sharedb* const* engines, int n, size_t len) {
+// The tile width with which a launch over `len` entries can run as the
+// rotation-structured GEMM, or -1: every engine holds sums and form maps, the
+// caller left the GEMM open (no tile width asked for) or chose the two-SM one,
+// and the quad GEMM is expected to take less.  Whether it does run depends on
+// the uploaded rows.
+static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t len, const PlainGemm& plain) {
+  uint32_t K[kMaxGemmProblems];
+  for (int i = 0; i < n; i++) {
+    const irs_sharedb* e = engines[i];
+    if (!e->sums || e->n_pad != engines[0]->n_pad || e->forms_pad != e->n_pad || offset < e->stale_end) return -1;
+    if (own_tiles(e)) return -1;
+    K[i] = (uint32_t)e->code_length;
+  }
   const irs_sharedb* e = engines[0];
-  if (e->pair || e->tile_override || e->block_n != 256) return false;
-  for (int i = 0; i < n; i++)
-    if (engines[i]->n_pad != e->n_pad) return false;
-  return few_tiles_for(engines, n, len, e->n_pad);
+  return quad_width_for(K, n, (uint32_t)len, (uint32_t)e->n_pad, plain.block_n, plain.pair, e->dm->n_sms);
 }
 
 static void fill_quad_problem(const irs_sharedb* db, const GemmProblem& g, int width, QuadProblem& pr) {
@@ -1499,10 +1506,8 @@ int irs_sharedb_runs_quads(irs_sharedb* const* engines, int n, size_t rows, size
     if (!engines[i]->sums || padded_query_rows(rows, engines[i]->n_cap) != n_pad || n_pad > engines[i]->n_cap)
       return IRS_OK;
   if (n_pad < kQuadMinRows || !len) return IRS_OK;
-  const int bn = gemm_block_n_for((uint32_t)n_pad);
-  const bool few = !pair && bn == 256 && few_tiles_for(engines, n, len, n_pad);
-  const bool on_pairs = !few && plain_pair_for(engines, n, len, n_pad, pair != 0);
-  *on = quad_width_for(K, n, (uint32_t)len, (uint32_t)n_pad, bn, on_pairs, engines[0]->dm->n_sms) >= 0;
+  const PlainGemm g = plain_gemm_for(engines, n, len, n_pad, pair != 0);
+  *on = quad_width_for(K, n, (uint32_t)len, (uint32_t)n_pad, g.block_n, g.pair, engines[0]->dm->n_sms) >= 0;
   return IRS_OK;
 }
 
@@ -1522,11 +1527,13 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
   }
   // the stall hook is the one-SM kernel's
   const bool stall = len && dm->stall_limit_ns && !dm->capturing;
-  const bool few = !stall && few_tiles(engines, n, len);
-  const bool pair = !stall && !few && plain_pair(engines, n, len);
+  const PlainGemm plain = stall ? PlainGemm{false, engines[0]->block_n} : plain_gemm(engines, n, len);
+  const Gemm kind = plain.pair                               ? Gemm::kPair
+                    : plain.block_n == engines[0]->block_n ? Gemm::kOneSm
+                    : plain.block_n == 64                  ? Gemm::k64
+                                                           : Gemm::k128;
   for (int i = 0; i < n; i++) {
-    int rc = fill_problem(engines[i], multipliers[i], offset, len,
-                          pair ? Gemm::kPair : few ? Gemm::kFewTiles : Gemm::kOneSm, P.prob[i]);
+    int rc = fill_problem(engines[i], multipliers[i], offset, len, kind, P.prob[i]);
     if (rc) return rc;
   }
   cudaStream_t s = party_stream(dm, engines[0]->peer, stream);
@@ -1547,7 +1554,7 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
     StageTimer timer(dm, s, "dot");
     SumReader lock(sum_holders(dm->device).mu);
     const bool captured = stream_captures(s);
-    const int width = stall ? -1 : quad_width(engines, n, offset, len, pair);
+    const int width = stall ? -1 : quad_width(engines, n, offset, len, plain);
     bool quads = width >= 0;
     for (int i = 0; i < n && !captured; i++) quads = quads && engines[i]->quad_rows;
     if (quads) {
@@ -1567,10 +1574,10 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
       P.skip = Q.run;
       CU(launch_quad_gemm(Q, dm->n_sms, s));
     }
-    if (!quads || captured) CU(launch_limb_gemm(P, few ? 128 : engines[0]->block_n, pair, dm->n_sms, s));
+    if (!quads || captured) CU(launch_limb_gemm(P, plain.block_n, plain.pair, dm->n_sms, s));
     for (int i = 0; i < n; i++)
       engines[i]->last_gemm =
-          quads ? (captured ? IRS_GEMM_CAPTURED : IRS_GEMM_QUAD) : pair ? IRS_GEMM_PAIR : IRS_GEMM_ONE_SM;
+          quads ? (captured ? IRS_GEMM_CAPTURED : IRS_GEMM_QUAD) : plain.pair ? IRS_GEMM_PAIR : IRS_GEMM_ONE_SM;
   }
   for (int i = 0; i < n; i++) {
     engines[i]->res_offset = offset;

@@ -770,9 +770,12 @@ int gemm_pair_n(uint32_t n_pad) {
 // 76.9 ms on 524,288 entries).  Row counts that are no multiple of the tile
 // part-fill the last one: the 64-row tile that would divide them runs at half
 // the rate (960 rows x 32,768 entries, one engine: 1.51 ms, against 0.81).
+// 832 and 896 rows (where the query capacity leaves no room for 1024) would fill
+// three quarters and less of a fourth 256-row tile: 896 rows, six engines x
+// 32,279 entries, 3.38 ms on four, 3.10 on seven of 128.
 int gemm_block_n_for(uint32_t n_pad) {
   if (n_pad == 0 || n_pad % 64) return 0;
-  return n_pad <= 64 ? 64 : n_pad <= 768 ? 128 : 256;
+  return n_pad <= 64 ? 64 : n_pad <= 896 ? 128 : 256;
 }
 
 // L2 policy of the one-SM kernel's loads (GemmParams::l2_hint), opt-in through
@@ -803,21 +806,60 @@ static uint32_t gemm_l2_hint() {
 // with): 39 tiles 13.2 / 14.3, 68 tiles 40 / 50.  Eight pay while all tiles run
 // at once; four while the longest do, and the shorter ones add at most half as
 // much again.
-static int gemm_k_split(const GemmParams& P, int block_n, int n_sms) {
-  uint32_t least = ~0u, most = 0;
-  for (int i = 0; i < P.n_prob; i++) {
-    least = std::min(least, P.prob[i].k_iters);
-    most = std::max(most, P.prob[i].k_iters);
+static int gemm_k_split(const uint32_t* k_iters, const uint32_t* tiles, int n_prob, int block_n, int n_sms) {
+  uint32_t least = ~0u, most = 0, total = 0;
+  for (int i = 0; i < n_prob; i++) {
+    least = std::min(least, k_iters[i]);
+    most = std::max(most, k_iters[i]);
+    total += tiles[i];
   }
   if (block_n > 128 || least < 8) return 1;
-  if (8 * P.total_tiles <= n_sms && least >= 16) return 8;
+  if (8 * total <= (uint32_t)n_sms && least >= 16) return 8;
   uint64_t longest = 0, blocks = 0;
-  for (int i = 0; i < P.n_prob; i++) {
-    const uint64_t tiles = (uint64_t)P.prob[i].tiles_m * P.prob[i].tiles_n;
-    if (P.prob[i].k_iters == most) longest += tiles;
-    blocks += tiles * P.prob[i].k_iters;
+  for (int i = 0; i < n_prob; i++) {
+    if (k_iters[i] == most) longest += tiles[i];
+    blocks += (uint64_t)tiles[i] * k_iters[i];
   }
   return 4 * longest <= (uint64_t)n_sms && 8 * blocks <= 3ull * (uint64_t)n_sms * most ? 4 : 1;
+}
+
+double last_done(const uint32_t* tiles, const double* cost, int n_prob, int units) {
+  double total = 0;
+  uint32_t count = 0;
+  for (int i = 0; i < n_prob; i++) {
+    total += tiles[i] * cost[i];
+    count += tiles[i];
+  }
+  constexpr int kMostUnits = 512;
+  // many rounds: the last one does not matter
+  if (count > 16u * (uint32_t)units || units > kMostUnits) return total / units;
+  double busy[kMostUnits] = {};
+  int k = 0, u = 0;
+  for (int i = 0; i < n_prob; i++)
+    for (uint32_t t = 0; t < tiles[i]; t++) {
+      busy[(size_t)((k & 1) ? units - 1 - u : u)] += cost[i];
+      if (++u == units) { u = 0; k++; }
+    }
+  return *std::max_element(busy, busy + units);
+}
+
+int few_rounds_tile(const uint32_t* K, int n_prob, uint32_t m_len, uint32_t n_pad, int n_sms) {
+  uint32_t one[kMaxGemmProblems], two[kMaxGemmProblems], k_iters[kMaxGemmProblems], total = 0, total_64 = 0;
+  double cost_one[kMaxGemmProblems], cost_two[kMaxGemmProblems];
+  for (int i = 0; i < n_prob; i++) {
+    const uint32_t m = (m_len + 127) / 128;
+    one[i] = m * ((n_pad + 127) / 128);
+    two[i] = (m_len + kBM2 - 1) / kBM2 * ((n_pad + kPairMaxN - 1) / kPairMaxN);
+    k_iters[i] = K[i] / 128;
+    cost_one[i] = k_iters[i] * kOneSmStep + 1000;
+    cost_two[i] = k_iters[i] * plain_pair_step(n_pad) + 1000;
+    total += one[i];
+    total_64 += m * (n_pad / 64);
+  }
+  if (total_64 <= (uint32_t)n_sms && gemm_k_split(k_iters, one, n_prob, 128, n_sms) == 1) return 64;
+  if (total <= (uint32_t)n_sms) return 128;
+  if (total > 4u * (uint32_t)n_sms) return 0;
+  return last_done(one, cost_one, n_prob, n_sms) < 0.97 * last_done(two, cost_two, n_prob, n_sms / 2) ? 128 : 0;
 }
 
 cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair, int n_sms, cudaStream_t stream) {
@@ -849,14 +891,17 @@ cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair, int n_sms, c
     P.pair_stages = std::min(kPairMaxStages, kPairRoom / pair_stage_bytes(P.pair_n));
   }
   P.total_tiles = 0;
+  uint32_t tiles[kMaxGemmProblems], k_iters[kMaxGemmProblems];
   for (int i = 0; i < P.n_prob; i++) {
     GemmProblem& pr = P.prob[i];
     pr.tiles_m = (pr.m_len + bm - 1) / bm;
     pr.tiles_n = (pr.n_pad + (uint32_t)block_n - 1) / (uint32_t)block_n;
-    P.total_tiles += (int)(pr.tiles_m * pr.tiles_n);
+    tiles[i] = pr.tiles_m * pr.tiles_n;
+    k_iters[i] = pr.k_iters;
+    P.total_tiles += (int)tiles[i];
   }
   if (pair) return launch_pair(P, n_sms, stream);
-  switch (P.test_stall ? 1 : gemm_k_split(P, block_n, n_sms)) {
+  switch (P.test_stall ? 1 : gemm_k_split(k_iters, tiles, P.n_prob, block_n, n_sms)) {
     case 4: return block_n == 64 ? launch_split<64, 4>(P, stream) : launch_split<128, 4>(P, stream);
     case 8: return block_n == 64 ? launch_split<64, 8>(P, stream) : launch_split<128, 8>(P, stream);
   }

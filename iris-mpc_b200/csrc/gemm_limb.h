@@ -90,6 +90,29 @@ bool gemm_pair_applies(bool pair, uint32_t n_pad);
 // Its widest tile for n_pad query rows (a multiple of 64, at most 256).
 int gemm_pair_n(uint32_t n_pad);
 
+// Cycles until the last of `units` SMs (or pairs) is done, tiles of the
+// problems dealt out in order.
+double last_done(const uint32_t* tiles, const double* cost, int n_prob, int units);
+
+// Cycles of a 128-byte K step, measured over launches of a few rounds (1.9 to 2
+// GHz): of a 128-row tile on one SM, and of the two-SM kernel's tiles over n_pad
+// rows (1300 for 128 rows, 1740 for 192, 2190 for 256).
+constexpr double kOneSmStep = 1340;
+inline double plain_pair_step(uint32_t n_pad) { return 400 + 7.0 * gemm_pair_n(n_pad); }
+
+// The width of the tiles, one to an SM, that a launch of few rounds over m_len
+// entries and n_pad rows of engines with code lengths K[0..n_prob) runs rather
+// than SM pairs or 256-row tiles: 128 or 64 rows, or 0 for no such launch.  Up to
+// a few rounds of tiles, what counts is how full the last round is; all in one
+// round, one-SM tiles take less, and 64-row ones least where they fit it and the
+// K loop of the 128-row ones would not be shared (3 engines, 1,984 rows x 89
+// entries: 62.5 / 70 us).  Over 3,000 launches of 1 to 6 engines x 64 to 2,304
+// rows x 32 to 23,000 entries, the choice between 128-row tiles and pairs is more
+// than 5% off the better one in 21, against 400 for a limit on the tiles (one
+// engine, 12,800 coefficients: 1,408 rows x 1,461 entries, 132 tiles of 128, 67 /
+// 105 us; 1,536 x 1,900, 180 tiles, 121 / 105).
+int few_rounds_tile(const uint32_t* K, int n_prob, uint32_t m_len, uint32_t n_pad, int n_sms);
+
 cudaError_t launch_limb_gemm(GemmParams& P, int block_n, bool pair, int n_sms, cudaStream_t stream);
 
 }  // namespace irs

@@ -421,44 +421,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
 }  // namespace
 
-// Cycles until the last of `units` SMs (or pairs) is done, tiles of the
-// problems dealt out in order.
-static double last_done(const uint32_t* tiles, const double* cost, int n_prob, int units) {
-  double total = 0;
-  uint32_t count = 0;
-  for (int i = 0; i < n_prob; i++) {
-    total += tiles[i] * cost[i];
-    count += tiles[i];
-  }
-  constexpr int kMostUnits = 512;
-  // many rounds: the last one does not matter
-  if (count > 16u * (uint32_t)units || units > kMostUnits) return total / units;
-  double busy[kMostUnits] = {};
-  int k = 0, u = 0;
-  for (int i = 0; i < n_prob; i++)
-    for (uint32_t t = 0; t < tiles[i]; t++) {
-      busy[(size_t)((k & 1) ? units - 1 - u : u)] += cost[i];
-      if (++u == units) { u = 0; k++; }
-    }
-  return *std::max_element(busy, busy + units);
-}
-
-// A 128-byte K step takes its MMAs (6 cycles per query column on a pair), or
-// the round trip of the three-stage pipeline where those are shorter: measured
-// about 1340 cycles, in the plain kernels as well (700 entries x 256 rows:
-// 100 steps in 0.069 ms).  The one-SM 256-row tile takes 1920 (shared memory
-// bandwidth, 80% of the MMA rate).  A product adds the drain of its
-// accumulators, and both kernels have to stream their DB planes.
+// Both sides by the rounds of their tiles (last_done) and measured cycles of a
+// 128-byte K step (gemm_limb.h has the plain ones; the one-SM 256-row tile
+// takes 2700): 1840 for 160 quads, 2070 for 192, 2530 for 256, and 1500 for the
+// drain of a product's accumulators.  Both kernels have to stream their DB
+// planes.  Over 2,500 launches of 1 to 6 engines x 576 to 2,304 rows x 1,024 to
+// 46,000 entries the choice is more than 5% off the better of the two in 75,
+// against 245 when the steps were taken for their MMAs' time (two engines, 1,088
+// rows x 1,975 entries: 290 us on the quad GEMM, 148 on 128-row tiles).
 int quad_width_for(const uint32_t* K, int n_prob, uint32_t m_len, uint32_t n_pad, int block_n, bool pair, int n_sms) {
-  constexpr double kRoundTrip = 1340, kDrain = 1000, kHbmBytesPerCycle = 3500;
+  constexpr double kDrain = 1500, kHbmBytesPerCycle = 3500;
   uint32_t tiles[kMaxGemmProblems];
   double cost[kMaxGemmProblems], bytes = 0;
-  for (int i = 0; i < n_prob; i++) bytes += 2.0 * K[i] * m_len;
-  const uint32_t bm = pair ? (uint32_t)kBM2 : (uint32_t)kBM;
+  const uint32_t bm = pair ? (uint32_t)kBM2 : (uint32_t)kBM, wide = pair ? 256u : (uint32_t)block_n;
+  const double step = pair ? plain_pair_step(n_pad) : block_n == 256 ? 2700 : kOneSmStep;
   for (int i = 0; i < n_prob; i++) {
-    const uint32_t bn = pair ? 256u : (uint32_t)block_n;
-    tiles[i] = (m_len + bm - 1) / bm * ((n_pad + bn - 1) / bn);
-    cost[i] = K[i] / 128 * (pair ? std::max(6.0 * gemm_pair_n(n_pad), kRoundTrip) : block_n == 256 ? 1920 : kRoundTrip) + kDrain;
+    bytes += 2.0 * K[i] * m_len;
+    tiles[i] = (m_len + bm - 1) / bm * ((n_pad + wide - 1) / wide);
+    cost[i] = K[i] / 128 * step + 1000;
   }
   const double plain = std::max(last_done(tiles, cost, n_prob, pair ? n_sms / 2 : n_sms), bytes / kHbmBytesPerCycle);
   int best = -1;
@@ -467,9 +447,12 @@ int quad_width_for(const uint32_t* K, int n_prob, uint32_t m_len, uint32_t n_pad
     const int bn = quad_tile_n(n_pad, w);
     for (int i = 0; i < n_prob; i++) {
       tiles[i] = (m_len + kBM2 - 1) / kBM2 * ((n_pad / 4 + bn - 1) / (uint32_t)bn);
-      cost[i] = kQuadProducts * (K[i] / 512.0 * std::max(6.0 * bn, kRoundTrip) + kDrain);
+      cost[i] = kQuadProducts * (K[i] / 512.0 * std::max(690 + 7.2 * bn, kOneSmStep) + kDrain);
     }
-    const double c = std::max(last_done(tiles, cost, n_prob, n_sms / 2), 2.25 * bytes / kHbmBytesPerCycle);
+    // (narrow tiles read more of the DB side per product: in launches of several
+    // rounds 128 quads take a tenth more than their step in one says)
+    const double c = std::max((w ? 1.1 : 1.0) * last_done(tiles, cost, n_prob, n_sms / 2),
+                              2.25 * bytes / kHbmBytesPerCycle);
     if (c < least) {
       least = c;
       best = w;
