@@ -151,7 +151,7 @@ struct irs_sharedb {
   std::vector<uint32_t*> old_flags;  // words of graphs over sums that are gone: zero, kept until destroy
   uint32_t flag_rows = 0;     // what the last upload left in it
   bool quad_rows = false;     // the uploaded rows are quads of rotations and the forms hold them
-  size_t stale_end = 0;       // records below it have sums that a small gather left behind
+  size_t stale_end = 0;       // records below it may have sums that a gather left behind
   size_t forms_pad = 0;       // padded rows that the form maps are for (0: none)
   bool dot_captured = false;  // a graph of this library reads the sums where quad_flag says so
   bool sums_pinned = false;   // another capture uses the sums: they stay until alloc_db or destroy
@@ -514,12 +514,21 @@ bool stream_captures(cudaStream_t s) {
   return false;
 }
 
-// Whether a gather of n records leaves the sums behind: for a few records the
-// quad GEMM does not run, and the sums would be the larger part of the gather.
-// (A captured launch runs it where it was captured, and a captured gather runs
-// whenever it is replayed.)
+// Whether a gather of n records leaves the sums behind, for the first dot that
+// wants them (fresh_sums): unless the rows uploaded so far are enough for the quad
+// GEMM, that dot may never come, and the sums would be a third of the gather
+// (4,000 records of 12,800: 75 us instead of 48).  A captured launch runs the GEMM that it was captured with,
+// and a captured gather runs whenever it is replayed: those keep the sums up.
 bool gather_skips_sums(const irs_sharedb* db, size_t n, cudaStream_t s) {
-  return n < kQuadMinRecords && !db->dot_captured && !db->sums_pinned && !stream_captures(s);
+  return (n < kQuadMinRecords || !db->have_query || db->n_pad < kQuadMinRows) && !db->dot_captured && !db->sums_pinned && !stream_captures(s);
+}
+
+// The sums of records [first, first + n) from the planes (the lock is held).
+cudaError_t derive_sums(irs_sharedb* db, size_t first, size_t n, cudaStream_t s) {
+  const size_t K = db->code_length, cap = db->db_cap, o = K / 2, i = 3 * K / 4;
+  uint8_t* inner = db->sums + 2 * cap * o;
+  return launch_derive_sums(db->db_lo + first * K, db->db_hi + first * K, (uint32_t)K, n, db->sums + first * o,
+                            db->sums + cap * o + first * o, inner + first * i, inner + cap * i + first * i, s);
 }
 
 // Brings the sums of records [first, first + n) in line with the planes, on
@@ -528,10 +537,15 @@ cudaError_t update_sums(irs_sharedb* db, size_t first, size_t n, cudaStream_t s)
   SumReader lock(sum_holders(db).mu);
   if (!db->sums || !n) return cudaSuccess;
   if (stream_captures(s)) db->sums_pinned = true;
-  const size_t K = db->code_length, cap = db->db_cap, o = K / 2, i = 3 * K / 4;
-  uint8_t* inner = db->sums + 2 * cap * o;
-  return launch_derive_sums(db->db_lo + first * K, db->db_hi + first * K, (uint32_t)K, n, db->sums + first * o,
-                            db->sums + cap * o + first * o, inner + first * i, inner + cap * i + first * i, s);
+  return derive_sums(db, first, n, s);
+}
+
+// Brings the sums that gathers left behind in line, on the party's stream, which
+// every dot waits for (the lock is held; no capture on that stream).
+cudaError_t fresh_sums(irs_sharedb* db) {
+  const cudaError_t e = derive_sums(db, 0, db->stale_end, db->dm->streams[db->peer]);
+  if (e == cudaSuccess) db->stale_end = 0;
+  return e;
 }
 
 // Prepares the query forms' tensor maps for the active row count; false where
@@ -1456,11 +1470,14 @@ static PlainGemm plain_gemm(irs_sharedb* const* engines, int n, size_t len) {
 // caller left the GEMM open (no tile width asked for) or chose the two-SM one,
 // and the quad GEMM is expected to take less.  Whether it does run depends on
 // the uploaded rows.
-static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t len, const PlainGemm& plain) {
+static int quad_width(irs_sharedb* const* engines, int n, size_t offset, size_t len, const PlainGemm& plain,
+                      bool captured) {
   uint32_t K[kMaxGemmProblems];
   for (int i = 0; i < n; i++) {
     const irs_sharedb* e = engines[i];
-    if (!e->sums || e->n_pad != engines[0]->n_pad || e->forms_pad != e->n_pad || offset < e->stale_end) return -1;
+    if (!e->sums || e->n_pad != engines[0]->n_pad || e->forms_pad != e->n_pad) return -1;
+    // (sums that a gather left behind are derived on the party's stream: not in a capture)
+    if (offset < e->stale_end && (captured || e->dm->capturing || stream_captures(e->dm->streams[e->peer]))) return -1;
     if (own_tiles(e)) return -1;
     K[i] = (uint32_t)e->code_length;
   }
@@ -1537,6 +1554,13 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
     if (rc) return rc;
   }
   cudaStream_t s = party_stream(dm, engines[0]->peer, stream);
+  SumReader lock(sum_holders(dm->device).mu);
+  const bool captured = stream_captures(s);
+  const int width = stall || !len ? -1 : quad_width(engines, n, offset, len, plain, captured);
+  bool quads = width >= 0;
+  for (int i = 0; i < n && !captured; i++) quads = quads && engines[i]->quad_rows;
+  for (int i = 0; i < n && quads; i++)
+    if (offset < engines[i]->stale_end) CU(fresh_sums(engines[i]));
   // The engines' inputs may have been written on their own party streams
   // (not while a graph is being captured: then all work is on the capture
   // stream and the uploads happened before the capture began).
@@ -1552,11 +1576,6 @@ int irs_sharedb_dot_many(irs_sharedb* const* engines, const uint16_t* multiplier
       dm->stall_limit_ns = 0;
     }
     StageTimer timer(dm, s, "dot");
-    SumReader lock(sum_holders(dm->device).mu);
-    const bool captured = stream_captures(s);
-    const int width = stall ? -1 : quad_width(engines, n, offset, len, plain);
-    bool quads = width >= 0;
-    for (int i = 0; i < n && !captured; i++) quads = quads && engines[i]->quad_rows;
     if (quads) {
       QuadParams Q;
       memset(&Q, 0, sizeof Q);

@@ -100,8 +100,8 @@ def test_row_tables(dm, oracle, K):
 
 
 def test_db_writes_and_gathers(dm):
-    """The records' sums follow every kind of write; a gather of few records
-    leaves the quad GEMM to launches past them until a larger one."""
+    """The records' sums follow every kind of write; those that a gather leaves
+    behind are brought in line by the next dot that reads them, outside captures."""
     K, n_db, n_q = 6400, 16384, 20
     rng = np.random.default_rng(3)
     e, src = _engine(dm, K, n_db, n_q * 32, 11), _engine(dm, K, n_db, 64, 12)
@@ -119,12 +119,29 @@ def test_db_writes_and_gathers(dm):
         assert np.array_equal(seen[-1], _plain(e, 0, n_db))
     for a, b in zip(seen, seen[1:]):
         assert not np.array_equal(a, b)
-    e.gather_records(src, np.arange(40, dtype=np.uint32))
-    e.set_db_len(n_db)
-    e.query_upload_slots(base, [(j, 0, 31, j) for j in range(n_q)])
-    e.dot(0, n_db, 1)
-    assert e.last_gemm()[0] == "pair"
-    assert np.array_equal(e.fetch_results(n_db), _plain(e, 0, n_db))
+    for n in (40, n_db):  # a few; and all of them while no rows are there for the quad GEMM
+        for captured in (False, True):
+            e.query_upload(base[:1])
+            e.gather_records(src, rng.permutation(n_db)[:n].astype(np.uint32))
+            e.set_db_len(n_db)
+            e.query_upload_slots(base, [(j, 0, 31, j) for j in range(n_q)])
+            past = _quad(e, 64, n_db - 64) if n == 40 else None  # records past those: no need
+            plain = _plain(e, 0, n_db)
+            assert past is None or np.array_equal(past, plain[:, 64:])
+            if captured:
+                dm.synchronize()
+                g = irisb200.Graph.capture(dm, lambda: e.dot(0, n_db, 1, dm.stream(0)))
+                assert e.last_gemm()[0] == "pair"
+                g.launch(dm.stream(2))
+                dm.synchronize()
+                assert np.array_equal(e.fetch_results(n_db), plain)
+                g.close()
+            e.dot(0, n_db, 1, dm.stream(2))  # on a stream of its own
+            dm.synchronize()
+            irisb200.dot_many([e], [1], 0, n_db, dm.stream(1))
+            assert e.last_gemm()[0] == "quad"
+            dm.synchronize()
+            assert np.array_equal(e.fetch_results(n_db), plain)
     e.close()
     src.close()
 
