@@ -517,8 +517,9 @@ bool stream_captures(cudaStream_t s) {
 // Whether a gather of n records leaves the sums behind, for the first dot that
 // wants them (fresh_sums): unless the rows uploaded so far are enough for the quad
 // GEMM, that dot may never come, and the sums would be a third of the gather
-// (4,000 records of 12,800, waited for: 110 us instead of 71).  A captured launch runs the GEMM that it was captured with,
-// and a captured gather runs whenever it is replayed: those keep the sums up.
+// (4,000 records of 12,800, waited for: 110 us instead of 71).  A captured launch
+// runs the GEMM that it was captured with, and a captured gather runs whenever it
+// is replayed: those keep the sums up.
 bool gather_skips_sums(const irs_sharedb* db, size_t n, cudaStream_t s) {
   return (n < kQuadMinRecords || !db->have_query || db->n_pad < kQuadMinRows) && !db->dot_captured && !db->sums_pinned && !stream_captures(s);
 }

@@ -16,6 +16,7 @@
 // GEMM (quad_gemm.cu) splits them.  A dot product does not depend on the order.
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <algorithm>
 #include "common.cuh"
 #include "launch_attr.cuh"
 #include "prep.h"
@@ -302,22 +303,28 @@ __device__ __forceinline__ void gr4_mul(const uint32_t a[4], const uint32_t b[4]
   o[3] = a[0] * b[3] + a[1] * b[2] + a[2] * b[1] + a[3] * b[0] + d6;
 }
 
-// One CTA per entry.  Mirrors the synthetic generator and the degree-1 Shamir
-// encoding the CPU oracle defines (iris bits from rng64, mask pairs kept with
-// probability 0.9, share randomness r = rng64(share seed, block)).
 // Seeded uniform bytes (splitmix64 of the 8-byte word index): random shares
 // for benchmark buffers whose values do not matter, only their bit activity.
-// With K > 0 the words go to a limb plane of rows of K in record order.
-__global__ void fill_random_kernel(uint64_t* __restrict__ p, size_t n_words, uint64_t seed, uint32_t K) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += (size_t)gridDim.x * blockDim.x) {
-    uint64_t z = seed + (i + 1) * 0x9E3779B97F4A7C15ull;
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    const size_t d = K ? i / (K / 8) * (K / 8) + plane_octet((uint32_t)(i % (K / 8)), K) : i;
-    p[d] = z ^ (z >> 31);
+__global__ void fill_random_kernel(uint64_t* __restrict__ p, size_t n_words, uint64_t seed) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += (size_t)gridDim.x * blockDim.x)
+    p[i] = rng64(seed, i);
+}
+// The same words, in record order, for a limb plane of `rows` rows of K: a thread
+// takes four consecutive words, one for each quarter.
+__global__ void fill_random_plane_kernel(uint64_t* __restrict__ p, size_t rows, uint64_t seed, uint32_t K) {
+  const uint32_t quarter = K / 32;  // words
+  const size_t n = rows * quarter;
+  for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+    const size_t r = n >> 32 ? t / quarter : (uint32_t)t / quarter;
+    uint64_t* out = p + r * 4 * quarter + (t - r * quarter);
+#pragma unroll
+    for (int q = 0; q < 4; q++) out[q * quarter] = rng64(seed, 4 * t + q);
   }
 }
 
+// One CTA per entry.  Mirrors the synthetic generator and the degree-1 Shamir
+// encoding the CPU oracle defines (iris bits from rng64, mask pairs kept with
+// probability 0.9, share randomness r = rng64(share seed, block)).
 __global__ void synth_db_kernel(uint64_t seed, uint32_t first, uint32_t count, SynthOut out) {
   __shared__ uint64_t code[200], mask[200];
   const uint32_t e = first + blockIdx.x;
@@ -441,10 +448,11 @@ cudaError_t launch_gather_rows(const uint8_t* src_lo, const uint8_t* src_hi, con
 }
 
 cudaError_t launch_fill_random(void* p, size_t bytes, uint64_t seed, uint32_t K, cudaStream_t stream) {
-  const size_t n = bytes / 8;
+  const size_t n = bytes / 8, threads = K ? n / 4 : n;
   if (n) {
-    const size_t blocks = (n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16;
-    fill_random_kernel<<<(unsigned)blocks, 256, 0, stream>>>(static_cast<uint64_t*>(p), n, seed, K);
+    const unsigned blocks = (unsigned)std::min<size_t>((threads + 255) / 256, 148 * 16);
+    if (K) fill_random_plane_kernel<<<blocks, 256, 0, stream>>>(static_cast<uint64_t*>(p), n / (K / 8), seed, K);
+    else fill_random_kernel<<<blocks, 256, 0, stream>>>(static_cast<uint64_t*>(p), n, seed);
   }
   return cudaGetLastError();
 }

@@ -103,3 +103,20 @@ def test_stored_limbs_need_no_free_memory():
             b.free()
         e.close()
         dm.close()
+
+
+@pytest.mark.parametrize("K,n", [(128, 3), (6400, 70), (12800, 2400)])
+def test_random_records_are_the_seeded_words(dm, K, n):
+    """fill_random: 64-bit word i of each limb, in record order, is splitmix64 of the seed at i."""
+    e = irisb200.ShareDB(0, dm, 64, 64, K, W.SEEDS[0])
+    e.alloc_db(n)
+    e.fill_random(99, n)
+
+    def limb(seed):
+        with np.errstate(over="ignore"):
+            z = np.uint64(seed) + np.arange(1, n * K // 8 + 1, dtype=np.uint64) * np.uint64(0x9E3779B97F4A7C15)
+            z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+            z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+        return (z ^ (z >> np.uint64(31))).view(np.uint8).astype(np.uint16).reshape(n, K)
+    assert np.array_equal(e.fetch_records(0, n), limb(99) | limb(99 ^ 0x5A5A5A5A5A5A5A5A) << 8)
+    e.close()
