@@ -72,7 +72,8 @@ struct irs_device_manager {
   cudaEvent_t graph_done = nullptr;  // complete when every graph launched so far has run
   cudaStream_t graph_join = nullptr;  // the graphs' streams meet here, and graph_done follows them
   cudaEvent_t graph_ran = nullptr;    // recorded after each graph launch, on its stream
-  cudaEvent_t uploads[3] = {nullptr, nullptr, nullptr};  // recorded on the parties' streams before one (and before a capture)
+  // recorded on the parties' streams before a graph launch or a capture
+  cudaEvent_t uploads[3] = {nullptr, nullptr, nullptr};
   bool host_sync = true;  // false: host-buffer calls return once enqueued (irs_device_manager_set_host_sync)
   // stage timers (irs_device_manager_set_timing): event pairs per label, resolved on read
   bool timing = false;
@@ -521,7 +522,8 @@ bool stream_captures(cudaStream_t s) {
 // runs the GEMM that it was captured with, and a captured gather runs whenever it
 // is replayed: those keep the sums up.
 bool gather_skips_sums(const irs_sharedb* db, size_t n, cudaStream_t s) {
-  return (n < kQuadMinRecords || !db->have_query || db->n_pad < kQuadMinRows) && !db->dot_captured && !db->sums_pinned && !stream_captures(s);
+  const bool wanted = n >= kQuadMinRecords && db->have_query && db->n_pad >= kQuadMinRows;
+  return !wanted && !db->dot_captured && !db->sums_pinned && !stream_captures(s);
 }
 
 // The sums of records [first, first + n) from the planes (the lock is held).
